@@ -2139,38 +2139,51 @@ struct GatherTerms {
     float energy, denom, depth, dissipation, normalPower, stiffness, viscous;
 };
 // Accumulator chains: 0-2 force and 3-5 torque (compensated), 6-14 the three
-// stress rows (subtracted), 15 energy, 16 denominator, 17 deepest overlap
+// stress rows (stored negated), 15 energy, 16 denominator, 17 deepest overlap
 // (maximum), 18 dissipation, 19 normal loss power, 20-21 timestep rates.
 constexpr uint32_t GATHER_CHAINS = 22;
-constexpr uint32_t GATHER_STRIDE = WARP + 1;  // padded rows: conflict-free on both sides
+// Row stride: 16-byte rows for the replay's float4 reads; at 36 words a
+// quarter warp's reads (and a warp's word stores) touch every bank once.
+constexpr uint32_t GATHER_STRIDE = WARP + 4;
 __device__ __forceinline__ f3 shfl3(f3 v, int lane) {
     return mk(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
               __shfl_sync(0xffffffffu, v.z, lane));
 }
 // Lane `chain` replays its accumulator chain over the `count` terms of one
-// round, in order (compensated sums, subtracted stress rows, maximum depth,
-// plain sums; the timestep rates only under the active-contact policy).
-__device__ __forceinline__ void replayChain(float (*terms)[GATHER_STRIDE], uint32_t count, uint32_t chain, bool rates,
+// round, in order.  Every chain runs the same instructions: the compensated
+// step (y = t + low, next = acc + y, low = y - (next - acc)), whose residual
+// only the force and torque chains keep.  With low = +0 the step is the plain
+// sum acc + t bit for bit (acc starts at +0 and is never -0, so a -0 term
+// read as +0 changes nothing); the stress rows are stored negated (a - b is
+// a + (-b)), and the maximum chain selects.  One loop for the warp, fed by
+// float4 shared loads, instead of one per kind of chain: those four diverged
+// and ran one after the other.  The gather went from 205 to 164 us for
+// 15,625 grains with 2.0 M contacts, 129 to 113 us for 50,000 with 950 k.
+__device__ __forceinline__ void replayChain(const float (*terms)[GATHER_STRIDE], uint32_t count, uint32_t chain,
                                             float& acc, float& accLow) {
-    if (chain < 6) {
-        for (uint32_t k = 0; k < count; ++k) {  // compensated3, one component
-            float y = __fadd_rn(terms[chain][k], accLow);
-            float nx = __fadd_rn(acc, y);
-            accLow = __fsub_rn(y, __fsub_rn(nx, acc));
-            acc = nx;
-        }
-    } else if (chain < 15) {
-        for (uint32_t k = 0; k < count; ++k) acc = __fsub_rn(acc, terms[chain][k]);
-    } else if (chain == 17) {
-        for (uint32_t k = 0; k < count; ++k) acc = mx(acc, terms[chain][k]);
-    } else if (chain < GATHER_CHAINS && (chain < 20 || rates)) {
-        for (uint32_t k = 0; k < count; ++k) acc = __fadd_rn(acc, terms[chain][k]);
+    const float* row = terms[min(chain, GATHER_CHAINS - 1)];
+    const bool compensated = chain < 6, maximum = chain == 17;
+    auto step = [&](float t) {
+        float y = __fadd_rn(t, accLow);
+        float nx = __fadd_rn(acc, y);
+        float low = __fsub_rn(y, __fsub_rn(nx, acc));
+        accLow = compensated ? low : 0.0f;
+        acc = maximum ? mx(acc, t) : nx;
+    };
+    uint32_t k = 0;
+    for (; k + 4 <= count; k += 4) {
+        float4 t = *reinterpret_cast<const float4*>(row + k);
+        step(t.x);
+        step(t.y);
+        step(t.z);
+        step(t.w);
     }
+    for (; k < count; ++k) step(row[k]);
 }
 __device__ __forceinline__ void storeTerms(float (*terms)[GATHER_STRIDE], uint32_t lane, const GatherTerms& g) {
     const float v[GATHER_CHAINS] = {g.force.x, g.force.y, g.force.z, g.torque.x, g.torque.y, g.torque.z,
-                                    g.s0.x, g.s0.y, g.s0.z, g.s1.x, g.s1.y, g.s1.z,
-                                    g.s2.x, g.s2.y, g.s2.z, g.energy, g.denom, g.depth,
+                                    -g.s0.x, -g.s0.y, -g.s0.z, -g.s1.x, -g.s1.y, -g.s1.z,
+                                    -g.s2.x, -g.s2.y, -g.s2.z, g.energy, g.denom, g.depth,
                                     g.dissipation, g.normalPower, g.stiffness, g.viscous};
 #pragma unroll
     for (uint32_t j = 0; j < GATHER_CHAINS; ++j) terms[j][lane] = v[j];
@@ -2211,7 +2224,7 @@ __global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Param
     if (r.control[0] != 0) return;
     uint32_t pairs = activePairs(r, c);
     __shared__ uint32_t window[8][4][WARP];  // per warp: B candidates, merged pairs, offsets, range ends
-    __shared__ float termRows[8][GATHER_CHAINS][GATHER_STRIDE];
+    __shared__ __align__(16) float termRows[8][GATHER_CHAINS][GATHER_STRIDE];
     uint32_t* wb = window[threadIdx.x >> 5][0];
     uint32_t* wp = window[threadIdx.x >> 5][1];
     uint32_t* wo = window[threadIdx.x >> 5][2];
@@ -2233,7 +2246,7 @@ __global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Param
                 uint32_t count = min(hi - lo, WARP);
                 if (laneId() < count) storeTerms(terms, laneId(), wallTerms(r, c, hi - 1 - laneId(), w, m_, bw, inverseInertia));
                 __syncwarp();
-                replayChain(terms, count, chain, c.activeTimestep != 0, acc, accLow);
+                replayChain(terms, count, chain, acc, accLow);
                 __syncwarp();
                 hi -= count;
             }
@@ -2324,7 +2337,7 @@ __global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Param
                     storeTerms(terms, lane, g);
                 }
                 __syncwarp();
-                replayChain(terms, count, chain, c.activeTimestep != 0, acc, accLow);
+                replayChain(terms, count, chain, acc, accLow);
                 __syncwarp();
             }
             __syncwarp();
