@@ -11,7 +11,7 @@
  *             (src/sand_atlas_dem/shaders/solver.slang:20-100) — the same
  *             order the reference CPU backend binds in its generated
  *             cpu_dispatch (src/sand_atlas_dem/cpu.py:189-300);
- *   [77, 136) this backend's extension buffers, in the order of
+ *   [77, 140) this backend's extension buffers, in the order of
  *             sand_atlas_dem_gb300.engine.EXTENSION_ORDER (leaf tables,
  *             node ranks, pair-by-second-grain runs, directed-pair branches,
  *             leaf masks, (directed pair, leaf) items and hit masks, contact
@@ -33,21 +33,28 @@
  *             the signed distance with its origin and cell size, and the
  *             triangle nearest to each cell centre, and the pose the stored
  *             node-filter results were built at: each grain's orientation,
- *             each pair's branch and the pair list itself, and the walk
- *             order of the stored exact-query list: each kept survivor's
- *             bucket (target shape, coarse cell), and the count and first
- *             slot of each bucket, and for the SDF geometry each pair's
+ *             each pair's branch and the pair list itself, and a
+ *             slot list (slots left to a walk; the culler's sorted
+ *             survivors) with the culler's per-shape counts and their
+ *             scan, and for the SDF geometry each pair's
  *             contact counts per virtual lane of the reference's 64-lane
  *             group, 32 words per pair, and per stored walk-list slot its
- *             nearest-triangle certificate: the point it was taken at with
- *             the distance gap, and the triangle with a tying triangle of
- *             another leaf (two words; or a dormant mark), and with planes the
+ *             nearest-triangle certificate (48 bytes: the point it was
+ *             taken at with the distance gap, and up to seven triangles)
+ *             and its state word (certified, not, or dormant), and with planes the
  *             plane-contact count of each (wall, grain), wall-major, its
  *             exclusive scan, and the first contact of each (wall, grain)
  *             on the side being written and on the committed side, and per
  *             stored walk-list slot its node record -- source grain, target
- *             grain, directed pair and packed sample index -- and its
- *             (item, node slot)).
+ *             grain, directed pair and packed sample index -- and the
+ *             contact it was last, and per distance-grid cell the list of the
+ *             triangles near it (256 bytes: a limit, the nearest triangle's
+ *             distance, 48 triangles nearest first and a byte each of
+ *             distance beyond the nearest; optional, 16 bytes where not kept),
+ *             the BVH leaf of each packed triangle, and the list of the
+ *             stored walk-list slots not dormant after their build and the
+ *             step's hits of those slots: a bit each, a count per 256 and
+ *             one per 16,384).
  * Value block (SDG_VALUE_COUNT doubles): the 25 reference Config scalars in
  * declaration order (solver.slang:12-19, normalized units as
  * src/sand_atlas_dem/gpu.py:490-518 builds them), then leaf mask words per
@@ -83,7 +90,7 @@
 extern "C" {
 #endif
 
-#define SDG_BUFFER_COUNT 136
+#define SDG_BUFFER_COUNT 140
 #define SDG_VALUE_COUNT 39
 #define SDG_PHASES 9
 

@@ -61,6 +61,8 @@ static int unpack(void* const* buffers, const uint64_t* bytes, const double* val
         for (int k = 0; k < 4; ++k)
             c.library16[k] = bytes ? uint32_t(std::min<uint64_t>(bytes[library[k]] / 16, 0xFFFFFFFFu)) : 0u;
     }
+    // The triangle lists are optional: used where the buffer holds them.
+    c.cellListsEnabled = bytes && bytes[77 + 59] >= uint64_t(c.shapes) * GRID * GRID * GRID * CELL_WORDS * 4;
     if (!(c.filterMargin >= 0.0f) || c.filterMargin > 1.0f) {
         g_error = "filter margin must lie in [0, 1] (target shape frame)";
         return 1;
@@ -110,8 +112,12 @@ static int unpack(void* const* buffers, const uint64_t* bytes, const double* val
             bytes[77 + 48] < (uint64_t(c.shapes) * WALK_BUCKETS + 1) * 4 ||
             bytes[77 + 49] < (uint64_t(c.shapes) * WALK_BUCKETS + 1) * 4 ||
             (c.meshGeometry == 0 && bytes[77 + 50] < uint64_t(c.pairCapacity) * 32 * 4) ||
-            bytes[77 + 51] < uint64_t(c.survivorCapacity) * 16 || bytes[77 + 52] < uint64_t(c.survivorCapacity) * 8 ||
-            bytes[77 + 57] < uint64_t(c.survivorCapacity) * 16 || bytes[77 + 58] < uint64_t(c.survivorCapacity) * 8 ||
+            bytes[77 + 51] < uint64_t(c.survivorCapacity) * 16 * CERT_ROWS ||
+            bytes[77 + 52] < uint64_t(c.survivorCapacity) * 4 ||
+            (c.meshGeometry != 0 && storedKeep(c) && bytes[77 + 60] < bytes[31] / 48 * 4) ||
+            bytes[77 + 61] < uint64_t(c.survivorCapacity) * 4 ||
+            bytes[77 + 62] < slotHitSize(c.survivorCapacity) * 4 ||
+            bytes[77 + 57] < uint64_t(c.survivorCapacity) * 16 || bytes[77 + 58] < uint64_t(c.survivorCapacity) * 4 ||
             (c.wallCount != 0 &&
              (bytes[70] < uint64_t(c.wallCount) * 16 || bytes[71] < uint64_t(c.wallCount) * 16 ||
               bytes[72] < uint64_t(c.wallCount) * 16 || bytes[73] < uint64_t(c.wallCount) * 16 ||
@@ -133,21 +139,33 @@ int unpack_params(void* const* buffers, const uint64_t* bytes, const double* val
     return unpack(buffers, bytes, values, nvalues, P);
 }
 
+// Whether the filter results (items, survivor and exact-query lists) are
+// stored and rebuilt only on the steps whose motion check asks for it.
+static bool storedFilters(const Config& c) { return c.meshGeometry != 0 && storedKeep(c); }
+
+// Contacts and their law; `build(body)` runs the filter build where the
+// results are stored.
+template <class Build>
+static void collectAndResolve(const Params& P, cudaStream_t s, Build&& build) {
+    if (storedFilters(P.c)) {
+        launch_contacts("collectHead", P, 0, s);
+        build([&](cudaStream_t b) { launch_contacts("collectBuild", P, 0, b); });
+        launch_contacts("collectTail", P, 0, s);
+        launch_contacts("resolveWalls", P, 0, s);
+    } else {
+        launch_contacts("collect", P, 0, s);
+        launch_contacts("resolveContacts", P, 0, s);
+    }
+}
+
 void launch_forces(const Params& P, cudaStream_t s, bool captureKinematics) {
     const Config& c = P.c;
     if (c.normalViscosity > 0 && captureKinematics) launch_state("captureContactKinematics", P, c.N, s);
     launch_contacts("neighbours", P, c.N, s);
-    launch_contacts("collect", P, 0, s);
-    launch_contacts("resolveContacts", P, 0, s);
+    collectAndResolve(P, s, [&](auto&& body) { body(s); });
     launch_contacts("gather", P, c.N, s);
     launch_contacts("gatherWallRows", P, c.N, s);
     if (c.activeTimestep) launch_state("checkContactTimestep", P, c.N, s);
-}
-
-// Whether the filter results (items, survivor and exact-query lists) are
-// stored and rebuilt only on the steps whose motion check asks for it.
-static bool storedFilters(const Config& c) {
-    return c.meshGeometry != 0 && c.filterMargin > 0.0f && c.cullerEnabled == 0;
 }
 
 // One step of Engine._advance_once (gpu.py:714-724); captureContactKinematics
@@ -169,14 +187,7 @@ static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
     if (c.wallCount) launch_state("advanceWalls", P, 1, s);
     launch_state("checkRebuild", P, c.N, s);
     branch(P.r.control + 4, [&](cudaStream_t b) { launch_contacts("neighbours", P, c.N, b); });
-    if (storedFilters(c)) {
-        launch_contacts("collectHead", P, 0, s);
-        branch(P.r.work + W_FILTER, [&](cudaStream_t b) { launch_contacts("collectBuild", P, 0, b); });
-        launch_contacts("collectTail", P, 0, s);
-    } else {
-        launch_contacts("collect", P, 0, s);
-    }
-    launch_contacts("resolveContacts", P, 0, s);
+    collectAndResolve(P, s, [&](auto&& body) { branch(P.r.work + W_FILTER, body); });
     launch_contacts("gather", P, c.N, s);
     launch_contacts("gatherWallRows", P, c.N, s);
     if (c.activeTimestep) launch_state("checkContactTimestep", P, c.N, s);

@@ -18,6 +18,7 @@ constexpr uint32_t EMPTY = 0xffffffffu;
 // A stored walk slot whose node was found farther outside its target than
 // any motion the stored filter results allow before their next build.
 constexpr uint32_t DORMANT = 0xfffffffeu;
+constexpr uint32_t CERTIFIED = 0;
 constexpr int RESOURCE_COUNT = 77;
 
 // Solver flags (src/sand_atlas_dem/gpu.py:11-26) plus one for bounded waits.
@@ -59,6 +60,9 @@ struct Config {
     // the library arrays the exact queries read: meshChildren, meshTriangles,
     // meshNormals, sample.  The step prefetches them into L2.
     uint32_t library16[4];
+    // Whether the caller's buffers hold the per-cell triangle lists (cellLists
+    // and triangleLeaf at full size).
+    uint32_t cellListsEnabled;
 };
 
 // Buffers: the reference Resources block (solver.slang:20-100) in declaration
@@ -110,7 +114,7 @@ struct Res {
     const uint32_t* oldContactStart;  // pairCapacity+1
     uint32_t* work;                   // 64 counters
     uint32_t* scanPartials;           // 2*SCAN_BLOCKS
-    float4* hitScratch;               // 2*survivorCapacity: (point/depth, normal/area) per survivor
+    float4* hitScratch;               // 2*survivorCapacity: (point/depth, normal/area) per survivor or stored slot
     uint32_t* candSurvCount;          // candidateCapacity+1: nodes of each item left for the exact query
     float4* dpairPlane;               // 2*pairCapacity: enclosure plane of the target facing the source
     const uint32_t* grainSpecimen;    // N: specimen of each grain
@@ -124,7 +128,7 @@ struct Res {
     uint2* survivors;                 // survivorCapacity: (item, node slot) of each surviving node
     uint32_t* survKeep;               // survivorCapacity+1: 1 = the learned culler keeps the survivor
     uint32_t* keepOffset;             // survivorCapacity+1: exclusive scan of survKeep
-    uint32_t* walkList;               // survivorCapacity: survivors left for the exact query
+    uint32_t* walkList;               // survivorCapacity: survivors left for the exact query (lists built every step)
     float4* dpairSourcePlane;         // 4*pairCapacity: the enclosure plane in the source frame, and its bound terms
     const float4* meshChildren;       // 4 per BVH node: both children's bounds (internal) or the triangle range
     float* distanceGrid;              // shapes x GRID^3: certified lower bound of the signed distance per cell
@@ -133,23 +137,26 @@ struct Res {
     float4* filterRefRotation;        // N: orientation when the filter results were built
     float4* filterRefBranch;          // pairCapacity: first-to-second branch when they were built
     uint2* filterRefPairs;            // pairCapacity: the pair list they were built on
-    uint32_t* walkKey;                // survivorCapacity: bucket of each kept survivor (target shape, coarse cell)
-    uint32_t* walkBucketCount;        // shapes x WALK_BUCKETS + 1: kept survivors per bucket
-    uint32_t* walkBucketOffset;       // shapes x WALK_BUCKETS + 1: first walk-list slot of each bucket
+    uint32_t* walkKey;                // survivorCapacity: the active slots left to a walk; the culler's sorted list
+    uint32_t* walkBucketCount;        // shapes x WALK_BUCKETS + 1: the culler's survivors per shape (first `shapes`)
+    uint32_t* walkBucketOffset;       // shapes x WALK_BUCKETS + 1: their scan
     uint32_t* sdfLaneCounts;          // SDF geometry, 32 x pairCapacity: contacts of virtual lanes l and l + 32
-    float4* walkCertPoint;            // survivorCapacity: per stored walk slot, where its certificate was taken, and the gap
-    uint2* walkCertTriangle;          // survivorCapacity: x its certified nearest triangle (EMPTY: none; DORMANT:
-                                      // cannot touch before the next build), y a triangle of another leaf tying it
-                                      // with the same result (EMPTY: none)
+    uint4* walkCert;                  // CERT_ROWS x survivorCapacity: per stored walk slot its certificate
+    uint32_t* walkState;              // survivorCapacity: per stored walk slot CERTIFIED, EMPTY (no certificate) or
+                                      // DORMANT (cannot touch before the next build)
     uint32_t* wallCounts;             // wallCount x N: plane contacts of each (wall, grain), wall-major
     uint32_t* wallOffsets;            // wallCount x N + 1: their exclusive scan
     uint32_t* sideWallStart;          // wallCount x N + 1: first contact of each (wall, grain), side being written
     const uint32_t* oldWallStart;     // wallCount x N + 1: the same on the committed side
     uint4* walkNode;                  // survivorCapacity: per stored walk slot (source, target, directed pair, packed sample)
-    uint2* walkItem;                  // survivorCapacity: per stored walk slot (item, node slot)
+    uint32_t* walkContact;            // survivorCapacity: per stored walk slot the contact it was last (a hint)
+    uint32_t* cellLists;              // shapes x GRID^3 x CELL_WORDS: the triangles near each grid cell
+    uint32_t* triangleLeaf;           // packed triangles: the BVH leaf holding each
+    uint32_t* walkActive;             // survivorCapacity: the stored walk slots not dormant after their build
+    uint32_t* walkHits;               // the step's hits of the active slots (see SlotHits)
 };
-constexpr int EXTENSION_COUNT = 59;
-constexpr uint32_t WALK_CELLS = 24;  // coarse cells per axis of a shape's grid box for the walk order
+constexpr int EXTENSION_COUNT = 63;
+constexpr uint32_t WALK_CELLS = 24;  // the walk-bucket arrays hold WALK_CELLS^3 words per shape
 constexpr uint32_t WALK_BUCKETS = WALK_CELLS * WALK_CELLS * WALK_CELLS;
 constexpr uint32_t GRID = 48;  // cells per axis of each shape's distance-bound grid
 constexpr int CULLER_PARAMS = 3 * 64 + 64 + 64 * 64 + 64 + 64 + 4;
@@ -175,6 +182,8 @@ constexpr int W_CERTIFIED = 15;     // exact queries answered by a certificate (
 constexpr int W_WALL_BASE = 16;     // first plane contact: the grain-grain contact total
 constexpr int W_REBUILDS = 17;      // steps that rebuilt the neighbour list (counter)
 constexpr int W_DORMANT = 18;       // dormant slots in the stored exact-query list
+constexpr int W_LAPSED = 20;        // stored walk slots without a certificate that holds this step
+constexpr int W_ACTIVE = 21;        // stored walk slots listed as live when the results were built
 constexpr int W_CULL_ROWS = 19;     // kept survivors in the culler's shape-sorted list
 
 struct Params {
@@ -305,19 +314,47 @@ __device__ __forceinline__ double imageShift(double d, double box) {
     return floor(__dadd_rn(__ddiv_rn(d, box), 0.5));
 }
 // Minimum-image branch j - i in FP64, cast to FP32 (cpu_scheduling.slang:10-15).
-__device__ __forceinline__ f3 centerBranch64(const Res& r, const Config& c, uint32_t i, uint32_t j) {
+struct Separation64 {
+    double d[3], box[3];
+};
+__device__ __forceinline__ Separation64 separation64(const Res& r, uint32_t i, uint32_t j) {
     float4 pi = r.position[i], pj = r.position[j], li = r.positionRemainder[i], lj = r.positionRemainder[j];
     float4 cell = r.cell[3 * specimenOf(r, i)];
-    double dx = __dadd_rn(__dsub_rn((double)pj.x, (double)pi.x), __dsub_rn((double)lj.x, (double)li.x));
-    double dy = __dadd_rn(__dsub_rn((double)pj.y, (double)pi.y), __dsub_rn((double)lj.y, (double)li.y));
-    double dz = __dadd_rn(__dsub_rn((double)pj.z, (double)pi.z), __dsub_rn((double)lj.z, (double)li.z));
-    if (c.periodic != 0) {
-        double bx = cell.x, by = cell.y, bz = cell.z;
-        dx = __dsub_rn(dx, __dmul_rn(imageShift(dx, bx), bx));
-        dy = __dsub_rn(dy, __dmul_rn(imageShift(dy, by), by));
-        dz = __dsub_rn(dz, __dmul_rn(imageShift(dz, bz), bz));
+    return {{__dadd_rn(__dsub_rn((double)pj.x, (double)pi.x), __dsub_rn((double)lj.x, (double)li.x)),
+             __dadd_rn(__dsub_rn((double)pj.y, (double)pi.y), __dsub_rn((double)lj.y, (double)li.y)),
+             __dadd_rn(__dsub_rn((double)pj.z, (double)pi.z), __dsub_rn((double)lj.z, (double)li.z))},
+            {cell.x, cell.y, cell.z}};
+}
+__device__ __forceinline__ float imaged(const Config& c, double d, double box) {
+    if (c.periodic != 0) d = __dsub_rn(d, __dmul_rn(imageShift(d, box), box));
+    return __double2float_rn(d);
+}
+__device__ __forceinline__ f3 centerBranch64(const Res& r, const Config& c, uint32_t i, uint32_t j) {
+    Separation64 s = separation64(r, i, j);
+    return {imaged(c, s.d[0], s.box[0]), imaged(c, s.d[1], s.box[1]), imaged(c, s.d[2], s.box[2])};
+}
+// The branch and the reverse one.  The raw separation changes sign exactly
+// (IEEE rounding is symmetric; an exact zero stays +0, hence 0 - x), and so
+// does the image wherever the shift is picked by the FP32 margins of
+// imageShift; near half a box (and beyond 1.45) the reverse is evaluated by
+// itself.  GB300 runs about two FP64 operations a cycle and SM: the second
+// evaluation was a third of the pair set-up.
+__device__ __forceinline__ void centerBranches64(const Res& r, const Config& c, uint32_t i, uint32_t j, f3& forward,
+                                                 f3& back) {
+    Separation64 s = separation64(r, i, j);
+    float f[3], b[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        f[a] = imaged(c, s.d[a], s.box[a]);
+        b[a] = __fsub_rn(0.0f, f[a]);
+        if (c.periodic != 0) {
+            float ad = fabsf(__double2float_rn(s.d[a])), fb = __double2float_rn(s.box[a]);
+            if (!(ad <= __fmul_rn(0.45f, fb)) && !(ad >= __fmul_rn(0.55f, fb) && ad <= __fmul_rn(1.45f, fb)))
+                b[a] = imaged(c, -s.d[a], s.box[a]);
+        }
     }
-    return {__double2float_rn(dx), __double2float_rn(dy), __double2float_rn(dz)};
+    forward = mk(f[0], f[1], f[2]);
+    back = mk(b[0], b[1], b[2]);
 }
 // solver.slang:154-158
 __device__ __forceinline__ f3 omega(const Res& r, uint32_t i, float4 q, f3 l) {
@@ -459,24 +496,10 @@ __device__ __forceinline__ bool sameResult(const Res& r, f3 q, uint32_t normal, 
            __float_as_uint(q.z) == __float_as_uint(q2.z) && __float_as_uint(n.x) == __float_as_uint(n2.x) &&
            __float_as_uint(n.y) == __float_as_uint(n2.y) && __float_as_uint(n.z) == __float_as_uint(n2.z);
 }
-// `Warp`: the whole warp runs one walk (p, shape, seed and reach the same on
-// every lane).  Every lane then holds the same stack and takes the same
-// decisions; the lanes evaluate a leaf's triangles together and its results
-// are taken in triangle order, so the walk and its result are the
-// one-thread walk's.  A few walks fill a warp each, instead of one lane of a
-// diverging warp each.
-// `children`/`nodeBase`: where the walk reads node n's record --
-// children + 4 (n - nodeBase): the library's meshChildren (base 0) or the
-// shape's records staged in shared memory (base: its first node); and
-// `triangles`/`triangleBase` likewise for triangle t's three vertices,
-// triangles + 3 (t - triangleBase).
-template <bool Warp>
-__device__ __forceinline__ float4 meshDistanceCertifiedT(const Res& r, uint32_t shape, f3 p, uint32_t seed,
-                                                         float reach, uint32_t& triangle, uint32_t& tie, float& gap,
-                                                         const float4* children, uint32_t nodeBase,
-                                                         const float4* triangles, uint32_t triangleBase) {
+__device__ __forceinline__ float4 meshDistanceCertified(const Res& r, uint32_t shape, f3 p, uint32_t seed, float reach,
+                                                        uint32_t& triangle, uint32_t& tie, float& gap) {
     uint32_t root = __ldg(&r.meshRoots[shape].x);
-    auto vertex = [&](uint32_t t, uint32_t k) { return xyz(triangles[3 * (t - triangleBase) + k]); };
+    auto vertex = [&](uint32_t t, uint32_t k) { return xyz(__ldg(&r.meshTriangles[3 * t + k])); };
     uint32_t pending[32];
     float pendingDistance[32];
     uint32_t top = 1;
@@ -515,10 +538,10 @@ __device__ __forceinline__ float4 meshDistanceCertifiedT(const Res& r, uint32_t 
         uint32_t slot = --top, node = pending[slot];
         float limit = __fmul_rn(second, 1.00000095367431640625f);
         if (pendingDistance[slot] > limit) continue;
-        const float4* record = children + 4 * size_t(node - nodeBase);
-        float4 r0 = record[0], r1 = record[1];
+        const float4* record = r.meshChildren + 4 * size_t(node);
+        float4 r0 = __ldg(record), r1 = __ldg(record + 1);
         if (__float_as_uint(r0.w) != LEAF_MARK) {
-            float4 r2 = record[2], r3 = record[3];
+            float4 r2 = __ldg(record + 2), r3 = __ldg(record + 3);
             uint32_t a = node + 1, b = __float_as_uint(r0.w);
             float da = boxDistance(xyz(r0), xyz(r1), p), db = boxDistance(xyz(r2), xyz(r3), p);
             if (da < db) { uint32_t s = a; a = b; b = s; float ds = da; da = db; db = ds; }
@@ -533,77 +556,17 @@ __device__ __forceinline__ float4 meshDistanceCertifiedT(const Res& r, uint32_t 
             continue;
         }
         uint32_t first = __float_as_uint(r0.x), count = __float_as_uint(r0.y);
-        if constexpr (Warp) {
-            const uint32_t lane = threadIdx.x & 31u;
-            for (uint32_t k0 = 0; k0 < count; k0 += 32) {
-                uint32_t t = first + k0 + lane, feature = 0;
-                f3 q = mk(0.f, 0.f, 0.f);
-                float distance = 0.f;
-                if (k0 + lane < count) {
-                    q = closestTriangle(p, vertex(t, 0), vertex(t, 1), vertex(t, 2), feature);
-                    f3 dq = p - q;
-                    distance = dot(dq, dq);
-                }
-                uint32_t m = min(32u, count - k0);
-                for (uint32_t j = 0; j < m; ++j) {
-                    f3 qj = mk(__shfl_sync(0xffffffffu, q.x, j), __shfl_sync(0xffffffffu, q.y, j),
-                               __shfl_sync(0xffffffffu, q.z, j));
-                    take(node, first + k0 + j, qj, __shfl_sync(0xffffffffu, feature, j),
-                         __shfl_sync(0xffffffffu, distance, j));
-                }
-            }
-        } else {
-            for (uint32_t k = 0; k < count; ++k) {
-                uint32_t t = first + k, feature;
-                f3 q = closestTriangle(p, vertex(t, 0), vertex(t, 1), vertex(t, 2), feature);
-                f3 dq = p - q;
-                take(node, t, q, feature, dot(dq, dq));
-            }
+        for (uint32_t k = 0; k < count; ++k) {
+            uint32_t t = first + k, feature;
+            f3 q = closestTriangle(p, vertex(t, 0), vertex(t, 1), vertex(t, 2), feature);
+            f3 dq = p - q;
+            take(node, t, q, feature, dot(dq, dq));
         }
     }
     triangle = found ? (nearestNormal / 7) | (partner << 30) : 0xFFFFFFFFu;
     tie = found ? tied : EMPTY;
     gap = found ? __fsub_rn(__fsqrt_rn(second), __fsqrt_rn(best)) : 0.f;
     return distanceResult(r, p, best, nearest, nearestNormal, found, false);
-}
-__device__ __forceinline__ float4 meshDistanceCertified(const Res& r, uint32_t shape, f3 p, uint32_t seed, float reach,
-                                                        uint32_t& triangle, uint32_t& tie, float& gap) {
-    return meshDistanceCertifiedT<false>(r, shape, p, seed, reach, triangle, tie, gap, r.meshChildren, 0u,
-                                         r.meshTriangles, 0u);
-}
-// The walk's result when the certified triangle (and its same-leaf partner,
-// encoded as by meshDistanceCertified, and its tie of another leaf) are
-// known to be nearer than every other: the same closest point, squared
-// distance and feature the walk records -- the partner's only where it is
-// strictly nearer, as the leaf's triangles are taken in order.  With a tie
-// (EMPTY: none) the result stands only where the tie gives the same result
-// bit for bit (the walk may reach either leaf first); `same` is cleared
-// otherwise, and the caller walks.
-// `a`, `b`, `c` are the certified triangle's vertices (loaded by the caller).
-__device__ __forceinline__ float4 meshDistanceAt(const Res& r, f3 p, uint32_t certified, uint32_t tie, float4 a,
-                                                 float4 b, float4 c, bool& same) {
-    uint32_t triangle = certified & 0x3FFFFFFFu, partner = certified >> 30, feature;
-    f3 q = closestTriangle(p, xyz(a), xyz(b), xyz(c), feature);
-    f3 dq = p - q;
-    float best = dot(dq, dq);
-    uint32_t normal = 7 * triangle + feature;
-    if (partner != 0) {
-        uint32_t other = triangle + partner, otherFeature;
-        f3 q2 = closestTriangle(p, xyz(__ldg(&r.meshTriangles[3 * other])), xyz(__ldg(&r.meshTriangles[3 * other + 1])),
-                                xyz(__ldg(&r.meshTriangles[3 * other + 2])), otherFeature);
-        f3 dq2 = p - q2;
-        float d2 = dot(dq2, dq2);
-        if (d2 < best) { best = d2; q = q2; normal = 7 * other + otherFeature; }
-    }
-    same = true;
-    if (tie != EMPTY) {
-        uint32_t tieFeature;
-        f3 q3 = closestTriangle(p, xyz(__ldg(&r.meshTriangles[3 * tie])), xyz(__ldg(&r.meshTriangles[3 * tie + 1])),
-                                xyz(__ldg(&r.meshTriangles[3 * tie + 2])), tieFeature);
-        f3 dq3 = p - q3;
-        same = __float_as_uint(dot(dq3, dq3)) == __float_as_uint(best) && sameResult(r, q3, 7 * tie + tieFeature, q, normal);
-    }
-    return distanceResult(r, p, best, q, normal, true, false);
 }
 // solver.slang:259-272.  With `grow` > 0 the root box and every hull plane
 // are moved out by that distance (unit normals): the test then admits every
@@ -791,24 +754,218 @@ __device__ __forceinline__ uint32_t gridCell(const Res& r, uint32_t shape, f3 lo
         return 0xFFFFFFFFu;
     return (uint32_t(gz) * GRID + uint32_t(gy)) * GRID + uint32_t(gx);
 }
-// Walk-order bucket of a node at `local` against `shape`: the shape, then
-// the coarse cell (WALK_CELLS per axis over the grid box, clamped).  Nodes
-// of one bucket take similar paths through the shape's BVH.
-__device__ __forceinline__ uint32_t walkBucket(const Res& r, uint32_t shape, f3 local) {
-    float4 info = __ldg(&r.distanceGridInfo[shape]);
-    float inv = __fdiv_rn(float(WALK_CELLS), __fmul_rn(info.w, float(GRID)));
-    float g[3] = {__fmul_rn(__fsub_rn(local.x, info.x), inv), __fmul_rn(__fsub_rn(local.y, info.y), inv),
-                  __fmul_rn(__fsub_rn(local.z, info.z), inv)};
-    uint32_t k[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        k[a] = g[a] >= float(WALK_CELLS - 1) ? WALK_CELLS - 1 : (g[a] >= 1.0f ? uint32_t(g[a]) : 0u);
-    return shape * WALK_BUCKETS + (k[2] * WALK_CELLS + k[1]) * WALK_CELLS + k[0];
-}
 __device__ __forceinline__ float distanceBound(const Res& r, uint32_t shape, f3 local) {
     uint32_t cell = gridCell(r, shape, local);
     if (cell == 0xFFFFFFFFu) return -1e30f;
     return __ldg(&r.distanceGrid[size_t(shape) * GRID * GRID * GRID + cell]);
+}
+// Triangle list of a grid cell, 256 bytes: word 0 the limit L and word 1 the
+// distance d1 of the nearest triangle, both from the cell centre (floats);
+// words 2-49 the triangles nearer to the centre than L, nearest first
+// (EMPTY-padded); words 50-61 a byte each: the distance beyond d1 in steps
+// of CELL_REACH h / 255, rounded down.  L is d1 + CELL_REACH h, or less
+// where more than CELL_TRIANGLES are nearer: every triangle not listed lies
+// at least L from the centre.  1.9 h covers twice the half diagonal
+// (2 x 0.866 h) of the cell, within which the list holds the nearest triangle
+// of every point of the cell, and 0.17 h beyond it for the gap of a
+// certificate.  48 places: with 24, 0.2% of the queries of the 5,120-triangle
+// shapes met a truncated list that could not decide.
+constexpr uint32_t CELL_TRIANGLES = 48, CELL_WORDS = 64, CELL_STEPS = 2 + CELL_TRIANGLES;
+constexpr float CELL_REACH = 1.9f;
+__device__ __forceinline__ float cellStep(float h) { return __fmul_rn(h, CELL_REACH / 255.0f); }
+// The grid cell nearest to `local` (clamped to the grid), and its centre.
+__device__ __forceinline__ uint32_t nearestCell(float4 info, f3 local, f3& centre) {
+    float inv = __fdiv_rn(1.0f, info.w);
+    float g[3] = {__fmul_rn(__fsub_rn(local.x, info.x), inv), __fmul_rn(__fsub_rn(local.y, info.y), inv),
+                  __fmul_rn(__fsub_rn(local.z, info.z), inv)};
+    uint32_t k[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) k[a] = g[a] >= float(GRID - 1) ? GRID - 1 : (g[a] >= 1.0f ? uint32_t(g[a]) : 0u);
+    centre = xyz(info) + mk(__fmul_rn(float(k[0]) + 0.5f, info.w), __fmul_rn(float(k[1]) + 0.5f, info.w),
+                            __fmul_rn(float(k[2]) + 0.5f, info.w));
+    return (k[2] * GRID + k[1]) * GRID + k[0];
+}
+// Rounding slack of a triangle distance at p (see k_nodeQuery).
+__device__ __forceinline__ float distanceSlack(f3 p) {
+    return __fmul_rn(4e-6f, __fadd_rn(1.0f, __fadd_rn(__fadd_rn(fabsf(p.x), fabsf(p.y)), fabsf(p.z))));
+}
+// Whether the walk from p reaches BVH leaf `first` before leaf `second`:
+// decided where their paths part, by the two children's box distances (the
+// nearer child is taken first, the second child on ties).
+__device__ __forceinline__ bool leafVisitedFirst(const Res& r, uint32_t shape, f3 p, uint32_t first, uint32_t second) {
+    uint32_t node = __ldg(&r.meshRoots[shape].x);
+    for (uint32_t depth = 0; depth < 32; ++depth) {
+        const float4* record = r.meshChildren + 4 * size_t(node);
+        uint32_t b = __float_as_uint(__ldg(&record[0].w));
+        if (b == LEAF_MARK) break;  // one leaf: not reached for two
+        bool inB = first >= b;
+        if (inB == (second >= b)) {
+            node = inB ? b : node + 1;
+            continue;
+        }
+        float da = boxDistance(xyz(__ldg(&record[0])), xyz(__ldg(&record[1])), p);
+        float db = boxDistance(xyz(__ldg(&record[2])), xyz(__ldg(&record[3])), p);
+        return inB ? !(da < db) : da < db;
+    }
+    return true;
+}
+// The smallest computed distance over a set of triangles taken one at a time,
+// with the triangle a walk over the whole shape records for it: on exact
+// ties the first the walk reaches (the earlier triangle of one leaf, the
+// leaf visited first otherwise), which matters only where the results
+// differ.  `undecided`: a tie among three or more with different results, not
+// ordered here; with `Ordered` every tie is ordered (the paths through the
+// BVH are compared even where the results agree).
+struct NearestTriangle {
+    float best;
+    f3 point;
+    uint32_t normal, triangle;
+    bool shared, undecided;
+};
+template <bool Ordered = false>
+__device__ __forceinline__ float considerTriangle(const Res& r, uint32_t shape, f3 p, uint32_t t, NearestTriangle& n) {
+    uint32_t feature;
+    f3 q = closestTriangle(p, xyz(__ldg(&r.meshTriangles[3 * t])), xyz(__ldg(&r.meshTriangles[3 * t + 1])),
+                           xyz(__ldg(&r.meshTriangles[3 * t + 2])), feature);
+    f3 dq = p - q;
+    float d = dot(dq, dq);
+    bool take = d < n.best;
+    if (take) {
+        n.shared = n.undecided = false;
+    } else if (d == n.best) {
+        if (!Ordered && sameResult(r, q, 7 * t + feature, n.point, n.normal)) {
+            n.shared = true;
+        } else {
+            // With another triangle sharing the recorded result, the order
+            // of all three would decide.
+            n.undecided |= n.shared;
+            uint32_t leaf = __ldg(&r.triangleLeaf[t]), other = __ldg(&r.triangleLeaf[n.triangle]);
+            take = leaf == other ? t < n.triangle : leafVisitedFirst(r, shape, p, leaf, other);
+        }
+    }
+    if (take) {
+        n.best = d;
+        n.point = q;
+        n.normal = 7 * t + feature;
+        n.triangle = t;
+    }
+    return d;
+}
+// Certificate of a stored walk slot, 48 bytes: the point p0 it was taken at
+// and the gap g (floats); up to CERT_TRIANGLES triangles, those nearer to p0
+// than the nearest one's distance plus g, nearest first (EMPTY-padded); and a
+// byte each for the second to fifth, the distance beyond the nearest's in
+// units of g / 256, rounded down.  Every other triangle lies at least g
+// farther from p0 than the nearest.  Row 0 (p0, g), row 1 (three triangles,
+// the bytes), row 2 (four triangles).
+constexpr uint32_t CERT_TRIANGLES = 7, CERT_ROWS = 3;
+struct CertificateBuilder {
+    float d[CERT_TRIANGLES + 1];  // squared distances, ascending
+    uint32_t id[CERT_TRIANGLES + 1];
+    __device__ __forceinline__ CertificateBuilder() {
+#pragma unroll
+        for (uint32_t k = 0; k <= CERT_TRIANGLES; ++k) { d[k] = 1e30f; id[k] = EMPTY; }
+    }
+    __device__ __forceinline__ void add(float distance, uint32_t t) {
+#pragma unroll
+        for (uint32_t k = 0; k <= CERT_TRIANGLES; ++k) {
+            bool before = distance < d[k];
+            float od = d[k];
+            uint32_t oi = id[k];
+            d[k] = before ? distance : od;
+            id[k] = before ? t : oi;
+            distance = before ? od : distance;
+            t = before ? oi : t;
+        }
+    }
+    // `gap`: no triangle but those added lies nearer than the nearest plus it.
+    __device__ __forceinline__ void write(uint4* record, f3 p, float gap) const {
+        float root = __fsqrt_rn(d[0]);
+        gap = fminf(gap, __fsub_rn(__fsqrt_rn(d[CERT_TRIANGLES]), root));
+        uint32_t ids[CERT_TRIANGLES], bytes = 0;
+        float scale = gap > 0.0f ? __fdiv_rn(255.99f, gap) : 0.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < CERT_TRIANGLES; ++k) {
+            float beyond = __fsub_rn(__fsqrt_rn(d[k]), root);
+            ids[k] = k == 0 || beyond < gap ? id[k] : EMPTY;
+            if (k >= 1 && k <= 4) bytes |= uint32_t(fminf(__fmul_rn(beyond, scale), 255.0f)) << (8 * (k - 1));
+        }
+        record[0] = make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), __float_as_uint(gap));
+        record[1] = make_uint4(ids[0], ids[1], ids[2], bytes);
+        record[2] = make_uint4(ids[3], ids[4], ids[5], ids[6]);
+    }
+};
+// The query at p from a slot's certificate: false where it lapsed (or the
+// recorded triangle is undecided).  Listed triangles are evaluated until the
+// next lies farther than the motion since p0 could make up for: the rest
+// stays strictly farther than the nearest, and the smallest computed distance
+// among the evaluated ones is what the walk records.
+__device__ __forceinline__ bool certificateQuery(const Res& r, const uint4* record, uint32_t shape, f3 p, float4& f) {
+    uint4 r0 = record[0], r1 = record[1];
+    f3 p0 = mk(__uint_as_float(r0.x), __uint_as_float(r0.y), __uint_as_float(r0.z));
+    float gap = __uint_as_float(r0.w);
+    float need = __fadd_rn(__fmul_rn(2.002f, length(p - p0)), distanceSlack(p));
+    if (!(need < gap)) return false;
+    NearestTriangle n{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+    uint32_t t = r1.x;
+    const float unit = __fmul_rn(gap, 1.0f / 256.0f);
+    for (uint32_t k = 0;;) {
+        considerTriangle(r, shape, p, t, n);
+        if (++k >= CERT_TRIANGLES) break;
+        t = k == 1 ? r1.y : (k == 2 ? r1.z : reinterpret_cast<const uint32_t*>(record + 2)[k - 3]);
+        float beyond = __fmul_rn(float((r1.w >> (8 * (min(k, 4u) - 1))) & 255u), unit);
+        if (t == EMPTY || beyond > need) break;
+    }
+    if (n.undecided) return false;
+    f = distanceResult(r, p, n.best, n.point, n.normal, true, false);
+    return true;
+}
+// The certifying walk's result from the triangle list of the cell nearest to
+// p, without a walk: the listed triangles are evaluated nearest first (from
+// the cell centre) until the next one's lower bound -- its centre distance
+// less |p - centre| -- passes the best distance by `reach`.  Every triangle
+// not evaluated then lies at least `bound` away, and while bound exceeds the
+// best distance by more than the rounding slack, the smallest computed
+// distance among the evaluated ones is the smallest of all: the triangle the
+// walk records.  Writes the slot's new certificate.  False where the list
+// cannot decide (a truncated list).
+__device__ __forceinline__ bool cellQuery(const Res& r, uint32_t shape, f3 p, float reach, uint4* record, float4& f) {
+    float4 info = __ldg(&r.distanceGridInfo[shape]);
+    f3 centre;
+    uint32_t cell = nearestCell(info, p, centre);
+    const uint32_t* words = r.cellLists + (size_t(shape) * GRID * GRID * GRID + cell) * CELL_WORDS;
+    uint4 head = __ldg(reinterpret_cast<const uint4*>(words));
+    float limit = __uint_as_float(head.x), d1 = __uint_as_float(head.y), step = cellStep(info.w);
+    float off = __fadd_rn(__fmul_rn(1.00001f, length(p - centre)), 1e-6f);
+    float root = 1e15f, bound = __fsub_rn(limit, off);
+    NearestTriangle n{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+    CertificateBuilder list;
+    for (uint32_t k = 0; k < CELL_TRIANGLES; ++k) {
+        uint32_t t = k == 0 ? head.z : (k == 1 ? head.w : __ldg(words + 2 + k));
+        if (t == EMPTY) break;
+        uint32_t steps = (__ldg(words + CELL_STEPS + (k >> 2)) >> (8 * (k & 3u))) & 255u;
+        float lower = __fsub_rn(__fadd_rn(d1, __fmul_rn(0.99999f, __fmul_rn(float(steps), step))), off);
+        if (lower > __fadd_rn(root, reach)) {
+            bound = fminf(bound, lower);
+            break;
+        }
+        float d = considerTriangle(r, shape, p, t, n);
+        root = __fsqrt_rn(n.best);
+        list.add(d, t);
+    }
+    if (n.triangle == EMPTY || !(__fsub_rn(bound, root) > distanceSlack(p))) return false;
+    if (n.undecided) {
+        // Rare: the listed triangles again, every tie ordered.
+        n = NearestTriangle{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+        for (uint32_t k = 0; k < CELL_TRIANGLES; ++k) {
+            uint32_t t = __ldg(words + 2 + k);
+            if (t == EMPTY) break;
+            considerTriangle<true>(r, shape, p, t, n);
+        }
+    }
+    list.write(record, p, __fsub_rn(bound, root));
+    f = distanceResult(r, p, n.best, n.point, n.normal, true, false);
+    return true;
 }
 // The triangle nearest to the centre of the cell holding `local` (a seed
 // for meshDistance), or EMPTY outside the grid.
@@ -819,6 +976,28 @@ __device__ __forceinline__ uint32_t gridSeed(const Res& r, uint32_t shape, f3 lo
 }
 
 // ---------------------------------------------------------------- helpers
+// The step's hits of the active slots: a bit per slot (32 slots a word), the
+// hits of each block of 256 slots and of each group of 64 blocks.  The slots
+// are in contact order, so a hit's contact index is the hits before it: its
+// group's and block's predecessors' totals and the bits below it.
+constexpr uint32_t HIT_BLOCK = 256, HIT_GROUP = 64;
+struct SlotHits {
+    uint32_t *words, *blocks, *groups;
+};
+__host__ __device__ __forceinline__ uint64_t slotHitWords(uint32_t capacity) {
+    return uint64_t(HIT_BLOCK / 32) * (capacity / HIT_BLOCK + 1);
+}
+__host__ __device__ __forceinline__ uint64_t slotHitGroups(uint32_t capacity) {
+    return capacity / (HIT_BLOCK * HIT_GROUP) + 1;
+}
+// Words of the buffer: the bits, the blocks, the groups.
+__host__ __device__ __forceinline__ uint64_t slotHitSize(uint32_t capacity) {
+    return slotHitWords(capacity) + capacity / HIT_BLOCK + 1 + slotHitGroups(capacity);
+}
+__device__ __forceinline__ SlotHits slotHits(const Res& r, const Config& c) {
+    uint32_t* blocks = r.walkHits + slotHitWords(c.survivorCapacity);
+    return {r.walkHits, blocks, blocks + c.survivorCapacity / HIT_BLOCK + 1};
+}
 // Whether the exact-query list itself is stored with the filter results
 // (built with grown tests and ordered by target shape and coarse cell).  Not
 // with the learned culler, whose calibrated decision is taken every step.

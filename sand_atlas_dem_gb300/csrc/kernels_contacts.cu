@@ -536,7 +536,8 @@ __global__ void k_pairSetup(const __grid_constant__ Params P) {
     bool check = r.work[W_FILTER] == 0;
     for (uint32_t p = gtid(); p < n; p += gstride()) {
         uint2 ij = r.pairs[p];
-        f3 branch[2] = {centerBranch64(r, c, ij.x, ij.y), centerBranch64(r, c, ij.y, ij.x)};
+        f3 branch[2];
+        centerBranches64(r, c, ij.x, ij.y, branch[0], branch[1]);
         r.dpairBranch[2 * p] = w4(branch[0], 0.f);
         r.dpairBranch[2 * p + 1] = w4(branch[1], 0.f);
         if (check && filterStale(r, margin, p, ij, branch[0])) atomicOr(&r.work[W_FILTER], 1u);
@@ -593,8 +594,15 @@ __global__ void k_resetContacts(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0) return;
+    if (storedKeep(c)) {
+        const SlotHits hits = slotHits(r, c);
+        for (uint64_t g = threadIdx.x; g < slotHitGroups(c.survivorCapacity); g += blockDim.x) hits.groups[g] = 0;
+    }
+    if (threadIdx.x != 0) return;
     r.control[2] = 0;
     r.control[6] = 0;
+    r.work[W_SLOW] = 0;
+    r.work[W_LAPSED] = 0;
     bool on = c.filterMargin > 0.0f;
     uint32_t base = __float_as_uint(c.filterMargin);
     bool valid = r.work[W_FILTER_VALID] != 0 && r.work[W_FILTER_BASE] == base;
@@ -700,8 +708,6 @@ __global__ void k_leafCull(const __grid_constant__ Params P) {
     float grow = __fmul_rn(1.001f, margin);
     if (margin > 0.0f) {
         for (uint32_t g = gtid(); g < c.N; g += gstride()) r.filterRefRotation[g] = r.rotation[g];
-        if (storedKeep(c))
-            for (uint32_t b = gtid(); b <= c.shapes * WALK_BUCKETS; b += gstride()) r.walkBucketCount[b] = 0;
         if (gtid() == 0) {
             r.work[W_FILTER_VALID] = 0;
             r.work[W_FILTER_PAIRS] = r.control[1];
@@ -911,11 +917,6 @@ __global__ void __launch_bounds__(256) k_survivorPrefilter(const __grid_constant
         // cannot be a contact (the exact query would find phi > 0).
         if (keep && c.distanceGridEnabled && distanceBound(r, r.shapeId[dst], local) > grow) keep = false;
         r.survKeep[s] = keep ? 1u : 0u;
-        if (keep && stored) {
-            uint32_t bucket = walkBucket(r, r.shapeId[dst], local);
-            r.walkKey[s] = bucket;
-            atomicAdd(&r.walkBucketCount[bucket], 1u);
-        }
     }
 }
 // Distance-bound grid of every shape (built once per library): one thread per
@@ -944,6 +945,100 @@ __global__ void k_distanceGrid(const __grid_constant__ Params P) {
         float slack = __fmul_rn(1e-5f, __fadd_rn(1.0f, __fadd_rn(__fadd_rn(fabsf(centre.x), fabsf(centre.y)),
                                                                  fabsf(centre.z))));
         r.distanceGrid[t] = __fsub_rn(__fsub_rn(phi, reach), slack);
+    }
+}
+// The BVH leaf of each packed triangle (cellQuery breaks ties by it).
+__global__ void k_triangleLeaf(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    for (uint32_t shape = blockIdx.x; shape < P.c.shapes; shape += gridDim.x) {
+        uint4 nodes = __ldg(&r.meshRoots[shape]);
+        for (uint32_t node = nodes.x + threadIdx.x; node < nodes.y; node += blockDim.x) {
+            float4 head = __ldg(&r.meshChildren[4 * size_t(node)]);
+            if (__float_as_uint(head.w) != LEAF_MARK) continue;
+            uint32_t first = __float_as_uint(head.x), count = __float_as_uint(head.y);
+            for (uint32_t k = 0; k < count; ++k) r.triangleLeaf[first + k] = node;
+        }
+    }
+}
+// The triangle list of every grid cell (dem_device.cuh), once per library: a
+// thread per cell walks the BVH for the triangles within CELL_REACH h of its
+// nearest one's distance (k_distanceGrid's), keeping the CELL_TRIANGLES
+// nearest in order; a list that overflows lowers its limit to the nearest
+// triangle left out.
+__global__ void __launch_bounds__(256) k_cellLists(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    const uint32_t cells = GRID * GRID * GRID;
+    for (uint32_t i = gtid(); i < c.shapes * cells; i += gstride()) {
+        uint32_t shape = i / cells, cell = i % cells;
+        float4 info = r.distanceGridInfo[shape];
+        uint32_t gx = cell % GRID, gy = (cell / GRID) % GRID, gz = cell / (GRID * GRID);
+        f3 p = xyz(info) + mk(__fmul_rn(float(gx) + 0.5f, info.w), __fmul_rn(float(gy) + 0.5f, info.w),
+                              __fmul_rn(float(gz) + 0.5f, info.w));
+        uint32_t* out = r.cellLists + size_t(i) * CELL_WORDS;
+        uint32_t seed = r.distanceGridTriangle[i];
+        if (seed == EMPTY) {
+            for (uint32_t k = 0; k < CELL_WORDS; ++k) out[k] = k >= 2 && k < CELL_STEPS ? EMPTY : 0u;
+            continue;
+        }
+        auto squared = [&](uint32_t t) {
+            uint32_t feature;
+            f3 q = closestTriangle(p, xyz(__ldg(&r.meshTriangles[3 * t])), xyz(__ldg(&r.meshTriangles[3 * t + 1])),
+                                   xyz(__ldg(&r.meshTriangles[3 * t + 2])), feature);
+            f3 dq = p - q;
+            return dot(dq, dq);
+        };
+        float d1 = __fsqrt_rn(squared(seed));
+        float limitRoot = __fadd_rn(d1, __fmul_rn(CELL_REACH, info.w)), limit = __fmul_rn(limitRoot, limitRoot);
+        uint32_t ids[CELL_TRIANGLES], count = 0;
+        float far[CELL_TRIANGLES];
+        uint32_t pending[32], top = 1;
+        pending[0] = __ldg(&r.meshRoots[shape].x);
+        while (top > 0) {
+            uint32_t node = pending[--top];
+            const float4* record = r.meshChildren + 4 * size_t(node);
+            float4 r0 = __ldg(record), r1 = __ldg(record + 1);
+            if (__float_as_uint(r0.w) != LEAF_MARK) {
+                float4 r2 = __ldg(record + 2), r3 = __ldg(record + 3);
+                uint32_t a = node + 1, b = __float_as_uint(r0.w);
+                float da = boxDistance(xyz(r0), xyz(r1), p), db = boxDistance(xyz(r2), xyz(r3), p);
+                float reach = __fmul_rn(limit, 1.00000095367431640625f);
+                if (da < db) { uint32_t t = a; a = b; b = t; float d = da; da = db; db = d; }
+                if (top + 2 > 32) { fail(r, F_STACK); break; }
+                if (da <= reach) pending[top++] = a;
+                if (db <= reach) pending[top++] = b;
+                continue;
+            }
+            uint32_t first = __float_as_uint(r0.x), leaf = __float_as_uint(r0.y);
+            for (uint32_t t = first; t < first + leaf; ++t) {
+                float d = squared(t);
+                if (d >= limit) continue;
+                if (count == CELL_TRIANGLES) {
+                    // Full: the farthest of them all sets the limit.
+                    if (d >= far[CELL_TRIANGLES - 1]) { limit = fminf(limit, d); continue; }
+                    limit = fminf(limit, far[CELL_TRIANGLES - 1]);
+                    --count;
+                }
+                uint32_t k = count++;
+                for (; k > 0 && far[k - 1] > d; --k) { far[k] = far[k - 1]; ids[k] = ids[k - 1]; }
+                far[k] = d;
+                ids[k] = t;
+            }
+        }
+        float step = cellStep(info.w);
+        d1 = count ? __fsqrt_rn(far[0]) : d1;
+        out[0] = __float_as_uint(__fmul_rn(__fsqrt_rn(limit), 0.999999f));
+        out[1] = __float_as_uint(d1);
+        uint32_t packed = 0;
+        for (uint32_t k = 0; k < CELL_TRIANGLES; ++k) {
+            out[2 + k] = k < count ? ids[k] : EMPTY;
+            float beyond = k < count ? __fmul_rn(__fdiv_rn(__fsub_rn(__fsqrt_rn(far[k]), d1), step), 0.99999f) : 0.0f;
+            packed |= uint32_t(fminf(fmaxf(beyond, 0.0f), 255.0f)) << (8 * (k & 3u));
+            if ((k & 3u) == 3u) {
+                out[CELL_STEPS + (k >> 2)] = packed;
+                packed = 0;
+            }
+        }
     }
 }
 // Learned culler over the kept survivors, on the tensor cores (culler.cuh).
@@ -1036,11 +1131,12 @@ __global__ void __launch_bounds__(CULLER_ROWS) k_cullSurvivors(const __grid_cons
         atomicAdd(&r.cullerStats[1], culled);
     }
 }
-// Survivors kept for the exact query (their survivor indices): in survivor
-// order, or, when the list is stored with the filter results, grouped by
-// walk bucket (each bucket filled from its end; the order within a bucket
-// is immaterial: every walk is independent and its hit lands in its
-// survivor's slot).
+// Survivors kept for the exact query, in survivor order, which is contact
+// order (pair, direction, leaf, node): their indices, or, when the list is
+// stored with the filter results, a slot each with what its exact query reads
+// every step (one load instead of the survivor -> item -> pair -> sample
+// chain).  In this order a warp's slots share their two grains and branch,
+// and the step's contacts leave it in place (k_emitSlots).
 __global__ void k_walkList(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
@@ -1050,23 +1146,19 @@ __global__ void k_walkList(const __grid_constant__ Params P) {
     if (stored && gtid() == 0) r.work[W_DORMANT] = 0;  // a new list: no slot sleeps yet
     for (uint32_t s = gtid(); s < n; s += gstride()) {
         if (!r.survKeep[s]) continue;
-        if (stored) {
-            uint32_t bucket = r.walkKey[s];
-            uint32_t slot = r.walkBucketOffset[bucket] + atomicSub(&r.walkBucketCount[bucket], 1u) - 1u;
+        uint32_t slot = r.keepOffset[s];
+        if (!stored) {
             r.walkList[slot] = s;
-            r.walkCertTriangle[slot] = make_uint2(EMPTY, EMPTY);
-            // The slot's node record: what its exact query reads every step
-            // (one load instead of the survivor -> item -> pair -> sample chain).
-            uint2 sv = r.survivors[s];
-            uint2 cd = r.candidates[sv.x];
-            uint2 ij = r.pairs[cd.x >> 1];
-            uint32_t src = (cd.x & 1) ? ij.y : ij.x, dst = (cd.x & 1) ? ij.x : ij.y;
-            uint32_t node = __ldg(&r.meshSampleIndices[__ldg(&r.meshClusterRanges[cd.y]).x + sv.y]);
-            r.walkNode[slot] = make_uint4(src, dst, cd.x, __ldg(&r.sampleInfo[r.shapeId[src]].x) + node);
-            r.walkItem[slot] = sv;
-        } else {
-            r.walkList[r.keepOffset[s]] = s;
+            continue;
         }
+        uint2 sv = r.survivors[s];
+        uint2 cd = r.candidates[sv.x];
+        uint2 ij = r.pairs[cd.x >> 1];
+        uint32_t src = (cd.x & 1) ? ij.y : ij.x, dst = (cd.x & 1) ? ij.x : ij.y;
+        uint32_t node = __ldg(&r.meshSampleIndices[__ldg(&r.meshClusterRanges[cd.y]).x + sv.y]);
+        r.walkNode[slot] = make_uint4(src, dst, cd.x, __ldg(&r.sampleInfo[r.shapeId[src]].x) + node);
+        r.walkState[slot] = EMPTY;
+        r.walkContact[slot] = EMPTY;
     }
 }
 // Survivor list in canonical (item, node slot) order.
@@ -1142,54 +1234,31 @@ __global__ void __launch_bounds__(256) k_nodeWalk(const __grid_constant__ Params
     }
 }
 // Exact queries of a stored list.  A stored list keeps its slots from step
-// to step, and each slot keeps a certificate: the nearest triangle T found by
-// a certifying walk at the point p0, and a gap g below which no other
-// triangle's distance lies above T's.  Distances are 1-Lipschitz in the
-// point, so while 2 |p - p0| + slack < g, T is still the unique nearest
-// triangle at p and the walk would record it with the values closestTriangle
-// gives for it: the step evaluates T alone (with its partner or tie, where it
-// has one).  The slack, 4e-6 (1 + |p|_1), covers the FP32 rounding of the
-// distances: with e the largest difference between a computed triangle
-// distance and the exact one (a few units in the last place of |p|, about
-// 3e-7 (1 + |p|) here), the other triangles stay strictly farther while
-// 2 |p - p0| + 4e = g; the slack is above 4e.  A dormant slot is skipped: its node cannot touch the target
-// before the stored results are built again.  The other slots are flagged
-// (survKeep, unused by a stored list while it is walked), listed in slot
-// order -- the walk-bucket order, so that a warp's walks stay coherent -- and
-// walked by k_nodeWalkSlow in full warps.
-__global__ void __launch_bounds__(256) k_nodeWalkKnown(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    if (r.control[0] != 0) return;
-    uint32_t n = min(r.work[W_KEPT], c.survivorCapacity);
-    for (uint32_t t = gtid(); t < n; t += gstride()) {
-        uint2 cert = r.walkCertTriangle[t];
-        uint32_t triangle = cert.x;
-        bool known = false;
-        if (triangle == DORMANT) {
-            known = true;
-        } else if (triangle != EMPTY) {
-            // Every load below depends only on the slot: they issue together.
-            uint32_t base = 3 * (triangle & 0x3FFFFFFFu);
-            float4 ta = __ldg(&r.meshTriangles[base]), tb = __ldg(&r.meshTriangles[base + 1]),
-                   tc = __ldg(&r.meshTriangles[base + 2]);
-            float4 cp = r.walkCertPoint[t];
-            WalkNode w = walkNode(r, t);
-            float slack = __fmul_rn(4e-6f, __fadd_rn(1.0f, __fadd_rn(__fadd_rn(fabsf(w.local.x), fabsf(w.local.y)),
-                                                                    fabsf(w.local.z))));
-            known = __fadd_rn(__fmul_rn(2.002f, length(w.local - xyz(cp))), slack) < cp.w;
-            if (known) {
-                float4 pd, na;
-                float4 f = meshDistanceAt(r, w.local, triangle, cert.y, ta, tb, tc, known);
-                if (known && nodeContactWith(r, c, w.rec.x, w.sp, w.bs, w.bd, w.qd, w.arm, f, pd, na)) {
-                    uint2 it = r.walkItem[t];
-                    recordHitAt(r, r.walkList[t], it.x, it.y, pd, na);
-                }
-            }
-        }
-        r.survKeep[t] = known ? 0u : 1u;
-    }
-}
+// to step, and each slot keeps a certificate: the triangles nearest to the
+// point p0 it was taken at and a gap g, every other triangle lying at least g
+// farther from p0 than the nearest.  Distances are 1-Lipschitz in the point,
+// so while 2 |p - p0| + slack < g the triangle the walk would record at p is
+// among the listed ones: the step evaluates those (one for most slots; the
+// faces of an edge or a vertex where that is the nearest feature) and takes
+// the smallest distance, as the walk does (considerTriangle).  The slack,
+// 4e-6 (1 + |p|_1), covers the FP32 rounding of the distances: with e the
+// largest difference between a computed triangle distance and the exact one
+// (a few units in the last place of |p|, about 3e-7 (1 + |p|) here), the
+// other triangles stay strictly farther while 2 |p - p0| + 4e < g; the slack
+// is above 4e.  Slots whose certificate lapsed and new slots are listed
+// (in blocks of consecutive slots: the walk-bucket order, so that a warp's
+// work stays coherent) and answered and certified again from their grid
+// cell's triangle list in a kernel of their own, in full warps
+// (k_nodeCertify); what a list cannot decide is walked (k_nodeWalkSlow).
+// Bound by the latency of dependent loads (under 30% of issue slots used),
+// so: few of them, and many warps.  One triangle a certificate left 2% of a
+// resting packing's slots and 15 to 25% of a relaxing one's to BVH walks every
+// step, whose chains of dependent node loads were the step's critical path;
+// with the faces of edges and vertices in the certificate, cell lists for the
+// lapsed ones and the fused emit and law below, a step went from 185 to 120 us
+// (10,000 grains at rest), 640 to 361 (50,000) and 1,848 to 914 (15,625
+// relaxing, 3.3 M live slots).
+//
 // Dormant slots.  Until the next build, the motion check of k_pairSetup
 // bounds chord_i r_i + |d branch| + chord_j r_j by m s_j (chord: of a
 // grain's rotation since the build; r: bounding radius; s: scale), so a node
@@ -1198,247 +1267,273 @@ __global__ void __launch_bounds__(256) k_nodeWalkKnown(const __grid_constant__ P
 // a node at distance |v| from the target's centre now lies within
 // m max(1, |v| / r_j) of it.  A node farther outside than the sum (times
 // 1.001, plus the distance rounding slack) cannot touch the target before
-// the next build, and its slot sleeps.
-// One slot's certifying walk (by its warp when `Warp`; lane 0 records).
-template <bool Warp>
-__device__ __forceinline__ void certifySlot(const Res& r, const Config& c, uint32_t t, float margin, float reach,
-                                            const float4* children, uint32_t nodeBase, const float4* triangles,
-                                            uint32_t triangleBase) {
-    WalkNode w = walkNode(r, t);
-    uint32_t shape = r.shapeId[w.rec.y], triangle, tie;
-    float gap;
-    float4 f = meshDistanceCertifiedT<Warp>(r, shape, w.local, gridSeed(r, shape, w.local), reach, triangle, tie, gap,
-                                            children, nodeBase, triangles, triangleBase);
-    if (Warp && laneId() != 0) return;
+// the next build, and its slot sleeps: it is skipped with one 8-byte load.
+__device__ __forceinline__ bool fallsAsleep(const WalkNode& w, float phi, float margin) {
     float slack = __fmul_rn(2e-5f, __fadd_rn(1.0f, __fadd_rn(__fadd_rn(fabsf(w.local.x), fabsf(w.local.y)),
                                                              fabsf(w.local.z))));
     float reachNow = fmaxf(1.0f, __fdiv_rn(__fmul_rn(length(w.local), w.bd.x), w.bd.z));
     float sleep = __fmul_rn(__fmul_rn(1.001f, margin), __fadd_rn(1.0f, reachNow));
-    bool dormant = triangle != EMPTY && f.w > __fadd_rn(sleep, slack);
+    return phi > __fadd_rn(sleep, slack);
+}
+__device__ __forceinline__ float certificateReach(float margin) { return __fadd_rn(__fmul_rn(2.01f, margin), 1e-4f); }
+// Appends the block's flagged threads' values to a list, in thread order
+// (called by every thread of a 256-thread block): one atomic per block.
+__device__ __forceinline__ void appendBlock(bool flagged, uint32_t value, uint32_t* list, uint32_t* count) {
+    __shared__ uint32_t warpBase[8], blockBase;
+    if (!__syncthreads_or(flagged)) return;
+    const uint32_t warp = threadIdx.x >> 5;
+    uint32_t ballot = __ballot_sync(0xffffffffu, flagged);
+    if (laneId() == 0) warpBase[warp] = __popc(ballot);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t total = 0;
+        for (uint32_t k = 0; k < 8; ++k) {
+            uint32_t n = warpBase[k];
+            warpBase[k] = total;
+            total += n;
+        }
+        blockBase = atomicAdd(count, total);
+    }
+    __syncthreads();
+    if (flagged) list[blockBase + warpBase[warp] + __popc(ballot & lanesBelow())] = value;
+    __syncthreads();
+}
+// The slot's contact record, in its scratch slot; whether it is a contact.
+__device__ __forceinline__ bool recordSlot(const Res& r, const Config& c, uint32_t t, const WalkNode& w, float4 f) {
+    float4 pd, na;
+    if (!nodeContactWith(r, c, w.rec.x, w.sp, w.bs, w.bd, w.qd, w.arm, f, pd, na)) return false;
+    r.hitScratch[2 * size_t(t)] = pd;
+    r.hitScratch[2 * size_t(t) + 1] = na;
+    return true;
+}
+// A hit of active slot i found after k_nodeQuery.
+__device__ __forceinline__ void lateHit(const SlotHits& hits, uint32_t i) {
+    atomicOr(&hits.words[i >> 5], 1u << (i & 31u));
+    atomicAdd(&hits.blocks[i / HIT_BLOCK], 1u);
+    atomicAdd(&hits.groups[i / (HIT_BLOCK * HIT_GROUP)], 1u);
+}
+// The active slots whose certificates hold, a block of 256 at a time: their
+// hit bits and counts.  The others are listed in survKeep.  Only the slots
+// their build left awake are visited (walkActive): 185 of 449 thousand on a
+// dense packing of 10,000 grains, and warps full of them instead of a third
+// full.
+__global__ void __launch_bounds__(HIT_BLOCK, 4) k_nodeQuery(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    if (r.control[0] != 0) return;
+    const SlotHits hits = slotHits(r, c);
+    uint32_t n = min(r.work[W_ACTIVE], c.survivorCapacity);
+    for (uint32_t base = blockIdx.x * HIT_BLOCK; base < n; base += gridDim.x * HIT_BLOCK) {
+        uint32_t i = base + threadIdx.x, t = i < n ? r.walkActive[i] : 0u;
+        uint32_t state = i < n ? r.walkState[t] : DORMANT;
+        bool lapsed = state == EMPTY, hit = false;
+        if (state == CERTIFIED) {
+            WalkNode w = walkNode(r, t);
+            float4 f;
+            if (certificateQuery(r, r.walkCert + size_t(CERT_ROWS) * t, r.shapeId[w.rec.y], w.local, f))
+                hit = recordSlot(r, c, t, w, f);
+            else
+                lapsed = true;
+        }
+        uint32_t ballot = __ballot_sync(0xffffffffu, hit);
+        if (laneId() == 0) hits.words[i >> 5] = ballot;
+        uint32_t count = __syncthreads_count(hit);
+        if (threadIdx.x == 0) {
+            hits.blocks[base / HIT_BLOCK] = count;
+            if (count) atomicAdd(&hits.groups[base / (HIT_BLOCK * HIT_GROUP)], count);
+        }
+        appendBlock(lapsed, i, r.survKeep, &r.work[W_LAPSED]);
+    }
+}
+// A new list's slots, certified from their grid cells' triangle lists (in the
+// filter build): the slots that fall asleep at once are left out of the
+// active list (survKeep, then its scan).
+__global__ void __launch_bounds__(256) k_certifyBuild(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
+    uint32_t n = min(r.work[W_KEPT], c.survivorCapacity);
+    const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]), reach = certificateReach(margin);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gstride()) {
+        uint32_t t = base + threadIdx.x;
+        bool asleep = false;
+        if (t < n) {
+            if (c.cellListsEnabled) {
+                WalkNode w = walkNode(r, t);
+                float4 f;
+                if (cellQuery(r, r.shapeId[w.rec.y], w.local, reach, r.walkCert + size_t(CERT_ROWS) * t, f)) {
+                    asleep = fallsAsleep(w, f.w, margin);
+                    r.walkState[t] = asleep ? DORMANT : CERTIFIED;
+                }
+            }
+            r.survKeep[t] = asleep ? 0u : 1u;
+        }
+        uint32_t slept = __syncthreads_count(asleep);
+        if (threadIdx.x == 0 && slept) atomicAdd(&r.work[W_DORMANT], slept);
+    }
+}
+// The listed active slots, from their grid cells' triangle lists; the
+// undecided ones (all of them without the lists) are listed in walkKey.
+__global__ void __launch_bounds__(256) k_nodeCertify(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    if (r.control[0] != 0) return;
+    uint32_t n = min(r.work[W_LAPSED], c.survivorCapacity);
+    const SlotHits hits = slotHits(r, c);
+    const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]), reach = certificateReach(margin);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gstride()) {
+        uint32_t k = base + threadIdx.x, i = 0;
+        bool slow = false, asleep = false;
+        if (k < n) {
+            i = r.survKeep[k];
+            slow = true;
+            if (c.cellListsEnabled) {
+                uint32_t t = r.walkActive[i];
+                WalkNode w = walkNode(r, t);
+                float4 f;
+                if (cellQuery(r, r.shapeId[w.rec.y], w.local, reach, r.walkCert + size_t(CERT_ROWS) * t, f)) {
+                    slow = false;
+                    asleep = fallsAsleep(w, f.w, margin);
+                    r.walkState[t] = asleep ? DORMANT : CERTIFIED;
+                    if (recordSlot(r, c, t, w, f)) lateHit(hits, i);
+                }
+            }
+        }
+        uint32_t slept = __syncthreads_count(asleep);
+        if (threadIdx.x == 0 && slept) atomicAdd(&r.work[W_DORMANT], slept);
+        appendBlock(slow, i, r.walkKey, &r.work[W_SLOW]);
+    }
+}
+// Records a slot's query: its certificate from the triangles at the nearest
+// distance (`ids`, EMPTY-padded) with every other one farther by `gap`.
+__device__ __forceinline__ void certifySlot(const Res& r, const Config& c, uint32_t i, uint32_t t, const WalkNode& w,
+                                            float4 f, uint32_t id0, uint32_t id1, uint32_t id2, float gap,
+                                            float margin) {
+    bool found = id0 != EMPTY, dormant = found && fallsAsleep(w, f.w, margin);
     if (dormant) {
         // One count per group of lanes marking slots together.
         uint32_t group = __activemask();
         if (laneId() == uint32_t(__ffs(group) - 1)) atomicAdd(&r.work[W_DORMANT], uint32_t(__popc(group)));
     }
-    r.walkCertTriangle[t] = dormant ? make_uint2(DORMANT, EMPTY) : make_uint2(triangle, tie);
-    r.walkCertPoint[t] = w4(w.local, gap);
-    float4 pd, na;
-    if (nodeContactWith(r, c, w.rec.x, w.sp, w.bs, w.bd, w.qd, w.arm, f, pd, na)) {
-        uint2 it = r.walkItem[t];
-        recordHitAt(r, r.walkList[t], it.x, it.y, pd, na);
+    r.walkState[t] = dormant ? DORMANT : (found ? CERTIFIED : EMPTY);
+    if (found && !dormant) {
+        uint4* record = r.walkCert + size_t(CERT_ROWS) * t;
+        record[0] = make_uint4(__float_as_uint(w.local.x), __float_as_uint(w.local.y), __float_as_uint(w.local.z),
+                               __float_as_uint(gap));
+        record[1] = make_uint4(id0, id1, id2, 0u);
+        record[2] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
     }
+    if (recordSlot(r, c, t, w, f)) lateHit(slotHits(r, c), i);
 }
-// A certifying walk for each listed slot, recording its new certificate.
-// Few walks (up to two per warp of the grid) run a warp each; more run a
-// lane each, in 32-slot runs of the list (coherent walks) dealt to the
-// blocks in turn, so that either way they spread over every SM.  Only a
-// list longer than `above` is walked here (k_nodeWalkStaged takes the
-// shorter ones; 0: every list).
-__global__ void __launch_bounds__(256) k_nodeWalkSlow(const __grid_constant__ Params P, uint32_t above) {
+// One slot's query by a whole block, without a walk: the threads test the
+// boxes of every BVH leaf of the shape (independent loads: no chain of
+// dependent visits) and evaluate the triangles of those within the reach of
+// the seed; the smallest distance over the threads is the one a walk records,
+// exact ties ordered as it visits them.  A few such slots a step are on its
+// critical path: a warp's certifying walk of one took 40 to 140 us of
+// dependent loads (the nodes near a 5,120-triangle shape's medial axis).
+__device__ __forceinline__ void scanSlot(const Res& r, const Config& c, uint32_t i, float margin, float reach) {
+    __shared__ float warpBest[8], warpOther[8];
+    __shared__ uint32_t warpTriangle[8];
+    const uint32_t t = r.walkActive[i];
+    WalkNode w = walkNode(r, t);
+    const uint32_t shape = r.shapeId[w.rec.y];
+    f3 centre;
+    uint32_t cell = nearestCell(__ldg(&r.distanceGridInfo[shape]), w.local, centre);
+    uint32_t seed = __ldg(&r.distanceGridTriangle[size_t(shape) * GRID * GRID * GRID + cell]);
+    NearestTriangle n{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+    float cap = 1e30f;
+    if (seed != EMPTY) {
+        float root = __fadd_rn(__fsqrt_rn(considerTriangle(r, shape, w.local, seed, n)), reach);
+        cap = nextafterf(__fmul_rn(__fmul_rn(root, root), 1.0000019073486328f), 1e30f);
+        n.best = 1e30f;
+        n.triangle = EMPTY;
+    }
+    float other = cap;
+    uint4 nodes = __ldg(&r.meshRoots[shape]);
+#pragma unroll 2
+    for (uint32_t node = nodes.x + threadIdx.x; node < nodes.y; node += blockDim.x) {
+        uint4 link = __ldg(&r.meshLinks[node]);
+        float away = meshBoxDistance(r, node, w.local);
+        if (link.z == 0 || away > cap) continue;
+        for (uint32_t k = 0; k < link.z; ++k) {
+            float before = n.best;
+            float d = considerTriangle<true>(r, shape, w.local, link.y + k, n);
+            other = fminf(other, d < before ? before : d);
+        }
+    }
+    // The smallest, its triangle (the first a walk visits among ties, which
+    // lie in different leaves), and the smallest of the other distances.
+    auto merge = [&](float& best, uint32_t& triangle, float& rest, float theirs, uint32_t next, float theirRest) {
+        rest = fminf(rest, theirRest);
+        if (next == EMPTY) return;
+        if (triangle == EMPTY || theirs < best ||
+            (theirs == best && leafVisitedFirst(r, shape, w.local, __ldg(&r.triangleLeaf[next]),
+                                                __ldg(&r.triangleLeaf[triangle])))) {
+            if (triangle != EMPTY) rest = fminf(rest, best);
+            best = theirs;
+            triangle = next;
+        } else {
+            rest = fminf(rest, theirs);
+        }
+    };
+    float best = n.best;
+    uint32_t triangle = n.triangle;
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+        float theirs = __shfl_down_sync(0xffffffffu, best, o), theirRest = __shfl_down_sync(0xffffffffu, other, o);
+        uint32_t next = __shfl_down_sync(0xffffffffu, triangle, o);
+        if (laneId() < uint32_t(o)) merge(best, triangle, other, theirs, next, theirRest);
+    }
+    if (laneId() == 0) {
+        warpBest[threadIdx.x >> 5] = best;
+        warpTriangle[threadIdx.x >> 5] = triangle;
+        warpOther[threadIdx.x >> 5] = other;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (uint32_t k = 1; k < 8; ++k) merge(best, triangle, other, warpBest[k], warpTriangle[k], warpOther[k]);
+        NearestTriangle found{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+        if (triangle != EMPTY) considerTriangle(r, shape, w.local, triangle, found);
+        float gap = triangle != EMPTY ? __fsub_rn(__fsqrt_rn(other), __fsqrt_rn(best)) : 0.0f;
+        float4 f = distanceResult(r, w.local, triangle != EMPTY ? found.best : cap, found.point, found.normal,
+                                  triangle != EMPTY, false);
+        certifySlot(r, c, i, t, w, f, triangle, EMPTY, EMPTY, gap, margin);
+    }
+    __syncthreads();  // before the next slot writes the shared rows
+}
+// The slots the triangle lists left undecided (all that lapsed, without the
+// lists).  Few run a block each (scanSlot; up to four per block of the grid);
+// more run a lane each, a certifying walk in 32-slot runs of the list
+// (coherent walks) dealt to the blocks in turn, so that either way they
+// spread over every SM.
+__global__ void __launch_bounds__(256) k_nodeWalkSlow(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0) return;
     uint32_t n = min(r.work[W_SLOW], c.survivorCapacity);
-    if (n <= above && above != 0) return;
     if (gtid() == 0) r.work[W_CERTIFIED] += min(r.work[W_KEPT], c.survivorCapacity) - n;
     float margin = __uint_as_float(r.work[W_FILTER_MARGIN]);
-    float reach = __fadd_rn(__fmul_rn(2.01f, margin), 1e-4f);
+    float reach = certificateReach(margin);
     uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
-    if (n <= 2 * warps) {
-        for (uint32_t i = warp; i < n; i += warps)
-            certifySlot<true>(r, c, r.walkKey[i], margin, reach, r.meshChildren, 0u, r.meshTriangles, 0u);
-    } else {
-        for (uint32_t i = 32 * warp + laneId(); i < n; i += 32 * warps)
-            certifySlot<false>(r, c, r.walkKey[i], margin, reach, r.meshChildren, 0u, r.meshTriangles, 0u);
+    if (n <= 4 * gridDim.x) {
+        // A slot a list left undecided has many triangles at about its
+        // nearest distance: no certificate is worth the ones within reach.
+        if (c.cellListsEnabled) reach = 0.0f;
+        for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) scanSlot(r, c, r.walkKey[k], margin, reach);
+        return;
     }
-}
-// The same walks with each target shape's BVH node records staged in shared
-// memory.  The slow list is in walk-bucket order, so each shape's walks form
-// one run of it (from the scan of the flags at the shape's first bucket to
-// the scan at the next shape's); the runs are cut into units of one shape,
-// dealt to the CTAs in turn.  A CTA copies its unit's shape records (one
-// 64-byte record per node, up to STAGE_BYTES) into shared memory by bulk
-// asynchronous copies completing on an mbarrier -- once per change of shape
-// -- and walks the unit: a warp per walk when the step has few walks, a lane
-// per walk otherwise.  Internal node visits then read shared memory instead
-// of L2; leaves read their triangles from the library as before.  A shape
-// whose records exceed the stage is walked from the library by the same CTA.
-constexpr uint32_t STAGE_THREADS = 512;
-constexpr uint32_t STAGE_BYTES = 192u << 10;
-constexpr uint32_t STAGE_MAX_SHAPES = 4096;
-constexpr uint32_t STAGE_CHUNK = 16u << 10;
-// The staged kernel runs one CTA per SM and takes lists of up to two walks
-// per warp of its grid; longer lists go to k_nodeWalkSlow (a lane per walk,
-// full occupancy), which hides the walks' load latency better there.
-__device__ __forceinline__ uint32_t smemAddress(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ bool mbarrierWait(uint32_t bar, uint32_t parity) {
-    // Bounded: about 2^22 polls (far beyond a 192 KB copy), then give up.
-    for (uint32_t k = 0; k < (1u << 22); ++k) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__global__ void __launch_bounds__(STAGE_THREADS, 1) k_nodeWalkStaged(const __grid_constant__ Params P) {
-    extern __shared__ __align__(128) unsigned char stageMemory[];
-    float4* stage = reinterpret_cast<float4*>(stageMemory);
-    uint32_t* unitStart = reinterpret_cast<uint32_t*>(stageMemory + STAGE_BYTES);  // shapes + 1
-    __shared__ __align__(8) uint64_t barrier;
-    __shared__ uint32_t warpTotals[STAGE_THREADS / 32], carry, liveFlag, triangleFirst, triangleEnd;
-    const Res& r = P.r;
-    const Config& c = P.c;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warpId = tid >> 5, warps = STAGE_THREADS / 32;
-    if (tid == 0) liveFlag = r.control[0] == 0 ? 1u : 0u;
-    __syncthreads();
-    if (!liveFlag) return;  // block-uniform
-    uint32_t n = min(r.work[W_SLOW], c.survivorCapacity);
-    if (n > 2u * gridDim.x * warps) return;  // a long list: k_nodeWalkSlow walks it
-    if (blockIdx.x == 0 && tid == 0) r.work[W_CERTIFIED] += min(r.work[W_KEPT], c.survivorCapacity) - n;
-    if (n == 0) return;
-    float margin = __uint_as_float(r.work[W_FILTER_MARGIN]);
-    float reach = __fadd_rn(__fmul_rn(2.01f, margin), 1e-4f);
-    // Walks per unit: one or two per warp, so that the units spread over
-    // every CTA.
-    uint32_t per = n <= gridDim.x * warps ? warps : 2u * warps;
-    // Units per shape, scanned into unitStart (exclusive; unitStart[shapes] = total).
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < c.shapes; base += STAGE_THREADS) {
-        uint32_t s = base + tid, units = 0;
-        if (s < c.shapes) {
-            uint32_t lo = r.keepOffset[r.walkBucketOffset[s * WALK_BUCKETS]];
-            uint32_t hi = r.keepOffset[r.walkBucketOffset[(s + 1) * WALK_BUCKETS]];
-            units = (hi - lo + per - 1) / per;
-        }
-        uint32_t x = units;
-#pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += y;
-        }
-        if (lane == 31) warpTotals[warpId] = x;
-        __syncthreads();
-        if (warpId == 0) {
-            uint32_t t = lane < warps ? warpTotals[lane] : 0u;
-#pragma unroll
-            for (uint32_t d = 1; d < 32; d <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, t, d);
-                if (lane >= d) t += y;
-            }
-            if (lane < warps) warpTotals[lane] = t;  // inclusive over warps
-        }
-        __syncthreads();
-        uint32_t before = carry + (warpId ? warpTotals[warpId - 1] : 0u) + x - units;
-        if (s < c.shapes) unitStart[s] = before;
-        __syncthreads();
-        if (tid == 0) carry += warpTotals[warps - 1];
-        __syncthreads();
-    }
-    if (tid == 0) unitStart[c.shapes] = carry;
-    uint32_t bar = smemAddress(&barrier);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    uint32_t total = unitStart[c.shapes], phase = 0, staged = EMPTY, stagedFirst = 0;
-    bool stalled = false, trianglesStaged = false;  // the same on every thread
-    for (uint32_t u = blockIdx.x; u < total && !stalled; u += gridDim.x) {
-        // The unit's shape: the last s with unitStart[s] <= u.
-        uint32_t lo = 0, hi = c.shapes;
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (unitStart[mid] <= u) lo = mid; else hi = mid;
-        }
-        uint32_t shape = lo;
-        uint32_t first = r.keepOffset[r.walkBucketOffset[shape * WALK_BUCKETS]] + (u - unitStart[shape]) * per;
-        uint32_t last = min(first + per, r.keepOffset[r.walkBucketOffset[(shape + 1) * WALK_BUCKETS]]);
-        uint4 nodes = __ldg(&r.meshRoots[shape]);
-        uint32_t bytes = (nodes.y - nodes.x) * 64u;
-        bool fits = bytes <= STAGE_BYTES;
-        if (fits && staged != shape) {
-            __syncthreads();  // every warp is done with the staged shape
-            if (tid == 0) {
-                triangleFirst = EMPTY;
-                triangleEnd = 0;
-                // The async proxy overwrites what the generic proxy read.
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-                const char* from = reinterpret_cast<const char*>(r.meshChildren + 4 * size_t(nodes.x));
-                uint32_t to = smemAddress(stage);
-                for (uint32_t off = 0; off < bytes; off += STAGE_CHUNK) {
-                    uint32_t size = min(STAGE_CHUNK, bytes - off);
-                    asm volatile(
-                        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                        ::"r"(to + off), "l"(from + off), "r"(size), "r"(bar)
-                        : "memory");
-                }
-            }
-            if (!mbarrierWait(bar, phase)) {
-                fail(r, F_WAIT);
-                stalled = true;  // block-uniform only if every thread timed out: re-checked below
-            }
-            phase ^= 1u;
-            staged = shape;
-            // Every thread leaves together if any thread gave up.
-            stalled = __syncthreads_or(stalled);
-            if (stalled) break;
-            // The shape's triangles: the range its leaves reference (a
-            // reduction over the staged records), staged after the records
-            // when both fit.
-            for (uint32_t k = tid; k < nodes.y - nodes.x; k += STAGE_THREADS) {
-                float4 head = stage[4 * k];
-                if (__float_as_uint(head.w) == LEAF_MARK) {
-                    atomicMin(&triangleFirst, __float_as_uint(head.x));
-                    atomicMax(&triangleEnd, __float_as_uint(head.x) + __float_as_uint(head.y));
-                }
-            }
-            __syncthreads();
-            stagedFirst = triangleFirst;
-            uint32_t triangleBytes = triangleEnd > stagedFirst ? (triangleEnd - stagedFirst) * 48u : 0u;
-            trianglesStaged = triangleBytes != 0 && bytes + triangleBytes <= STAGE_BYTES;
-            if (trianglesStaged) {
-                if (tid == 0) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(triangleBytes)
-                                 : "memory");
-                    const char* from = reinterpret_cast<const char*>(r.meshTriangles + 3 * size_t(stagedFirst));
-                    uint32_t to = smemAddress(stage) + bytes;
-                    for (uint32_t off = 0; off < triangleBytes; off += STAGE_CHUNK) {
-                        uint32_t size = min(STAGE_CHUNK, triangleBytes - off);
-                        asm volatile(
-                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                            ::"r"(to + off), "l"(from + off), "r"(size), "r"(bar)
-                            : "memory");
-                    }
-                }
-                if (!mbarrierWait(bar, phase)) {
-                    fail(r, F_WAIT);
-                    stalled = true;
-                }
-                phase ^= 1u;
-                stalled = __syncthreads_or(stalled);
-                if (stalled) break;
-            }
-        }
-        const float4* children = fits ? stage : r.meshChildren;
-        uint32_t base = fits ? nodes.x : 0u;
-        bool local = fits && trianglesStaged;
-        const float4* triangles = local ? stage + 4 * size_t(nodes.y - nodes.x) : r.meshTriangles;
-        uint32_t triangleBase = local ? stagedFirst : 0u;
-        for (uint32_t i = first + warpId; i < last; i += warps)
-            certifySlot<true>(r, c, r.walkKey[i], margin, reach, children, base, triangles, triangleBase);
-    }
-    if (stalled && tid == 0) {
-        // A copy may still be landing: wait for it (bounded) before the
-        // shared memory is released.
-        mbarrierWait(bar, phase ^ 1u);
+    for (uint32_t k = 32 * warp + laneId(); k < n; k += 32 * warps) {
+        uint32_t i = r.walkKey[k], t = r.walkActive[i], triangle, tie;
+        float gap;
+        WalkNode w = walkNode(r, t);
+        uint32_t shape = r.shapeId[w.rec.y];
+        float4 f = meshDistanceCertified(r, shape, w.local, gridSeed(r, shape, w.local), reach, triangle, tie, gap);
+        // The triangle with its same-leaf partner and its tie, all at its
+        // distance; every other one is farther by the gap.
+        uint32_t at = triangle & 0x3FFFFFFFu, partner = triangle >> 30;
+        if (triangle == EMPTY) at = EMPTY, partner = 0;
+        certifySlot(r, c, i, t, w, f, at, partner ? at + partner : tie, partner ? tie : EMPTY, gap, margin);
     }
 }
 // L2 prefetch, first in a step, of what the step's exact queries read
@@ -1456,12 +1551,12 @@ __global__ void k_prefetch(const __grid_constant__ Params P) {
     const Config& c = P.c;
     constexpr uint32_t CHUNK = 16u << 10;
     uint32_t kept = storedKeep(c) ? min(r.work[W_KEPT], c.survivorCapacity) : 0u;
-    const void* base[9] = {r.meshChildren, r.meshTriangles, r.meshNormals, r.sample, r.walkCertTriangle,
-                           r.walkCertPoint, r.walkNode, r.walkItem, r.walkList};
-    uint64_t size[9] = {16ull * c.library16[0], 16ull * c.library16[1], 16ull * c.library16[2],
-                        16ull * c.library16[3], 8ull * kept, 16ull * kept, 16ull * kept, 8ull * kept, 4ull * kept};
+    const void* base[8] = {r.meshTriangles, r.meshNormals, r.sample, r.walkActive, r.walkState,
+                           r.walkCert, r.walkNode, r.walkContact};
+    uint64_t size[8] = {16ull * c.library16[1], 16ull * c.library16[2], 16ull * c.library16[3], 4ull * kept,
+                        4ull * kept, 16ull * CERT_ROWS * kept, 16ull * kept, 4ull * kept};
     uint32_t chunk = gtid();
-    for (int k = 0; k < 9; ++k) {
+    for (int k = 0; k < 8; ++k) {
         uint64_t bytes = size[k] & ~uint64_t(15);
         uint64_t chunks = (bytes + CHUNK - 1) / CHUNK;
         for (; chunk < chunks; chunk += gstride()) {
@@ -1529,39 +1624,8 @@ __global__ void __launch_bounds__(256) k_nodeEmit(const __grid_constant__ Params
         }
     }
 }
-// The same contact records from a stored exact-query list, a thread per
-// stored slot instead of a warp per item: a slot whose node hit (its bit in
-// its item's hit mask) writes its record at its item's offset plus the
-// number of the item's hits at lower node slots -- the canonical place
-// k_nodeEmit gives it -- from the slot's own node record (source, target,
-// directed pair, packed sample) and its hit scratch.  Dormant slots never
-// hit.  The item masks are cleared by k_clearHits afterwards (a slot cannot
-// clear its item's mask while the item's other hits still read it).
-__global__ void k_clearHits(const __grid_constant__ Params P);
-__global__ void __launch_bounds__(256) k_emitSlots(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    if (r.control[0] != 0) return;
-    uint32_t n = min(r.work[W_KEPT], c.survivorCapacity);
-    for (uint32_t t = gtid(); t < n; t += gstride()) {
-        if (r.walkCertTriangle[t].x == DORMANT) continue;
-        uint2 it = r.walkItem[t];
-        uint2 m = r.candHitMask[it.x];
-        uint32_t word = it.y < WARP ? m.x : m.y, bit = 1u << (it.y & 31u);
-        if (!(word & bit)) continue;
-        uint32_t rank = (it.y < WARP ? 0u : __popc(m.x)) + __popc(word & (bit - 1u));
-        uint32_t slot = r.candHitOffset[it.x] + rank, from = r.walkList[t];
-        if (slot >= c.contactCapacity || from >= c.survivorCapacity) { fail(r, F_CONTACT); continue; }
-        uint4 rec = r.walkNode[t];
-        uint32_t node = rec.w - __ldg(&r.sampleInfo[r.shapeId[rec.x]].x);
-        r.meta[slot] = make_uint4(rec.x, rec.y, node, 0);
-        r.pointDepth[slot] = r.hitScratch[2 * from];
-        r.normalArea[slot] = r.hitScratch[2 * from + 1];
-        r.contactPair[slot] = rec.z >> 1;
-    }
-}
 // Per pair: first contact of the pair on the side being written, and counts.
-__device__ __forceinline__ void contactStart(const Params& P) {
+__global__ void k_contactStart(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
     uint32_t n = activePairs(r, c);
@@ -1580,21 +1644,6 @@ __device__ __forceinline__ void contactStart(const Params& P) {
         }
     }
 }
-__global__ void k_contactStart(const __grid_constant__ Params P) { contactStart(P); }
-// Hit masks and counts of every item back to zero for the next step (also
-// after a failed step, whose walks may have set bits), and the per-pair
-// contact starts (k_contactStart) in the same launch.
-__global__ void k_clearHits(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    uint32_t n = min(r.work[W_CANDIDATES], c.candidateCapacity);
-    for (uint32_t i = gtid(); i < n; i += gstride()) {
-        r.candHitMask[i] = make_uint2(0u, 0u);
-        r.candHitCount[i] = 0;
-    }
-    contactStart(P);
-}
-
 // ------------------------------------------------------------ SDF geometry
 // solver.slang:188-200: trilinear signed distance and gradient from the
 // target shape's grid, in the FP32 order of the reference's generated CPU
@@ -2071,7 +2120,45 @@ __global__ void k_resolveWalls(const __grid_constant__ Params P) {
     uint32_t n = activeContacts(r, c);
     for (uint32_t id = min(r.work[W_WALL_BASE], n) + gtid(); id < n; id += gstride()) resolveWall(r, c, id, r.meta[id]);
 }
-// solver.slang:702-749 (particle-particle contacts)
+// solver.slang:702-749: the law of grain-grain contact `id` (source i, target
+// j, normal and area, arm and depth, branch), with the slip of its committed
+// slot `old` (EMPTY: none).  Returns whether it slides.
+__device__ __forceinline__ bool resolveGrain(const Res& r, const Config& c, uint32_t id, uint32_t i, uint32_t j,
+                                             float4 na, float4 pd, f3 branch, uint32_t old) {
+    f3 nrm = xyz(na), arm = xyz(pd);
+    float viscosity = c.normalViscosity;
+    f3 wi = viscosity > 0 ? xyz(r.forceOmega[i]) : omegaOf(r, i);
+    f3 wj = viscosity > 0 ? xyz(r.forceOmega[j]) : omegaOf(r, j);
+    f3 elastic = mk(0.f, 0.f, 0.f);
+    if (old != EMPTY)
+        elastic = transported(xyz(r.oldSlip[old]), xyz(r.oldNormal[old]), nrm,
+                              __fmul_rn(__fmul_rn(0.5f, dot(wi + wj, nrm)), c.dt));
+    f3 translation = viscosity > 0 ? xyz(r.forceVelocity[i]) - xyz(r.forceVelocity[j])
+                                   : xyz(r.velocity[i]) - xyz(r.velocity[j]);
+    f3 rv = ((translation - xyz(r.cell[3 * specimenOf(r, i) + 1]) * branch) + cross(wi, arm)) - cross(wj, arm - branch);
+    elastic = elastic + (rv - nrm * dot(rv, nrm)) * c.dt;
+    f3 trial = elastic;
+    float area = na.w, depth = pd.w;
+    float fn, lossPower;
+    normalResponse(depth, area, dot(rv, nrm), c.kn, viscosity, 0.5f, fn, lossPower);
+    r.normalLossPower[id] = lossPower;
+    float ktA = __fmul_rn(__fmul_rn(-0.5f, c.kt), area);
+    f3 ft = ktA * elastic;
+    float magnitude = length(ft);
+    bool sliding = magnitude > __fmul_rn(c.mu, fn) && magnitude > 0;
+    if (sliding) {
+        ft = ft * __fdiv_rn(__fmul_rn(c.mu, fn), magnitude);
+        elastic = (-ft) / __fmul_rn(__fmul_rn(0.5f, c.kt), area);
+    }
+    r.slip[id] = w4(elastic, mx(0.0f, -dot(ft, trial - elastic)));
+    float4 cf = w4(fn * nrm + ft,
+                   __fmul_rn(__fmul_rn(0.25f, area), __fadd_rn(__fmul_rn(__fmul_rn(c.kn, depth), depth),
+                                                               __fmul_rn(c.kt, dot(elastic, elastic)))));
+    r.contactForce[id] = cf;
+    if (!isfinite(cf.x) || !isfinite(cf.y) || !isfinite(cf.z) || !isfinite(cf.w) || !isfinite(lossPower))
+        fail(r, F_NONFINITE);
+    return sliding;
+}
 __global__ void k_resolve(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
@@ -2082,48 +2169,108 @@ __global__ void k_resolve(const __grid_constant__ Params P) {
     if (c.wallCount != 0) n = min(n, r.work[W_WALL_BASE]);
     for (uint32_t id = gtid(); id < n; id += gstride()) {
         uint4 key = r.meta[id];
-        uint32_t i = key.x, j = key.y;
-        f3 nrm = xyz(r.normalArea[id]);
-        float viscosity = c.normalViscosity;
-        f3 wi = viscosity > 0 ? xyz(r.forceOmega[i]) : omegaOf(r, i);
-        f3 wj = viscosity > 0 ? xyz(r.forceOmega[j]) : omegaOf(r, j);
-        f3 elastic = mk(0.f, 0.f, 0.f);
-        if (c.historyStep != 0) {
-            uint32_t old = historySlot(r, c, i, j, key.z);
-            if (old != EMPTY)
-                elastic = transported(xyz(r.oldSlip[old]), xyz(r.oldNormal[old]), nrm,
-                                      __fmul_rn(__fmul_rn(0.5f, dot(wi + wj, nrm)), c.dt));
-        }
-        f3 arm = xyz(r.pointDepth[id]);
-        uint32_t p = r.contactPair[id];
-        f3 branch = xyz(r.dpairBranch[2 * p + (i > j ? 1 : 0)]);
-        f3 translation = viscosity > 0 ? xyz(r.forceVelocity[i]) - xyz(r.forceVelocity[j])
-                                       : xyz(r.velocity[i]) - xyz(r.velocity[j]);
-        f3 rv = ((translation - xyz(r.cell[3 * specimenOf(r, i) + 1]) * branch) + cross(wi, arm)) - cross(wj, arm - branch);
-        elastic = elastic + (rv - nrm * dot(rv, nrm)) * c.dt;
-        f3 trial = elastic;
-        float area = r.normalArea[id].w, depth = r.pointDepth[id].w;
-        float fn, lossPower;
-        normalResponse(depth, area, dot(rv, nrm), c.kn, viscosity, 0.5f, fn, lossPower);
-        r.normalLossPower[id] = lossPower;
-        float ktA = __fmul_rn(__fmul_rn(-0.5f, c.kt), area);
-        f3 ft = ktA * elastic;
-        float magnitude = length(ft);
-        if (magnitude > __fmul_rn(c.mu, fn) && magnitude > 0) {
-            ft = ft * __fdiv_rn(__fmul_rn(c.mu, fn), magnitude);
-            elastic = (-ft) / __fmul_rn(__fmul_rn(0.5f, c.kt), area);
+        uint32_t old = c.historyStep != 0 ? historySlot(r, c, key.x, key.y, key.z) : EMPTY;
+        f3 branch = xyz(r.dpairBranch[2 * r.contactPair[id] + (key.x > key.y ? 1 : 0)]);
+        if (resolveGrain(r, c, id, key.x, key.y, r.normalArea[id], r.pointDepth[id], branch, old))
             atomicAdd(&r.control[6], 1u);
-        }
-        r.slip[id] = w4(elastic, mx(0.0f, -dot(ft, trial - elastic)));
-        float4 cf = w4(fn * nrm + ft,
-                       __fmul_rn(__fmul_rn(0.25f, area), __fadd_rn(__fmul_rn(__fmul_rn(c.kn, depth), depth),
-                                                                   __fmul_rn(c.kt, dot(elastic, elastic)))));
-        r.contactForce[id] = cf;
-        if (!isfinite(cf.x) || !isfinite(cf.y) || !isfinite(cf.z) || !isfinite(cf.w) || !isfinite(lossPower))
-            fail(r, F_NONFINITE);
     }
 }
-
+// The contact records of a stored exact-query list, and with `Law` the
+// contact law of each in the same pass (the step; the named phases of a
+// dispatch run them apart).  The active slots are in contact order, so the
+// kernel is a stream compaction: a block of 256 slots adds up the hits of the
+// groups and blocks before it (at most a few hundred words), each thread the
+// bits below its own, and the slots that hit write their contacts in place,
+// consecutive threads to consecutive contacts.  The first slot of each pair
+// also writes the pair's first contact (for the pairs before it without
+// slots too).  A slot keeps the contact it became (walkContact): on the next
+// step that contact's committed key is its own, which spares the search of
+// the pair's committed run; where the key does not match (another step's
+// contacts were committed) or the slot was no contact, the search decides.
+template <bool Law>
+__global__ void __launch_bounds__(HIT_BLOCK) k_emitSlots(const __grid_constant__ Params P) {
+    __shared__ uint32_t warpSum[HIT_BLOCK / 32];
+    const Res& r = P.r;
+    const Config& c = P.c;
+    if (r.control[0] != 0) return;
+    const SlotHits hits = slotHits(r, c);
+    const uint32_t n = min(r.work[W_ACTIVE], c.survivorCapacity), pairs = activePairs(r, c);
+    const uint32_t lane = laneId(), warp = threadIdx.x >> 5;
+    if (n == 0) {
+        for (uint32_t p = gtid(); p <= pairs; p += gstride()) r.sideContactStart[p] = 0;
+        return;
+    }
+    // Contacts on the committed side: a hint must lie below them.
+    const uint32_t committed = Law && c.historyStep != 0 ? r.oldContactStart[r.oldPairOffsets[c.N]] : 0u;
+    for (uint32_t b = blockIdx.x; b * HIT_BLOCK < n; b += gridDim.x) {
+        const uint32_t group = b / HIT_GROUP;
+        uint32_t before = 0;
+        for (uint32_t k = threadIdx.x; k < group; k += HIT_BLOCK) before += hits.groups[k];
+        if (threadIdx.x < b % HIT_GROUP) before += hits.blocks[group * HIT_GROUP + threadIdx.x];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) warpSum[warp] = before;
+        __syncthreads();
+        uint32_t contact = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < HIT_BLOCK / 32; ++k) contact += warpSum[k];
+        const uint32_t* words = hits.words + b * (HIT_BLOCK / 32);
+        contact += __reduce_add_sync(0xffffffffu, lane < warp ? __popc(words[lane]) : 0u);
+        const uint32_t word = words[warp];
+        const bool hit = (word >> lane) & 1u;
+        contact += __popc(word & lanesBelow());
+        // This slot's contact index, or the next one's.
+        const uint32_t i = b * HIT_BLOCK + threadIdx.x;
+        const bool valid = i < n;
+        const uint32_t t = valid ? r.walkActive[i] : 0u;
+        const uint4 rec = valid ? r.walkNode[t] : make_uint4(0u, 0u, 2 * pairs, 0u);
+        const uint32_t pair = rec.z >> 1;
+        uint32_t from = __shfl_up_sync(0xffffffffu, pair, 1) + 1;
+        if (lane == 0) from = i == 0 ? 0u : (valid ? (r.walkNode[r.walkActive[i - 1]].z >> 1) + 1 : pairs);
+        // First contacts of the pairs up to this slot's; of the rest after the last slot.
+        uint32_t upTo = valid ? pair + 1 : from;
+        if (valid && upTo - from <= 4)
+            for (; from < upTo; ++from) r.sideContactStart[from] = contact;
+        const bool last = i == n - 1;
+        for (uint32_t wide = __ballot_sync(0xffffffffu, from < upTo || last); wide; wide &= wide - 1) {
+            uint32_t k = __ffs(wide) - 1, first = __shfl_sync(0xffffffffu, from, k), end = __shfl_sync(0xffffffffu, upTo, k);
+            uint32_t value = __shfl_sync(0xffffffffu, contact, k);
+            for (uint32_t q = first + lane; q < end; q += WARP) r.sideContactStart[q] = value;
+            if (__shfl_sync(0xffffffffu, uint32_t(last), k)) {
+                uint32_t total = value + __shfl_sync(0xffffffffu, uint32_t(hit), k);
+                for (uint32_t q = end + lane; q <= pairs; q += WARP) r.sideContactStart[q] = total;
+                if (lane == 0) {
+                    r.control[2] = total;
+                    if (total > c.contactCapacity) fail(r, F_CONTACT);
+                }
+            }
+        }
+        bool sliding = false;
+        if (hit && contact < c.contactCapacity) {
+            const float4 pd = r.hitScratch[2 * size_t(t)], na = r.hitScratch[2 * size_t(t) + 1];
+            const uint32_t node = rec.w - __ldg(&r.sampleInfo[r.shapeId[rec.x]].x);
+            r.meta[contact] = make_uint4(rec.x, rec.y, node, 0);
+            r.pointDepth[contact] = pd;
+            r.normalArea[contact] = na;
+            if (Law) {
+                uint32_t old = EMPTY;
+                if (c.historyStep != 0) {
+                    uint32_t hint = r.walkContact[t];
+                    if (hint < committed) {
+                        uint4 m = r.oldMeta[hint];
+                        if (m.x == rec.x && m.y == rec.y && m.z == node) old = hint;
+                    }
+                    if (old == EMPTY) old = historySlot(r, c, rec.x, rec.y, node);
+                }
+                sliding = resolveGrain(r, c, contact, rec.x, rec.y, na, pd, xyz(r.dpairBranch[rec.z]), old);
+            } else {
+                r.contactPair[contact] = pair;
+            }
+            r.walkContact[t] = contact;
+        }
+        uint32_t slides = __syncthreads_count(sliding);  // also before warpSum is written again
+        if (threadIdx.x == 0 && slides) atomicAdd(&r.control[6], slides);
+    }
+}
 // -------------------------------------------------------------------- gather
 // solver.slang:760-811, one warp per grain.  Contacts of grain g are taken in
 // the order the reference's linked lists hold them (descending contact id):
@@ -2231,6 +2378,8 @@ __global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Param
     uint32_t* we = window[threadIdx.x >> 5][3];
     float (*terms)[GATHER_STRIDE] = termRows[threadIdx.x >> 5];
     const uint32_t chain = laneId();
+    for (uint32_t p = gtid(); p < pairs; p += gstride())
+        r.contactCounts[p] = r.sideContactStart[p + 1] - r.sideContactStart[p];
     for (uint32_t id = warpGlobal(); id < c.N; id += warpStride()) {
         // This lane's chain: running value and compensation residual.
         float acc = 0.f, accLow = 0.f;
@@ -2440,7 +2589,7 @@ static void collectHead(const Params& P, cudaStream_t s) {
     const Res& r = P.r;
     const Config& c = P.c;
     uint32_t T = 256;
-    k_resetContacts<<<1, 1, 0, s>>>(P);
+    k_resetContacts<<<1, storedKeep(c) ? T : 1, 0, s>>>(P);
     k_pairSetup<<<grid(c.cullBlocksPerSM, 8), T, 0, s>>>(P);
     if (c.meshGeometry == 0) {
         k_sdfCount<<<grid(c.queryBlocksPerSM, 8), T, 0, s>>>(P);
@@ -2486,13 +2635,15 @@ static void collectFilter(const Params& P, cudaStream_t s) {
         k_cullPlace<<<g, 256, 0, s>>>(P);
         k_cullSurvivors<<<grid(0, 4), CULLER_ROWS, 0, s>>>(P);  // 4 x 64 TMEM columns per SM
     }
-    if (c.filterMargin > 0.0f && c.cullerEnabled == 0)
-        launch_step_scan(r, r.walkBucketCount, r.walkBucketOffset, ScanCount{nullptr, 0, 0, c.shapes * WALK_BUCKETS}, true,
-                    r.work + W_KEPT, r.work + W_FILTER, s);
-    else
-        launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_SURVIVORS, c.survivorCapacity, 1, 0}, true,
-                    r.work + W_KEPT, nullptr, s);
+    const bool stored = storedKeep(c);
+    launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_SURVIVORS, c.survivorCapacity, 1, 0}, true,
+                     r.work + W_KEPT, stored ? r.work + W_FILTER : nullptr, s);
     k_walkList<<<grid(c.contactBlocksPerSM, 8), 256, 0, s>>>(P);
+    if (stored) {
+        k_certifyBuild<<<grid(c.walkBlocksPerSM, 8), 256, 0, s>>>(P);
+        launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_KEPT, c.survivorCapacity, 1, 0}, true,
+                         r.work + W_ACTIVE, r.work + W_FILTER, s, r.walkActive);
+    }
 }
 // The exact queries.
 static void collectWalk(const Params& P, cudaStream_t s) {
@@ -2502,27 +2653,9 @@ static void collectWalk(const Params& P, cudaStream_t s) {
         k_sdfEmit<<<grid(c.queryBlocksPerSM, 8), 256, 0, s>>>(P);
     } else if (c.filterMargin > 0.0f && c.cullerEnabled == 0) {
         uint32_t g = grid(c.walkBlocksPerSM, 8);
-        k_nodeWalkKnown<<<g, 256, 0, s>>>(P);
-        // The flags' scan also lists the flagged slots in slot order (the
-        // walk-bucket order) into walkKey.
-        launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_KEPT, c.survivorCapacity, 1, 0}, true,
-                         r.work + W_SLOW, nullptr, s, r.walkKey);
-        if (c.shapes <= STAGE_MAX_SHAPES) {
-            size_t dynamic = STAGE_BYTES + 4 * (size_t(c.shapes) + 1);
-            // The opt-in shared-memory limit, set once per device.
-            static uint64_t attributed = 0;
-            int device = 0;
-            cudaGetDevice(&device);
-            if (device < 64 && !((attributed >> device) & 1u)) {
-                cudaFuncSetAttribute(k_nodeWalkStaged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(STAGE_BYTES + 4 * (STAGE_MAX_SHAPES + 1)));
-                attributed |= uint64_t(1) << device;
-            }
-            k_nodeWalkStaged<<<smCount(), STAGE_THREADS, dynamic, s>>>(P);
-            k_nodeWalkSlow<<<g, 256, 0, s>>>(P, 2u * smCount() * (STAGE_THREADS / 32));
-        } else {
-            k_nodeWalkSlow<<<g, 256, 0, s>>>(P, 0u);
-        }
+        k_nodeQuery<<<g, 256, 0, s>>>(P);
+        k_nodeCertify<<<g, 256, 0, s>>>(P);
+        k_nodeWalkSlow<<<g, 256, 0, s>>>(P);
     } else {
         k_nodeWalk<<<grid(c.walkBlocksPerSM, 8), 256, 0, s>>>(P);
     }
@@ -2531,21 +2664,21 @@ static void collectQuery(const Params& P, cudaStream_t s) {
     collectFilter(P, s);
     collectWalk(P, s);
 }
-// Canonical offsets of the hits, the contact records and per-pair starts.
+// The contact records and per-pair starts (with a list built every step, also
+// the canonical offsets of the hits).
 static void collectEmit(const Params& P, cudaStream_t s) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (c.meshGeometry == 0) return;
-    launch_step_scan(r, r.candHitCount, r.candHitOffset, ScanCount{r.work + W_CANDIDATES, c.candidateCapacity, 1, 0}, true,
-                r.control + 2, nullptr, s);
     uint32_t g = grid(c.contactBlocksPerSM, 8);
     if (storedKeep(c)) {
-        k_emitSlots<<<g, 256, 0, s>>>(P);
-        k_clearHits<<<g, 256, 0, s>>>(P);  // and the per-pair contact starts
-    } else {
-        k_nodeEmit<<<g, 256, 0, s>>>(P);
-        k_contactStart<<<g, 256, 0, s>>>(P);
+        k_emitSlots<false><<<g, HIT_BLOCK, 0, s>>>(P);
+        return;
     }
+    launch_step_scan(r, r.candHitCount, r.candHitOffset, ScanCount{r.work + W_CANDIDATES, c.candidateCapacity, 1, 0}, true,
+                r.control + 2, nullptr, s);
+    k_nodeEmit<<<g, 256, 0, s>>>(P);
+    k_contactStart<<<g, 256, 0, s>>>(P);
 }
 // Plane contacts after the grain-grain ones: counts, their scan, records.
 static void collectWalls(const Params& P, cudaStream_t s) {
@@ -2563,12 +2696,16 @@ static void contacts(const Params& P, cudaStream_t s) {
     collectEmit(P, s);
     collectWalls(P, s);
 }
-// The exact queries, contact emit and plane contacts: the part of the
-// collector every step runs once the filter results are in place.
+// The exact queries, contact records with their law, and plane contacts: the
+// part of the collector every step runs once the stored filter results are
+// in place.
 static void collectTail(const Params& P, cudaStream_t s) {
     collectWalk(P, s);
-    collectEmit(P, s);
+    k_emitSlots<true><<<grid(P.c.contactBlocksPerSM, 8), HIT_BLOCK, 0, s>>>(P);
     collectWalls(P, s);
+}
+static void resolveWalls(const Params& P, cudaStream_t s) {
+    if (P.c.wallCount) k_resolveWalls<<<grid(0, 2), 256, 0, s>>>(P);
 }
 
 int launch_contacts(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s) {
@@ -2589,10 +2726,15 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
     else if (name == "collectEmit") collectEmit(P, s);
     else if (name == "resolveContacts") {
         k_resolve<<<grid(c.contactBlocksPerSM, 8), T, 0, s>>>(P);
-        if (c.wallCount) k_resolveWalls<<<grid(0, 2), T, 0, s>>>(P);
+        resolveWalls(P, s);
     }
+    else if (name == "resolveWalls") resolveWalls(P, s);
     else if (name == "distanceGrid") {
-        if (c.meshGeometry != 0) k_distanceGrid<<<grid(0, 8), T, 0, s>>>(P);
+        if (c.meshGeometry != 0) {
+            k_distanceGrid<<<grid(0, 8), T, 0, s>>>(P);
+            if (storedKeep(c)) k_triangleLeaf<<<min(c.shapes, grid(0, 8)), T, 0, s>>>(P);
+            if (c.cellListsEnabled) k_cellLists<<<grid(0, 8), T, 0, s>>>(P);
+        }
     }
     else if (name == "gather") k_gather<<<min(blocks(c.N, 8), max(1u, grid(c.gatherWarps, 64) / 8)), T, 0, s>>>(P);
     else if (name == "collectWalls") collectWalls(P, s);

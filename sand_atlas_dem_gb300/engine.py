@@ -46,11 +46,16 @@ EXTENSION_ORDER = (
     "cullerMargin", "cullerStats", "candSurvMask", "candSurvOffset", "survivors", "survKeep", "keepOffset",
     "walkList", "dpairSourcePlane", "meshChildren", "distanceGrid", "distanceGridInfo", "distanceGridTriangle",
     "filterRefRotation", "filterRefBranch", "filterRefPairs", "walkKey", "walkBucketCount", "walkBucketOffset",
-    "sdfLaneCounts", "walkCertPoint", "walkCertTriangle", "wallCounts", "wallOffsets", "sideWallStart",
-    "oldWallStart", "walkNode", "walkItem",
+    "sdfLaneCounts", "walkCert", "walkState", "wallCounts", "wallOffsets", "sideWallStart",
+    "oldWallStart", "walkNode", "walkContact", "cellLists", "triangleLeaf",
+    "walkActive", "walkHits",
 )
 DISTANCE_GRID = 48  # cells per axis of each shape's distance-bound grid (csrc GRID)
 WALK_BUCKETS = 24**3  # walk-order buckets per shape (csrc WALK_BUCKETS)
+CELL_LIST_BYTES = 256  # triangle list of one distance-grid cell (csrc CELL_WORDS)
+# Largest library the triangle lists are kept for (28 MB a shape: 606 shapes);
+# beyond it the exact queries walk the BVH.
+CELL_LIST_LIMIT = 16 << 30
 CULLER_PARAMS = 3 * 64 + 64 + 64 * 64 + 64 + 64 + 4
 CULLER_MARGINS = 1 + 8**3  # per shape: whole-shape margin, then one per cell (csrc CULLER_MARGINS)
 BUFFER_ORDER = RESOURCE_ORDER + EXTENSION_ORDER
@@ -311,10 +316,19 @@ class Engine:
             "walkKey": 4 * self.survivor_capacity, "walkBucketCount": 4 * (len(library.shapes) * WALK_BUCKETS + 1),
             "walkBucketOffset": 4 * (len(library.shapes) * WALK_BUCKETS + 1),
             "sdfLaneCounts": 4 * 32 * pc if spec.contact_geometry == "sdf" else 16,
-            "walkCertPoint": 16 * self.survivor_capacity, "walkCertTriangle": 8 * self.survivor_capacity,
-            "walkNode": 16 * self.survivor_capacity, "walkItem": 8 * self.survivor_capacity,
+            "walkCert": 48 * self.survivor_capacity, "walkState": 4 * self.survivor_capacity,
+            "walkActive": 4 * self.survivor_capacity,
+            # A bit per slot, a count per 256 slots and one per 16,384 (csrc slotHitSize).
+            "walkHits": 4 * (9 * (self.survivor_capacity // 256 + 1) + self.survivor_capacity // 16384 + 1),
+            "walkNode": 16 * self.survivor_capacity, "walkContact": 4 * self.survivor_capacity,
             "wallCounts": 4 * walls, "wallOffsets": 4 * (walls + 1),
         }
+        # The triangle lists serve the stored exact-query list (not the SDF
+        # geometry, nor an engine that filters every step).
+        lists = CELL_LIST_BYTES * len(library.shapes) * DISTANCE_GRID**3
+        listed = self.filter_margin > 0 and lists <= CELL_LIST_LIMIT
+        sizes["cellLists"] = lists if listed else 16
+        sizes["triangleLeaf"] = self.buffers["meshTriangles"].size // 12 if self.filter_margin > 0 else 16
         for name, nbytes in sizes.items():
             self.buffers[name] = DeviceBuffer(self, nbytes)
         side_sizes = {
