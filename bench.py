@@ -372,6 +372,8 @@ def launches(e, steps, rebuilds, builds):
     runs, plus the neighbour-build body on rebuild steps and the filter-build
     body on filter-build steps."""
     lib, h = e.lib, e._native
+    if lib.sdg_engine_persistent(h) == 1:
+        return steps  # each step its own persistent launch, the bodies inside
     return (lib.sdg_engine_kernels_per_step(h) * steps + lib.sdg_engine_branch_kernels(h, 0) * rebuilds
             + lib.sdg_engine_branch_kernels(h, 1) * builds)
 

@@ -53,8 +53,8 @@
  *             distance beyond the nearest; optional, 16 bytes where not kept),
  *             the BVH leaf of each packed triangle, and the list of the
  *             stored walk-list slots not dormant after their build and the
- *             step's hits of those slots: a bit each, a count per 256 and
- *             one per 16,384).
+ *             step's hits of those slots: a count per 4,096, one per
+ *             262,144 and a bit each).
  * Value block (SDG_VALUE_COUNT doubles): the 25 reference Config scalars in
  * declaration order (solver.slang:12-19, normalized units as
  * src/sand_atlas_dem/gpu.py:490-518 builds them), then leaf mask words per
@@ -190,9 +190,12 @@ void sdg_engine_destroy(void* engine);
 /*
  * Advances `steps` timesteps starting from the history side the buffers
  * describe (meta/slip/normalArea/... = side written first), alternating
- * sides every step as gpu.py:725 does.  use_graph != 0 replays captured
- * graphs (recaptured when buffers or values change).  No host
- * synchronization; solver flags accumulate in control[0].
+ * sides every step as gpu.py:725 does.  use_graph != 0 runs the steps in one
+ * persistent cooperative launch where the stored exact-query list is small
+ * enough for it (a few hundred thousand live slots), else replays captured
+ * graphs (recaptured when buffers or values change); 0 launches kernel by
+ * kernel.  The results are the same.  No host synchronization; solver flags
+ * accumulate in control[0].
  */
 int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes, const double* values,
                        uint32_t nvalues, uint32_t steps, uint32_t use_graph, void* stream);
@@ -268,7 +271,7 @@ int sdg_culler_inside_max_cells(const void* points, const void* predictions, uin
 
 /*
  * Kernel launches of a captured step that skips both conditional bodies (0
- * before the first capture).  The captured step holds the neighbour build
+ * before the first advance).  The captured step holds the neighbour build
  * and, with stored filter results, the filter build as conditional-node
  * bodies keyed on device flags (the reference re-encodes the rebuild
  * dispatches every step and lets them exit early, gpu.py:547-565).
@@ -280,6 +283,8 @@ int sdg_engine_kernels_per_step(void* engine);
  * (steps that build the stored filter results).  -1 for a bad argument.
  */
 int sdg_engine_branch_kernels(void* engine, int branch);
+/* 1 if the last sdg_engine_advance ran its steps in one persistent launch. */
+int sdg_engine_persistent(void* engine);
 
 /*
  * The two median-split trees of the packed mesh layout, built on the device

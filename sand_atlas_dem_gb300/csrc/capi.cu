@@ -171,7 +171,7 @@ void launch_forces(const Params& P, cudaStream_t s, bool captureKinematics) {
 // One step of Engine._advance_once (gpu.py:714-724); captureContactKinematics
 // is fused into beginStep when the normal law is viscous.  The two parts that
 // most steps skip -- the neighbour build (device flag control[4], set by
-// checkRebuild) and the filter build (work[W_FILTER], set by the pair set-up's
+// beginStep and advanceCell) and the filter build (work[W_FILTER], set by the pair set-up's
 // motion check) -- go through `branch(flag, body)`: plain launches run the
 // body on s (its kernels return at once when the flag is clear); graph
 // capture makes it the body of a conditional node keyed on the flag.
@@ -185,9 +185,12 @@ static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
     launch_state("beginStep", B, c.N, s);
     launch_state("advanceCell", P, c.specimens, s);
     if (c.wallCount) launch_state("advanceWalls", P, 1, s);
-    launch_state("checkRebuild", P, c.N, s);
     branch(P.r.control + 4, [&](cudaStream_t b) { launch_contacts("neighbours", P, c.N, b); });
     collectAndResolve(P, s, [&](auto&& body) { branch(P.r.work + W_FILTER, body); });
+    if (!c.wallCount && !c.activeTimestep) {
+        launch_contacts("gatherFinish", P, c.N, s);
+        return;
+    }
     launch_contacts("gather", P, c.N, s);
     launch_contacts("gatherWallRows", P, c.N, s);
     if (c.activeTimestep) launch_state("checkContactTimestep", P, c.N, s);
@@ -232,9 +235,15 @@ struct Engine {
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     StepKernels kernels;
     cudaStream_t aux = nullptr;  // captures the conditional bodies
+    Params last = {};            // of the last advance
+    bool persistent = false;     // the last advance ran persistent launches
+    // Active slots as last reported by the device (pinned), which picks the
+    // step's form; UINT32_MAX before the first report.
+    uint32_t *active = nullptr, *activeDevice = nullptr;
     ~Engine() {
         reset();
         if (aux) cudaStreamDestroy(aux);
+        if (active) cudaFreeHost(active);
     }
     void reset() {
         for (auto& e : exec)
@@ -243,6 +252,36 @@ struct Engine {
         kernels = StepKernels{};
     }
 };
+
+// The persistent step serves up to 300,000 active slots (both forms measured
+// beside it: at 185 k it takes 89 us against the launched step's 121, at
+// 425 k 376 against 354); before the first report a dense packing's 18 slots
+// a grain are assumed.  Up to 6,000 grains its phases are latency-bound and
+// take the 512-thread form.
+constexpr uint32_t RUN_ACTIVE_SLOTS = 300'000, RUN_SLOTS_PER_GRAIN = 18, RUN_NARROW_GRAINS = 6'000;
+// Steps of one launch (even: each starts on the same history side): a few
+// milliseconds at a time, so that a long chunk shares the GPU.
+constexpr uint32_t RUN_STEPS = 64;
+static bool runsPersistent(Engine& e, const Config& c) {
+    static const bool cooperative = [] {
+        int device = 0, value = 0;
+        return cudaGetDevice(&device) == cudaSuccess &&
+               cudaDeviceGetAttribute(&value, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && value != 0;
+    }();
+    if (!e.active) {
+        if (cudaHostAlloc(reinterpret_cast<void**>(&e.active), sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(reinterpret_cast<void**>(&e.activeDevice), e.active, 0) != cudaSuccess) {
+            cudaGetLastError();
+            if (e.active) cudaFreeHost(e.active);
+            e.active = e.activeDevice = nullptr;
+        } else {
+            *e.active = UINT32_MAX;
+        }
+    }
+    const uint32_t known = e.active ? *static_cast<volatile uint32_t*>(e.active) : UINT32_MAX;
+    const uint64_t slots = known != UINT32_MAX ? known : uint64_t(RUN_SLOTS_PER_GRAIN) * c.N;
+    return cooperative && slots <= RUN_ACTIVE_SLOTS;
+}
 
 static uint32_t kernelNodes(cudaGraph_t graph) {
     size_t count = 0;
@@ -347,7 +386,7 @@ int sdg_dispatch(const char* kernel, uint32_t count, void* const* buffers, const
 
 // Phase timing of one step (events between the launch groups of
 // launch_step; not graph-captured).  phase_ms receives SDG_PHASES values:
-// drift (checkContactTimestep, beginStep, advanceCell, checkRebuild),
+// drift (checkContactTimestep, beginStep, advanceCell),
 // neighbours, pair setup + leaf cull + item emit, node filter + survivor
 // list, exact node queries, contact emit, friction history + contact law, force gather, final kick.
 int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes, const double* values,
@@ -368,7 +407,6 @@ int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes
     launch_state("beginStep", B, c.N, s);
     launch_state("advanceCell", P, c.specimens, s);
     if (c.wallCount) launch_state("advanceWalls", P, 1, s);
-    launch_state("checkRebuild", P, c.N, s);
     cudaEventRecord(ev[1], s);
     launch_contacts("neighbours", P, c.N, s);
     cudaEventRecord(ev[2], s);
@@ -531,6 +569,16 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
         for (uint32_t k = 0; k < steps; ++k) launch_step(side[k & 1], s);
         return record(cudaGetLastError(), "advance");
     }
+    e->last = P;
+    e->persistent = storedFilters(P.c) && runsPersistent(*e, P.c);
+    if (e->persistent) {
+        for (uint32_t k = 0; k < steps; k += RUN_STEPS)
+            if (int rc = record(cudaError_t(launch_run(side[0], side[1], std::min(RUN_STEPS, steps - k),
+                                                       P.c.N > RUN_NARROW_GRAINS, e->activeDevice, s)),
+                                "persistent steps"))
+                return rc;
+        return 0;
+    }
     // Orientation-independent key: the side whose buffers sort first is 0.
     bool flipped = std::memcmp(&side[0], &side[1], sizeof(Params)) > 0;
     const Params& first = side[flipped ? 1 : 0];
@@ -551,14 +599,35 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
     uint32_t start = flipped ? 1u : 0u;
     for (uint32_t k = 0; k < steps; ++k)
         if (int rc = record(cudaGraphLaunch(e->exec[(start + k) & 1], s), "graph launch")) return rc;
+    if (storedFilters(P.c) && e->active && steps)
+        return record(cudaMemcpyAsync(e->active, P.r.work + W_ACTIVE, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "active");
     return 0;
 }
 
+// The kernels of the last advance's step as a graph (captured here, launching
+// nothing, where the steps ran persistent).
+static const StepKernels& stepKernels(Engine* e) {
+    if (e->kernels.always == 0 && e->last.c.N != 0) {
+        cudaStream_t s = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        StepKernels counted;
+        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) {
+            if ((e->aux || cudaStreamCreateWithFlags(&e->aux, cudaStreamNonBlocking) == cudaSuccess) &&
+                capture(e->last, s, e->aux, &exec, &counted) == 0) {
+                e->kernels = counted;
+                cudaGraphExecDestroy(exec);
+            }
+            cudaStreamDestroy(s);
+        }
+    }
+    return e->kernels;
+}
+
 // Kernel launches of a captured step that skips both conditional bodies (0
-// before the first graph capture).
+// before the first advance).
 int sdg_engine_kernels_per_step(void* engine) {
     Engine* e = static_cast<Engine*>(engine);
-    return e ? int(e->kernels.always) : -1;
+    return e ? int(stepKernels(e).always) : -1;
 }
 
 // Kernel launches inside conditional body `branch` of a captured step: 0 =
@@ -567,7 +636,13 @@ int sdg_engine_kernels_per_step(void* engine) {
 int sdg_engine_branch_kernels(void* engine, int branch) {
     Engine* e = static_cast<Engine*>(engine);
     if (!e || branch < 0 || branch > 1) return -1;
-    return int(e->kernels.branch[branch]);
+    return int(stepKernels(e).branch[branch]);
+}
+
+// Whether the last sdg_engine_advance ran all its steps in one persistent launch.
+int sdg_engine_persistent(void* engine) {
+    Engine* e = static_cast<Engine*>(engine);
+    return e ? int(e->persistent) : -1;
 }
 
 }  // extern "C"

@@ -184,6 +184,7 @@ constexpr int W_REBUILDS = 17;      // steps that rebuilt the neighbour list (co
 constexpr int W_DORMANT = 18;       // dormant slots in the stored exact-query list
 constexpr int W_LAPSED = 20;        // stored walk slots without a certificate that holds this step
 constexpr int W_ACTIVE = 21;        // stored walk slots listed as live when the results were built
+constexpr int W_MOVED = 22;         // a grain asks for a neighbour build (cleared when control[4] is set)
 constexpr int W_CULL_ROWS = 19;     // kept survivors in the culler's shape-sorted list
 
 struct Params {
@@ -977,26 +978,34 @@ __device__ __forceinline__ uint32_t gridSeed(const Res& r, uint32_t shape, f3 lo
 
 // ---------------------------------------------------------------- helpers
 // The step's hits of the active slots: a bit per slot (32 slots a word), the
-// hits of each block of 256 slots and of each group of 64 blocks.  The slots
-// are in contact order, so a hit's contact index is the hits before it: its
-// group's and block's predecessors' totals and the bits below it.
-constexpr uint32_t HIT_BLOCK = 256, HIT_GROUP = 64;
+// hits of each group of 4,096 slots and of each set of 64 groups.  The slots
+// are in contact order, so a hit's contact index is the hits before it: the
+// totals of the sets, groups and words before its own and the bits below it.
+// A warp adds those up by itself: at most a few words a lane.
+constexpr uint32_t HIT_WORDS = 128, HIT_GROUPS = 64;  // words per group, groups per set
 struct SlotHits {
-    uint32_t *words, *blocks, *groups;
+    uint32_t *words, *groups, *sets;
 };
-__host__ __device__ __forceinline__ uint64_t slotHitWords(uint32_t capacity) {
-    return uint64_t(HIT_BLOCK / 32) * (capacity / HIT_BLOCK + 1);
+__host__ __device__ __forceinline__ uint32_t slotHitGroups(uint32_t capacity) { return capacity / (32 * HIT_WORDS) + 1; }
+__host__ __device__ __forceinline__ uint32_t slotHitSets(uint32_t capacity) {
+    return capacity / (32 * HIT_WORDS * HIT_GROUPS) + 1;
 }
-__host__ __device__ __forceinline__ uint64_t slotHitGroups(uint32_t capacity) {
-    return capacity / (HIT_BLOCK * HIT_GROUP) + 1;
-}
-// Words of the buffer: the bits, the blocks, the groups.
+// Words of the buffer: the groups, the sets, the bits.
 __host__ __device__ __forceinline__ uint64_t slotHitSize(uint32_t capacity) {
-    return slotHitWords(capacity) + capacity / HIT_BLOCK + 1 + slotHitGroups(capacity);
+    return uint64_t(slotHitGroups(capacity)) * (HIT_WORDS + 1) + slotHitSets(capacity);
 }
 __device__ __forceinline__ SlotHits slotHits(const Res& r, const Config& c) {
-    uint32_t* blocks = r.walkHits + slotHitWords(c.survivorCapacity);
-    return {r.walkHits, blocks, blocks + c.survivorCapacity / HIT_BLOCK + 1};
+    uint32_t* sets = r.walkHits + slotHitGroups(c.survivorCapacity);
+    return {sets + slotHitSets(c.survivorCapacity), r.walkHits, sets};
+}
+// The hits before word w (by a whole warp; the same on every lane).
+__device__ __forceinline__ uint32_t hitsBefore(const SlotHits& hits, uint32_t w) {
+    const uint32_t lane = threadIdx.x & 31u, group = w / HIT_WORDS, set = group / HIT_GROUPS;
+    uint32_t sum = 0;
+    for (uint32_t k = lane; k < set; k += 32) sum += hits.sets[k];
+    for (uint32_t k = set * HIT_GROUPS + lane; k < group; k += 32) sum += hits.groups[k];
+    for (uint32_t k = group * HIT_WORDS + lane; k < w; k += 32) sum += __popc(hits.words[k]);
+    return __reduce_add_sync(0xffffffffu, sum);
 }
 // Whether the exact-query list itself is stored with the filter results
 // (built with grown tests and ordered by target shape and coarse cell).  Not
@@ -1014,7 +1023,17 @@ __device__ __forceinline__ uint32_t activeContacts(const Res& r, const Config& c
     uint32_t n = r.control[2];
     return n < c.contactCapacity ? n : c.contactCapacity;
 }
-__device__ __forceinline__ uint32_t gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
+// Index of a thread's warp over the grid.  In the wide CTAs of the persistent
+// step (one per SM) the warps are dealt to the CTAs in turn: work that fills
+// a part of the grid spreads over every SM (a step of 1,000 grains 61 -> 41
+// us, of 10,000 grains 110 -> 93).  The launched kernels keep each 256-thread
+// CTA's work contiguous, eight CTAs to an SM (dealt in turn it costs a step of
+// 50,000 grains 30 us of L1 misses).
+__device__ __forceinline__ uint32_t warpIndex() {
+    return blockDim.x > 256 ? (threadIdx.x >> 5) * gridDim.x + blockIdx.x
+                            : (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+}
+__device__ __forceinline__ uint32_t gtid() { return warpIndex() * 32u + (threadIdx.x & 31u); }
 __device__ __forceinline__ uint32_t gstride() { return gridDim.x * blockDim.x; }
 
 // ------------------------------------------------------------------ planes
@@ -1053,16 +1072,28 @@ __device__ __forceinline__ Sum2 wallCentreDistance(const Res& r, uint32_t body, 
 // per-(wall, grain) total (solver.slang:135-146).
 __device__ __forceinline__ float wallStepWork(const Res& r, const Config& c, uint32_t id, float dt) {
     float total = 0.f;
-    for (uint32_t w = 0; w < c.wallCount; ++w) {
-        uint32_t index = w * c.N + id;
-        float increment = __fmul_rn(dt, r.wallRows[3 * index + 1].w);
-        float4 state = r.wallAccumulated[index];
-        float y = __fadd_rn(increment, state.y);
-        float high = __fadd_rn(state.x, y);
-        float low = __fsub_rn(y, __fsub_rn(high, state.x));
-        r.wallAccumulated[index] = make_float4(high, low, 0.f, 0.f);
-        r.wallRows[3 * index + 2] = make_float4(__fadd_rn(high, low), 0.f, 0.f, 0.f);
-        total = __fadd_rn(total, increment);
+    // Four planes' rows at a time, loaded before any is stored.
+    for (uint32_t w0 = 0; w0 < c.wallCount; w0 += 4) {
+        float power[4];
+        float4 state[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            uint32_t index = min(w0 + k, c.wallCount - 1) * c.N + id;
+            power[k] = r.wallRows[3 * index + 1].w;
+            state[k] = r.wallAccumulated[index];
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (w0 + k >= c.wallCount) break;
+            uint32_t index = (w0 + k) * c.N + id;
+            float increment = __fmul_rn(dt, power[k]);
+            float y = __fadd_rn(increment, state[k].y);
+            float high = __fadd_rn(state[k].x, y);
+            float low = __fsub_rn(y, __fsub_rn(high, state[k].x));
+            r.wallAccumulated[index] = make_float4(high, low, 0.f, 0.f);
+            r.wallRows[3 * index + 2] = make_float4(__fadd_rn(high, low), 0.f, 0.f, 0.f);
+            total = __fadd_rn(total, increment);
+        }
     }
     return total;
 }

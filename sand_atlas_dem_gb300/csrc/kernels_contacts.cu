@@ -12,14 +12,14 @@
 // hash table and linked lists, so every run is reproducible bit for bit.
 #include <cuda_runtime.h>
 #include "culler.cuh"
-#include "dem_device.cuh"
 #include "launch.h"
+#include "state_device.cuh"
 
 namespace sdg {
 
 constexpr uint32_t WARP = 32;
 __device__ __forceinline__ uint32_t laneId() { return threadIdx.x & 31u; }
-__device__ __forceinline__ uint32_t warpGlobal() { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
+__device__ __forceinline__ uint32_t warpGlobal() { return warpIndex(); }
 __device__ __forceinline__ uint32_t warpStride() { return (gridDim.x * blockDim.x) >> 5; }
 __device__ __forceinline__ uint32_t lanesBelow() { return (1u << laneId()) - 1u; }
 
@@ -139,17 +139,16 @@ __device__ __forceinline__ uint32_t binFlat(uint4 sb, const uint32_t b[3]) {
 }
 __device__ __forceinline__ uint32_t modIndex(int a, uint32_t n) { return uint32_t((a % int(n) + int(n)) % int(n)); }
 
-__global__ void k_binsClear(const __grid_constant__ Params P) {
+__device__ __forceinline__ void binsClear(const Params& P) {
     const Res& r = P.r;
     if (r.control[4] == 0) return;
     for (uint32_t b = gtid(); b < P.c.binCount; b += gstride()) r.binCounts[b] = 0;
 }
+__global__ void k_binsClear(const __grid_constant__ Params P) { binsClear(P); }
 // solver.slang:350-359
-__global__ void k_binsFill(const __grid_constant__ Params P) {
+__device__ __forceinline__ void binGrain(const Params& P, uint32_t id) {
     const Res& r = P.r;
     const Config& c = P.c;
-    uint32_t id = gtid();
-    if (id >= c.N || r.control[4] == 0) return;
     f3 p = xyz(r.position[id]), pl = xyz(r.positionRemainder[id]);
     if (!finite3(p) || !finite3(pl)) { fail(r, F_NONFINITE); return; }
     uint32_t sp = specimenOf(r, id);
@@ -168,6 +167,11 @@ __global__ void k_binsFill(const __grid_constant__ Params P) {
     if (slot < c.binCapacity) r.binParticles[bin * c.binCapacity + slot] = id;
     else fail(r, F_BIN);
 }
+__device__ __forceinline__ void binsFill(const Params& P) {
+    if (P.r.control[4] == 0) return;
+    for (uint32_t id = gtid(); id < P.c.N; id += gstride()) binGrain(P, id);
+}
+__global__ void k_binsFill(const __grid_constant__ Params P) { binsFill(P); }
 // Order each bin's slots by grain id: the serial reference fills bins in id
 // order, which fixes the pair order downstream.  Rank sort in shared memory.
 __global__ void k_binsSort(const __grid_constant__ Params P) {
@@ -189,6 +193,45 @@ __global__ void k_binsSort(const __grid_constant__ Params P) {
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < occ; k += blockDim.x) r.binParticles[bin * cap + k] = sorted[k];
         __syncthreads();
+    }
+}
+// The same order by a warp per bin without shared memory (the persistent
+// step's small bins): each lane ranks its grains among the bin's, all read
+// before any is written.
+__device__ __forceinline__ void binsOrder(const Params& P) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    for (uint32_t bin = warpGlobal(); bin < c.binCount; bin += warpStride()) {
+        const uint32_t occ = min(r.binCounts[bin], c.binCapacity);
+        uint32_t* slots = r.binParticles + size_t(bin) * c.binCapacity;
+        // Up to 32 grains a lane at a time keep their ranks in registers;
+        // larger bins take the serial insertion of one lane.
+        if (occ > 128) {
+            if (laneId() == 0)
+                for (uint32_t a = 1; a < occ; ++a) {
+                    uint32_t v = slots[a], k = a;
+                    while (k > 0 && slots[k - 1] > v) { slots[k] = slots[k - 1]; --k; }
+                    slots[k] = v;
+                }
+            __syncwarp();
+            continue;
+        }
+        uint32_t id[4], rank[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            id[j] = laneId() + 32 * j < occ ? slots[laneId() + 32 * j] : EMPTY;
+            rank[j] = 0;
+        }
+        for (uint32_t k = 0; k < occ; ++k) {
+            const uint32_t v = slots[k];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) rank[j] += v < id[j];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            if (id[j] != EMPTY) slots[rank[j]] = id[j];
+        __syncwarp();
     }
 }
 // ---- radix-sorted cell list (solver.slang:345-359 fills the bins serially,
@@ -438,12 +481,13 @@ __device__ __forceinline__ void findPairsWarp(const Res& r, const Config& c, uin
     }
     if (!Emit && lane == 0) r.pairCounts[id] = count;
 }
-__global__ void __launch_bounds__(256) k_pairsCountWarp(const __grid_constant__ Params P) {
+__device__ __forceinline__ void pairsCountWarp(const Params& P) {
     if (P.r.control[4] == 0) return;
     for (uint32_t id = warpGlobal(); id < P.c.N; id += warpStride()) findPairsWarp<false>(P.r, P.c, id);
 }
+__global__ void __launch_bounds__(256) k_pairsCountWarp(const __grid_constant__ Params P) { pairsCountWarp(P); }
 // solver.slang:388-392 (the pair total is written by the scan)
-__global__ void __launch_bounds__(256) k_pairsEmitWarp(const __grid_constant__ Params P) {
+__device__ __forceinline__ void pairsEmitWarp(const Params& P) {
     const Res& r = P.r;
     if (r.control[4] == 0) return;
     if (gtid() == 0) r.work[W_REBUILDS] += 1u;
@@ -455,8 +499,9 @@ __global__ void __launch_bounds__(256) k_pairsEmitWarp(const __grid_constant__ P
         r.referenceCell[2 * sp] = r.cell[3 * sp];
     }
 }
+__global__ void __launch_bounds__(256) k_pairsEmitWarp(const __grid_constant__ Params P) { pairsEmitWarp(P); }
 // Pairs grouped by their second grain, ascending pair id per grain.
-__global__ void k_byJReset(const __grid_constant__ Params P) {
+__device__ __forceinline__ void byJReset(const Params& P) {
     const Res& r = P.r;
     if (r.control[4] == 0) return;
     for (uint32_t g = gtid(); g <= P.c.N; g += gstride()) {
@@ -464,13 +509,15 @@ __global__ void k_byJReset(const __grid_constant__ Params P) {
         if (g < P.c.N) r.byJCursor[g] = 0;
     }
 }
-__global__ void k_byJCount(const __grid_constant__ Params P) {
+__global__ void k_byJReset(const __grid_constant__ Params P) { byJReset(P); }
+__device__ __forceinline__ void byJCount(const Params& P) {
     const Res& r = P.r;
     if (r.control[4] == 0) return;
     uint32_t n = activePairs(r, P.c);
     for (uint32_t p = gtid(); p < n; p += gstride()) atomicAdd(&r.byJCounts[r.pairs[p].y], 1u);
 }
-__global__ void k_byJFill(const __grid_constant__ Params P) {
+__global__ void k_byJCount(const __grid_constant__ Params P) { byJCount(P); }
+__device__ __forceinline__ void byJFill(const Params& P) {
     const Res& r = P.r;
     if (r.control[4] == 0) return;
     uint32_t n = activePairs(r, P.c);
@@ -480,17 +527,20 @@ __global__ void k_byJFill(const __grid_constant__ Params P) {
         r.byJPairs[r.byJOffsets[j] + slot] = p;
     }
 }
-__global__ void k_byJSort(const __grid_constant__ Params P) {
+__global__ void k_byJFill(const __grid_constant__ Params P) { byJFill(P); }
+__device__ __forceinline__ void byJSort(const Params& P) {
     const Res& r = P.r;
-    uint32_t g = gtid();
-    if (g >= P.c.N || r.control[4] == 0) return;
-    uint32_t begin = r.byJOffsets[g], end = r.byJOffsets[g + 1];
-    for (uint32_t a = begin + 1; a < end; ++a) {
-        uint32_t v = r.byJPairs[a], k = a;
-        while (k > begin && r.byJPairs[k - 1] > v) { r.byJPairs[k] = r.byJPairs[k - 1]; --k; }
-        r.byJPairs[k] = v;
+    if (r.control[4] == 0) return;
+    for (uint32_t g = gtid(); g < P.c.N; g += gstride()) {
+        uint32_t begin = r.byJOffsets[g], end = r.byJOffsets[g + 1];
+        for (uint32_t a = begin + 1; a < end; ++a) {
+            uint32_t v = r.byJPairs[a], k = a;
+            while (k > begin && r.byJPairs[k - 1] > v) { r.byJPairs[k] = r.byJPairs[k - 1]; --k; }
+            r.byJPairs[k] = v;
+        }
     }
 }
+__global__ void k_byJSort(const __grid_constant__ Params P) { byJSort(P); }
 
 // ------------------------------------------------------------ collection
 // Per pair: FP64 branches of both directions, root cull mask and 3x4
@@ -527,7 +577,7 @@ __device__ __forceinline__ bool filterStale(const Res& r, float margin, uint32_t
     float slack = 1e-5f * (1.0f + bi.z + bj.z + length(branch));
     return 1.001f * drift + slack > margin * fminf(bi.x, bj.x);
 }
-__global__ void k_pairSetup(const __grid_constant__ Params P) {
+__device__ __forceinline__ void pairSetup(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0) return;
@@ -546,11 +596,17 @@ __global__ void k_pairSetup(const __grid_constant__ Params P) {
     uint32_t grains = c.N;
     for (uint32_t g = gtid(); g <= grains; g += gstride())
         r.sidePairOffsets[g] = g < grains ? min(r.pairOffsets[g], n) : n;
+    if (storedKeep(c)) {
+        // The step's hit counts (groups and sets) start from zero.
+        const uint32_t counts = slotHitGroups(c.survivorCapacity) + slotHitSets(c.survivorCapacity);
+        for (uint32_t g = gtid(); g < counts; g += gstride()) r.walkHits[g] = 0;
+    }
 }
+__global__ void k_pairSetup(const __grid_constant__ Params P) { pairSetup(P); }
 // Root cull masks and source-to-target transforms of every directed pair
 // (prepareMeshPairs, solver.slang:468-489), on steps that build the filter
 // results, with the tests grown by the margin.
-__global__ void k_pairMasks(const __grid_constant__ Params P) {
+__device__ __forceinline__ void pairMasks(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
@@ -581,6 +637,7 @@ __global__ void k_pairMasks(const __grid_constant__ Params P) {
         r.meshPairMask[p] = mask;
     }
 }
+__global__ void k_pairMasks(const __grid_constant__ Params P) { pairMasks(P); }
 // resetMeshContacts (solver.slang:396-403)
 // The stored filter results (items, survivor masks and list) serve this step
 // if they are complete and were built under this configured margin on a
@@ -590,36 +647,32 @@ __global__ void k_pairMasks(const __grid_constant__ Params P) {
 // and 16 m: a build within 8 collector runs of the last one doubles it, a
 // build after more than 64 halves it (a larger margin keeps a few more nodes
 // in the stored lists; it never changes a result).
-__global__ void k_resetContacts(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    if (r.control[0] != 0) return;
-    if (storedKeep(c)) {
-        const SlotHits hits = slotHits(r, c);
-        for (uint64_t g = threadIdx.x; g < slotHitGroups(c.survivorCapacity); g += blockDim.x) hits.groups[g] = 0;
-    }
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void resetContacts(const Res& r, const Config& c, bool pairsKnown) {
+    // Loads first: a store would make each of them wait for the one before.
+    const uint32_t complete = r.work[W_FILTER_VALID], configured = r.work[W_FILTER_BASE], pairs = r.work[W_FILTER_PAIRS];
+    const uint32_t runs = r.work[W_FILTER_STEPS], age = r.work[W_FILTER_AGE] + 1u, current = r.control[1];
+    const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]);
+    bool on = c.filterMargin > 0.0f;
+    bool valid = complete != 0 && configured == __float_as_uint(c.filterMargin);
+    bool build = !on || !valid || (pairsKnown && pairs != current);
     r.control[2] = 0;
     r.control[6] = 0;
     r.work[W_SLOW] = 0;
     r.work[W_LAPSED] = 0;
-    bool on = c.filterMargin > 0.0f;
-    uint32_t base = __float_as_uint(c.filterMargin);
-    bool valid = r.work[W_FILTER_VALID] != 0 && r.work[W_FILTER_BASE] == base;
-    bool build = !on || !valid || r.work[W_FILTER_PAIRS] != r.control[1];
     r.work[W_FILTER] = build ? 1u : 0u;
-    r.work[W_FILTER_STEPS] += 1u;
+    r.work[W_FILTER_STEPS] = runs + 1u;
     if (on) {
-        uint32_t age = r.work[W_FILTER_AGE] + 1u;
         r.work[W_FILTER_AGE] = age;
-        float current = __uint_as_float(r.work[W_FILTER_MARGIN]);
         float next = c.filterMargin;
         if (valid)
-            next = age <= 8u ? fminf(2.0f * current, 16.0f * c.filterMargin)
-                             : (age > 64u ? fmaxf(0.5f * current, c.filterMargin) : current);
+            next = age <= 8u ? fminf(2.0f * margin, 16.0f * c.filterMargin)
+                             : (age > 64u ? fmaxf(0.5f * margin, c.filterMargin) : margin);
         r.work[W_FILTER_NEXT] = __float_as_uint(next);
     }
     if (build) r.work[W_CANDIDATES] = 0;
+}
+__global__ void k_resetContacts(const __grid_constant__ Params P) {
+    if (P.r.control[0] == 0) resetContacts(P.r, P.c, true);
 }
 // Flat leaf cull: one warp per directed pair; meshPairBounds (solver.slang:
 // 404-417) + meshBoxMayContact (:274-288) on every leaf, gated by the root
@@ -698,12 +751,11 @@ __device__ __forceinline__ float4 enclosurePlane(const Res& r, uint32_t j, uint3
 }
 // Runs on steps that build the filter results: with a margin every test is
 // grown by it and the pose the results are built at is recorded.
-__global__ void k_leafCull(const __grid_constant__ Params P) {
+__device__ __forceinline__ void leafCull(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.work[W_FILTER] == 0) return;
     uint32_t n = 2 * activePairs(r, c);
-    bool live = r.control[0] == 0;
     float margin = buildMargin(r, c);
     float grow = __fmul_rn(1.001f, margin);
     if (margin > 0.0f) {
@@ -781,7 +833,8 @@ __global__ void k_leafCull(const __grid_constant__ Params P) {
         if (laneId() == 0) r.dpairLeafCount[d] = count;
     }
 }
-__global__ void k_leafEmit(const __grid_constant__ Params P) {
+__global__ void k_leafCull(const __grid_constant__ Params P) { leafCull(P, P.r.control[0] == 0); }
+__device__ __forceinline__ void leafEmit(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
@@ -804,6 +857,7 @@ __global__ void k_leafEmit(const __grid_constant__ Params P) {
         }
     }
 }
+__global__ void k_leafEmit(const __grid_constant__ Params P) { leafEmit(P); }
 // Node query in stages.  The filter stage (one warp per (directed pair,
 // leaf) item, two nodes per lane) applies the one-dot enclosure-plane test
 // in the source frame and records each item's surviving nodes as a 64-bit
@@ -818,7 +872,7 @@ __global__ void k_leafEmit(const __grid_constant__ Params P) {
 // the item's hit mask (integer atomics: the result does not depend on their
 // order) and keeps its record in the survivor's scratch slot; the emit pass
 // copies hits to their canonical offsets.
-__global__ void __launch_bounds__(256) k_nodeFilter(const __grid_constant__ Params P) {
+__device__ __forceinline__ void nodeFilter(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     uint32_t n = min(r.work[W_CANDIDATES], c.candidateCapacity);
@@ -867,6 +921,7 @@ __global__ void __launch_bounds__(256) k_nodeFilter(const __grid_constant__ Para
         }
     }
 }
+__global__ void __launch_bounds__(256) k_nodeFilter(const __grid_constant__ Params P) { nodeFilter(P); }
 // Source node, partner and target-frame position of survivor s (the same
 // expressions as nodePrefilter: the same arm and local bits).
 struct SurvivorNode {
@@ -896,7 +951,7 @@ __device__ __forceinline__ SurvivorNode survivorNode(const Res& r, uint32_t s) {
 // runs only on build steps, with the plane, hull and grid tests grown by the
 // margin (a node the grid bounds farther than the margin from the surface
 // cannot reach it while the results serve).
-__global__ void __launch_bounds__(256) k_survivorPrefilter(const __grid_constant__ Params P) {
+__device__ __forceinline__ void survivorPrefilter(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     bool stored = storedKeep(c);
@@ -919,6 +974,7 @@ __global__ void __launch_bounds__(256) k_survivorPrefilter(const __grid_constant
         r.survKeep[s] = keep ? 1u : 0u;
     }
 }
+__global__ void __launch_bounds__(256) k_survivorPrefilter(const __grid_constant__ Params P) { survivorPrefilter(P); }
 // Distance-bound grid of every shape (built once per library): one thread per
 // cell evaluates the exact signed distance at the cell centre (meshDistance,
 // the query the contacts use) and stores phi - (half diagonal) x 1.001 -
@@ -1137,7 +1193,7 @@ __global__ void __launch_bounds__(CULLER_ROWS) k_cullSurvivors(const __grid_cons
 // every step (one load instead of the survivor -> item -> pair -> sample
 // chain).  In this order a warp's slots share their two grains and branch,
 // and the step's contacts leave it in place (k_emitSlots).
-__global__ void k_walkList(const __grid_constant__ Params P) {
+__device__ __forceinline__ void walkList(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     bool stored = storedKeep(c);
@@ -1161,10 +1217,11 @@ __global__ void k_walkList(const __grid_constant__ Params P) {
         r.walkContact[slot] = EMPTY;
     }
 }
+__global__ void k_walkList(const __grid_constant__ Params P) { walkList(P); }
 // Survivor list in canonical (item, node slot) order.
 // On a build step with a margin, it also marks the stored results complete
 // when no list overflowed.
-__global__ void k_survivorList(const __grid_constant__ Params P) {
+__device__ __forceinline__ void survivorList(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
@@ -1185,6 +1242,7 @@ __global__ void k_survivorList(const __grid_constant__ Params P) {
         }
     }
 }
+__global__ void k_survivorList(const __grid_constant__ Params P) { survivorList(P); }
 // Exact query, one thread per kept survivor.
 __device__ __forceinline__ void recordHitAt(const Res& r, uint32_t s, uint32_t item, uint32_t slot, float4 pd,
                                             float4 na) {
@@ -1246,8 +1304,7 @@ __global__ void __launch_bounds__(256) k_nodeWalk(const __grid_constant__ Params
 // (a few units in the last place of |p|, about 3e-7 (1 + |p|) here), the
 // other triangles stay strictly farther while 2 |p - p0| + 4e < g; the slack
 // is above 4e.  Slots whose certificate lapsed and new slots are listed
-// (in blocks of consecutive slots: the walk-bucket order, so that a warp's
-// work stays coherent) and answered and certified again from their grid
+// and answered and certified again from their grid
 // cell's triangle list in a kernel of their own, in full warps
 // (k_nodeCertify); what a list cannot decide is walked (k_nodeWalkSlow).
 // Bound by the latency of dependent loads (under 30% of issue slots used),
@@ -1277,9 +1334,9 @@ __device__ __forceinline__ bool fallsAsleep(const WalkNode& w, float phi, float 
 }
 __device__ __forceinline__ float certificateReach(float margin) { return __fadd_rn(__fmul_rn(2.01f, margin), 1e-4f); }
 // Appends the block's flagged threads' values to a list, in thread order
-// (called by every thread of a 256-thread block): one atomic per block.
+// (called by every thread of the block): one atomic per block.
 __device__ __forceinline__ void appendBlock(bool flagged, uint32_t value, uint32_t* list, uint32_t* count) {
-    __shared__ uint32_t warpBase[8], blockBase;
+    __shared__ uint32_t warpBase[32], blockBase;
     if (!__syncthreads_or(flagged)) return;
     const uint32_t warp = threadIdx.x >> 5;
     uint32_t ballot = __ballot_sync(0xffffffffu, flagged);
@@ -1287,7 +1344,7 @@ __device__ __forceinline__ void appendBlock(bool flagged, uint32_t value, uint32
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t total = 0;
-        for (uint32_t k = 0; k < 8; ++k) {
+        for (uint32_t k = 0; k < blockDim.x >> 5; ++k) {
             uint32_t n = warpBase[k];
             warpBase[k] = total;
             total += n;
@@ -1309,22 +1366,21 @@ __device__ __forceinline__ bool recordSlot(const Res& r, const Config& c, uint32
 // A hit of active slot i found after k_nodeQuery.
 __device__ __forceinline__ void lateHit(const SlotHits& hits, uint32_t i) {
     atomicOr(&hits.words[i >> 5], 1u << (i & 31u));
-    atomicAdd(&hits.blocks[i / HIT_BLOCK], 1u);
-    atomicAdd(&hits.groups[i / (HIT_BLOCK * HIT_GROUP)], 1u);
+    atomicAdd(&hits.groups[i / (32 * HIT_WORDS)], 1u);
+    atomicAdd(&hits.sets[i / (32 * HIT_WORDS * HIT_GROUPS)], 1u);
 }
-// The active slots whose certificates hold, a block of 256 at a time: their
-// hit bits and counts.  The others are listed in survKeep.  Only the slots
-// their build left awake are visited (walkActive): 185 of 449 thousand on a
-// dense packing of 10,000 grains, and warps full of them instead of a third
-// full.
-__global__ void __launch_bounds__(HIT_BLOCK, 4) k_nodeQuery(const __grid_constant__ Params P) {
+// The active slots whose certificates hold: their hit bits and counts.  The
+// others are listed in survKeep.  Only the slots their build left awake are
+// visited (walkActive): 185 of 449 thousand on a dense packing of 10,000
+// grains, and warps full of them instead of a third full.
+__device__ __forceinline__ void nodeQuery(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     const SlotHits hits = slotHits(r, c);
     uint32_t n = min(r.work[W_ACTIVE], c.survivorCapacity);
-    for (uint32_t base = blockIdx.x * HIT_BLOCK; base < n; base += gridDim.x * HIT_BLOCK) {
-        uint32_t i = base + threadIdx.x, t = i < n ? r.walkActive[i] : 0u;
+    for (uint32_t base = 0; base < n; base += gstride()) {  // the same rounds for every thread of the block
+        uint32_t i = base + gtid(), t = i < n ? r.walkActive[i] : 0u;
         uint32_t state = i < n ? r.walkState[t] : DORMANT;
         bool lapsed = state == EMPTY, hit = false;
         if (state == CERTIFIED) {
@@ -1336,26 +1392,28 @@ __global__ void __launch_bounds__(HIT_BLOCK, 4) k_nodeQuery(const __grid_constan
                 lapsed = true;
         }
         uint32_t ballot = __ballot_sync(0xffffffffu, hit);
-        if (laneId() == 0) hits.words[i >> 5] = ballot;
-        uint32_t count = __syncthreads_count(hit);
-        if (threadIdx.x == 0) {
-            hits.blocks[base / HIT_BLOCK] = count;
-            if (count) atomicAdd(&hits.groups[base / (HIT_BLOCK * HIT_GROUP)], count);
+        if (laneId() == 0 && i < n) {
+            hits.words[i >> 5] = ballot;
+            if (ballot) {
+                atomicAdd(&hits.groups[i / (32 * HIT_WORDS)], uint32_t(__popc(ballot)));
+                atomicAdd(&hits.sets[i / (32 * HIT_WORDS * HIT_GROUPS)], uint32_t(__popc(ballot)));
+            }
         }
         appendBlock(lapsed, i, r.survKeep, &r.work[W_LAPSED]);
     }
 }
+__global__ void __launch_bounds__(256, 4) k_nodeQuery(const __grid_constant__ Params P) { nodeQuery(P, P.r.control[0] == 0); }
 // A new list's slots, certified from their grid cells' triangle lists (in the
 // filter build): the slots that fall asleep at once are left out of the
 // active list (survKeep, then its scan).
-__global__ void __launch_bounds__(256) k_certifyBuild(const __grid_constant__ Params P) {
+__device__ __forceinline__ void certifyBuild(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
+    if (!live || r.work[W_FILTER] == 0) return;
     uint32_t n = min(r.work[W_KEPT], c.survivorCapacity);
     const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]), reach = certificateReach(margin);
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gstride()) {
-        uint32_t t = base + threadIdx.x;
+    for (uint32_t base = 0; base < n; base += gstride()) {
+        uint32_t t = base + gtid();
         bool asleep = false;
         if (t < n) {
             if (c.cellListsEnabled) {
@@ -1372,17 +1430,18 @@ __global__ void __launch_bounds__(256) k_certifyBuild(const __grid_constant__ Pa
         if (threadIdx.x == 0 && slept) atomicAdd(&r.work[W_DORMANT], slept);
     }
 }
+__global__ void __launch_bounds__(256) k_certifyBuild(const __grid_constant__ Params P) { certifyBuild(P, P.r.control[0] == 0); }
 // The listed active slots, from their grid cells' triangle lists; the
 // undecided ones (all of them without the lists) are listed in walkKey.
-__global__ void __launch_bounds__(256) k_nodeCertify(const __grid_constant__ Params P) {
+__device__ __forceinline__ void nodeCertify(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     uint32_t n = min(r.work[W_LAPSED], c.survivorCapacity);
     const SlotHits hits = slotHits(r, c);
     const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]), reach = certificateReach(margin);
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gstride()) {
-        uint32_t k = base + threadIdx.x, i = 0;
+    for (uint32_t base = 0; base < n; base += gstride()) {
+        uint32_t k = base + gtid(), i = 0;
         bool slow = false, asleep = false;
         if (k < n) {
             i = r.survKeep[k];
@@ -1404,6 +1463,7 @@ __global__ void __launch_bounds__(256) k_nodeCertify(const __grid_constant__ Par
         appendBlock(slow, i, r.walkKey, &r.work[W_SLOW]);
     }
 }
+__global__ void __launch_bounds__(256) k_nodeCertify(const __grid_constant__ Params P) { nodeCertify(P, P.r.control[0] == 0); }
 // Records a slot's query: its certificate from the triangles at the nearest
 // distance (`ids`, EMPTY-padded) with every other one farther by `gap`.
 __device__ __forceinline__ void certifySlot(const Res& r, const Config& c, uint32_t i, uint32_t t, const WalkNode& w,
@@ -1433,8 +1493,8 @@ __device__ __forceinline__ void certifySlot(const Res& r, const Config& c, uint3
 // critical path: a warp's certifying walk of one took 40 to 140 us of
 // dependent loads (the nodes near a 5,120-triangle shape's medial axis).
 __device__ __forceinline__ void scanSlot(const Res& r, const Config& c, uint32_t i, float margin, float reach) {
-    __shared__ float warpBest[8], warpOther[8];
-    __shared__ uint32_t warpTriangle[8];
+    __shared__ float warpBest[32], warpOther[32];
+    __shared__ uint32_t warpTriangle[32];
     const uint32_t t = r.walkActive[i];
     WalkNode w = walkNode(r, t);
     const uint32_t shape = r.shapeId[w.rec.y];
@@ -1492,7 +1552,7 @@ __device__ __forceinline__ void scanSlot(const Res& r, const Config& c, uint32_t
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (uint32_t k = 1; k < 8; ++k) merge(best, triangle, other, warpBest[k], warpTriangle[k], warpOther[k]);
+        for (uint32_t k = 1; k < blockDim.x >> 5; ++k) merge(best, triangle, other, warpBest[k], warpTriangle[k], warpOther[k]);
         NearestTriangle found{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
         if (triangle != EMPTY) considerTriangle(r, shape, w.local, triangle, found);
         float gap = triangle != EMPTY ? __fsub_rn(__fsqrt_rn(other), __fsqrt_rn(best)) : 0.0f;
@@ -1507,15 +1567,15 @@ __device__ __forceinline__ void scanSlot(const Res& r, const Config& c, uint32_t
 // more run a lane each, a certifying walk in 32-slot runs of the list
 // (coherent walks) dealt to the blocks in turn, so that either way they
 // spread over every SM.
-__global__ void __launch_bounds__(256) k_nodeWalkSlow(const __grid_constant__ Params P) {
+__device__ __forceinline__ void nodeWalkSlow(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     uint32_t n = min(r.work[W_SLOW], c.survivorCapacity);
     if (gtid() == 0) r.work[W_CERTIFIED] += min(r.work[W_KEPT], c.survivorCapacity) - n;
     float margin = __uint_as_float(r.work[W_FILTER_MARGIN]);
     float reach = certificateReach(margin);
-    uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+    uint32_t warps = warpStride(), warp = warpGlobal();
     if (n <= 4 * gridDim.x) {
         // A slot a list left undecided has many triangles at about its
         // nearest distance: no certificate is worth the ones within reach.
@@ -1536,6 +1596,7 @@ __global__ void __launch_bounds__(256) k_nodeWalkSlow(const __grid_constant__ Pa
         certifySlot(r, c, i, t, w, f, at, partner ? at + partner : tie, partner ? tie : EMPTY, gap, margin);
     }
 }
+__global__ void __launch_bounds__(256) k_nodeWalkSlow(const __grid_constant__ Params P) { nodeWalkSlow(P, P.r.control[0] == 0); }
 // L2 prefetch, first in a step, of what the step's exact queries read
 // through chains of dependent loads: the packed library (BVH node records,
 // triangles, pseudonormals, node samples) and, with a stored exact-query
@@ -1966,10 +2027,10 @@ __device__ uint32_t wallItem(const Res& r, const Config& c, uint32_t item, Sum2 
 // other.  A warp's 32 items are a grid of warps apart: the grains near a wall
 // are runs of consecutive items, spread this way over many warps.  Records
 // where the plane contacts start.
-__global__ void k_wallCount(const __grid_constant__ Params P) {
+__device__ __forceinline__ void wallCount(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     if (gtid() == 0) r.work[W_WALL_BASE] = r.control[2];
     uint32_t items = c.N * c.wallCount, lane = laneId(), stride = warpStride(), first = warpGlobal();
     for (uint32_t base = 0; base < items; base += stride * WARP) {
@@ -1985,12 +2046,13 @@ __global__ void k_wallCount(const __grid_constant__ Params P) {
         }
     }
 }
+__global__ void k_wallCount(const __grid_constant__ Params P) { wallCount(P, P.r.control[0] == 0); }
 // The plane contacts appended after the grain-grain ones (gpu.py:544-545),
 // per-(wall, grain) starts and the new contact total.
-__global__ void k_wallEmit(const __grid_constant__ Params P) {
+__device__ __forceinline__ void wallEmit(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     uint32_t items = c.N * c.wallCount, base0 = r.work[W_WALL_BASE], lane = laneId();
     for (uint32_t i = gtid(); i <= items; i += gstride()) r.sideWallStart[i] = base0 + r.wallOffsets[i];
     if (gtid() == 0) {
@@ -2008,6 +2070,7 @@ __global__ void k_wallEmit(const __grid_constant__ Params P) {
         }
     }
 }
+__global__ void k_wallEmit(const __grid_constant__ Params P) { wallEmit(P, P.r.control[0] == 0); }
 // Within one (wall, grain) run, the order of a node's contact: its position in
 // the grain's cluster order (mesh) or its index (SDF).
 __device__ __forceinline__ uint32_t wallKey(const Res& r, const Config& c, uint32_t body, uint32_t node) {
@@ -2083,7 +2146,7 @@ __device__ __forceinline__ void resolveWall(const Res& r, const Config& c, uint3
 // solver.slang:834-856: per (wall, grain), the reaction, its moment about
 // the origin and the wall power over the grain's contacts with that wall, in
 // its linked-list order (descending contact id), and the accumulated work.
-__global__ void k_gatherWallRows(const __grid_constant__ Params P) {
+__device__ __forceinline__ void gatherWallRows(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0) return;
@@ -2111,15 +2174,17 @@ __global__ void k_gatherWallRows(const __grid_constant__ Params P) {
         r.wallRows[3 * item + 2] = make_float4(__fadd_rn(work.x, work.y), 0.f, 0.f, 0.f);
     }
 }
+__global__ void k_gatherWallRows(const __grid_constant__ Params P) { gatherWallRows(P); }
 
 // solver.slang:702-733: the plane contacts, after the grain-grain ones.
-__global__ void k_resolveWalls(const __grid_constant__ Params P) {
+__device__ __forceinline__ void resolveWalls(const Params& P) {
     const Res& r = P.r;
     const Config& c = P.c;
     if (r.control[0] != 0) return;
     uint32_t n = activeContacts(r, c);
     for (uint32_t id = min(r.work[W_WALL_BASE], n) + gtid(); id < n; id += gstride()) resolveWall(r, c, id, r.meta[id]);
 }
+__global__ void k_resolveWalls(const __grid_constant__ Params P) { resolveWalls(P); }
 // solver.slang:702-749: the law of grain-grain contact `id` (source i, target
 // j, normal and area, arm and depth, branch), with the slip of its committed
 // slot `old` (EMPTY: none).  Returns whether it slides.
@@ -2177,57 +2242,41 @@ __global__ void k_resolve(const __grid_constant__ Params P) {
 }
 // The contact records of a stored exact-query list, and with `Law` the
 // contact law of each in the same pass (the step; the named phases of a
-// dispatch run them apart).  The active slots are in contact order, so the
-// kernel is a stream compaction: a block of 256 slots adds up the hits of the
-// groups and blocks before it (at most a few hundred words), each thread the
-// bits below its own, and the slots that hit write their contacts in place,
-// consecutive threads to consecutive contacts.  The first slot of each pair
+// dispatch run them apart).  The active slots are in contact order, so this
+// is a stream compaction: a warp takes 32 slots, adds up the hits before them
+// (hitsBefore), and the slots that hit write their contacts in place,
+// consecutive lanes to consecutive contacts.  The first slot of each pair
 // also writes the pair's first contact (for the pairs before it without
 // slots too).  A slot keeps the contact it became (walkContact): on the next
 // step that contact's committed key is its own, which spares the search of
 // the pair's committed run; where the key does not match (another step's
 // contacts were committed) or the slot was no contact, the search decides.
 template <bool Law>
-__global__ void __launch_bounds__(HIT_BLOCK) k_emitSlots(const __grid_constant__ Params P) {
-    __shared__ uint32_t warpSum[HIT_BLOCK / 32];
+__device__ __forceinline__ void emitSlots(const Params& P, bool live) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     const SlotHits hits = slotHits(r, c);
-    const uint32_t n = min(r.work[W_ACTIVE], c.survivorCapacity), pairs = activePairs(r, c);
-    const uint32_t lane = laneId(), warp = threadIdx.x >> 5;
+    const uint32_t n = min(r.work[W_ACTIVE], c.survivorCapacity), pairs = activePairs(r, c), lane = laneId();
     if (n == 0) {
         for (uint32_t p = gtid(); p <= pairs; p += gstride()) r.sideContactStart[p] = 0;
         return;
     }
     // Contacts on the committed side: a hint must lie below them.
     const uint32_t committed = Law && c.historyStep != 0 ? r.oldContactStart[r.oldPairOffsets[c.N]] : 0u;
-    for (uint32_t b = blockIdx.x; b * HIT_BLOCK < n; b += gridDim.x) {
-        const uint32_t group = b / HIT_GROUP;
-        uint32_t before = 0;
-        for (uint32_t k = threadIdx.x; k < group; k += HIT_BLOCK) before += hits.groups[k];
-        if (threadIdx.x < b % HIT_GROUP) before += hits.blocks[group * HIT_GROUP + threadIdx.x];
-        before = __reduce_add_sync(0xffffffffu, before);
-        if (lane == 0) warpSum[warp] = before;
-        __syncthreads();
-        uint32_t contact = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < HIT_BLOCK / 32; ++k) contact += warpSum[k];
-        const uint32_t* words = hits.words + b * (HIT_BLOCK / 32);
-        contact += __reduce_add_sync(0xffffffffu, lane < warp ? __popc(words[lane]) : 0u);
-        const uint32_t word = words[warp];
-        const bool hit = (word >> lane) & 1u;
-        contact += __popc(word & lanesBelow());
-        // This slot's contact index, or the next one's.
-        const uint32_t i = b * HIT_BLOCK + threadIdx.x;
+    for (uint32_t w = warpGlobal(); 32 * w < n; w += warpStride()) {
+        const uint32_t i = 32 * w + lane;
         const bool valid = i < n;
         const uint32_t t = valid ? r.walkActive[i] : 0u;
         const uint4 rec = valid ? r.walkNode[t] : make_uint4(0u, 0u, 2 * pairs, 0u);
-        const uint32_t pair = rec.z >> 1;
+        const uint32_t word = hits.words[w], pair = rec.z >> 1;
+        const bool hit = (word >> lane) & 1u;
+        // This slot's contact index, or the next one's.
+        const uint32_t contact = hitsBefore(hits, w) + __popc(word & lanesBelow());
         uint32_t from = __shfl_up_sync(0xffffffffu, pair, 1) + 1;
-        if (lane == 0) from = i == 0 ? 0u : (valid ? (r.walkNode[r.walkActive[i - 1]].z >> 1) + 1 : pairs);
+        if (lane == 0) from = i == 0 ? 0u : (r.walkNode[r.walkActive[i - 1]].z >> 1) + 1;
         // First contacts of the pairs up to this slot's; of the rest after the last slot.
-        uint32_t upTo = valid ? pair + 1 : from;
+        const uint32_t upTo = valid ? pair + 1 : from;
         if (valid && upTo - from <= 4)
             for (; from < upTo; ++from) r.sideContactStart[from] = contact;
         const bool last = i == n - 1;
@@ -2267,10 +2316,13 @@ __global__ void __launch_bounds__(HIT_BLOCK) k_emitSlots(const __grid_constant__
             }
             r.walkContact[t] = contact;
         }
-        uint32_t slides = __syncthreads_count(sliding);  // also before warpSum is written again
-        if (threadIdx.x == 0 && slides) atomicAdd(&r.control[6], slides);
+        uint32_t slides = __popc(__ballot_sync(0xffffffffu, sliding));
+        if (lane == 0 && slides) atomicAdd(&r.control[6], slides);
     }
 }
+template <bool Law>
+__global__ void __launch_bounds__(256) k_emitSlots(const __grid_constant__ Params P) { emitSlots<Law>(P, P.r.control[0] == 0); }
+
 // -------------------------------------------------------------------- gather
 // solver.slang:760-811, one warp per grain.  Contacts of grain g are taken in
 // the order the reference's linked lists hold them (descending contact id):
@@ -2363,20 +2415,22 @@ __device__ __forceinline__ GatherTerms wallTerms(const Res& r, const Config& c, 
     g.normalPower = r.normalLossPower[contact];
     return g;
 }
-// Three CTAs of 256 per SM (at most 80 registers): measured faster than the
-// unbounded 101-register build (two CTAs) and than four CTAs (spills).
-__global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Params P) {
+// A warp's scratch: B candidates, merged pairs, offsets and range ends of a
+// window of pairs, and the terms of a round.
+struct GatherScratch {
+    uint32_t window[4][WARP];
+    float terms[GATHER_CHAINS][GATHER_STRIDE];
+};
+// With `finish` each warp also runs the closing half kick of the grains it
+// gathered, a lane a grain (no plane, no timestep guard in between): one
+// launch and one round of latency less than a kernel of its own.
+__device__ __forceinline__ void gather(const Params& P, GatherScratch& scratch, bool live, bool finish) {
     const Res& r = P.r;
     const Config& c = P.c;
-    if (r.control[0] != 0) return;
+    if (!live) return;
     uint32_t pairs = activePairs(r, c);
-    __shared__ uint32_t window[8][4][WARP];  // per warp: B candidates, merged pairs, offsets, range ends
-    __shared__ __align__(16) float termRows[8][GATHER_CHAINS][GATHER_STRIDE];
-    uint32_t* wb = window[threadIdx.x >> 5][0];
-    uint32_t* wp = window[threadIdx.x >> 5][1];
-    uint32_t* wo = window[threadIdx.x >> 5][2];
-    uint32_t* we = window[threadIdx.x >> 5][3];
-    float (*terms)[GATHER_STRIDE] = termRows[threadIdx.x >> 5];
+    uint32_t *wb = scratch.window[0], *wp = scratch.window[1], *wo = scratch.window[2], *we = scratch.window[3];
+    float (*terms)[GATHER_STRIDE] = scratch.terms;
     const uint32_t chain = laneId();
     for (uint32_t p = gtid(); p < pairs; p += gstride())
         r.contactCounts[p] = r.sideContactStart[p + 1] - r.sideContactStart[p];
@@ -2502,29 +2556,279 @@ __global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Param
         if (laneId() == 0) {
             f3 f = mk(sums[0], sums[1], sums[2]) + mk(lows[0], lows[1], lows[2]);
             f3 t = mk(sums[3], sums[4], sums[5]) + mk(lows[3], lows[4], lows[5]);
-            f3 stress0 = mk(sums[6], sums[7], sums[8]), stress1 = mk(sums[9], sums[10], sums[11]),
-               stress2 = mk(sums[12], sums[13], sums[14]);
-            float energy = sums[15], denom = sums[16], maxDepth = sums[17], dissipation = sums[18],
-                  normalPower = sums[19], stiffnessRate = sums[20], viscousRate = sums[21];
-            r.timestepRows[id] = make_float4(stiffnessRate, viscousRate, 0.f, 0.f);
-            float4 ns = r.normalDamping[id];
-            ns.z = normalPower;
-            r.normalDamping[id] = ns;
-            r.force[id] = w4(f, maxDepth);
-            r.torque[id] = w4(t, dissipation);
-            r.particleStress[3 * id] = w4(stress0, 0.f);
-            r.particleStress[3 * id + 1] = w4(stress1, 0.f);
-            r.particleStress[3 * id + 2] = w4(stress2, 0.f);
-            f3 v = xyz(r.velocity[id]);
-            float kinetic = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(m_, dot(v, v)), dot(xyz(r.momentum[id]), omegaOf(r, id))));
-            r.particleDiagnostic[id] = make_float4(kinetic, energy, length(f), denom);
-            float4 high = r.accumulated[id], low = r.accumulatedRemainder[id];
-            compensated4(high, low, make_float4(dissipation, 0.f, 0.f, 0.f));
-            r.accumulated[id] = high;
-            r.accumulatedRemainder[id] = low;
+            // energy, denominator, deepest overlap, dissipation, normal loss power, timestep rates: 15-21
+            r.timestepRows[id] = make_float4(sums[20], sums[21], 0.f, 0.f);
+            r.force[id] = w4(f, sums[17]);
+            r.torque[id] = w4(t, sums[18]);
+            r.particleStress[3 * id] = make_float4(sums[6], sums[7], sums[8], 0.f);
+            r.particleStress[3 * id + 1] = make_float4(sums[9], sums[10], sums[11], 0.f);
+            r.particleStress[3 * id + 2] = make_float4(sums[12], sums[13], sums[14], 0.f);
+            r.particleDiagnostic[id] = make_float4(sums[19], sums[15], 0.f, sums[16]);
+        }
+    }
+    // The rest of each grain's rows, a lane a grain of those the warp
+    // gathered (one round of loads for all of them, not one a grain).
+    __syncwarp();
+    for (uint32_t id = warpGlobal() + laneId() * warpStride(); id < c.N; id += WARP * warpStride()) {
+        KickRows k = kickRows(r, id);
+        float4 diagnostic = r.particleDiagnostic[id];
+        f3 rate = xyz(r.cell[3 * specimenOf(r, id) + 1]);
+        f3 v = xyz(k.v), w = omegaRows(k.inertia, k.q, xyz(k.l) + xyz(k.ll));
+        float kinetic = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(k.mass, dot(v, v)), dot(xyz(k.l), w)));
+        k.damping.z = diagnostic.x;
+        compensated4(k.high, k.low, make_float4(k.torque.w, 0.f, 0.f, 0.f));
+        r.particleDiagnostic[id] = make_float4(kinetic, diagnostic.y, length(xyz(k.force)), diagnostic.w);
+        if (finish) {
+            finishRows(r, c, id, k, rate);
+        } else {
+            r.normalDamping[id] = k.damping;
+            r.accumulated[id] = k.high;
+            r.accumulatedRemainder[id] = k.low;
         }
     }
 }
+// Three CTAs of 256 per SM (at most 80 registers): measured faster than the
+// unbounded 101-register build (two CTAs) and than four CTAs (spills).
+__global__ void __launch_bounds__(256, 3) k_gather(const __grid_constant__ Params P, bool finish) {
+    __shared__ __align__(16) GatherScratch scratch[8];
+    gather(P, scratch[threadIdx.x >> 5], P.r.control[0] == 0, finish);
+}
+
+// ------------------------------------------------------- the persistent step
+// Whole steps in one cooperative launch: every phase of a step as above, one
+// CTA per SM going through all of them with a barrier over the grid in
+// between, and the neighbour and filter builds taken when their device flags
+// ask for them.  What a launched step costs besides its kernels -- 4 us per
+// graph launch, 1.2 us per kernel boundary and 10 us per conditional node
+// that does not run (two a step) -- becomes five barriers of 1.3 us.
+//
+// The barriers carry everything a kernel boundary would: writes before one
+// are visible after it on every SM.  Branches around barriers depend only on
+// words no CTA writes between the barrier before the branch and the next one
+// (never on control[0], which any thread may set at any time).
+//
+// Two widths: 512 threads (up to 128 registers, no spills) where the phases
+// are chains of dependent latencies, 768 (80 registers) where they fill the
+// SMs.  Step, us (512 / 768 / launched): 125 grains 50 / 54 / 78; 1,000 loose
+// 36 / 40 / 69; 343 walled 95 / 102 / 129; 10,000 dense (185 k active slots)
+// 93 / 89 / 121; but 4,913 walled (425 k) 402 / 376 / 354 and 50,000 (1.1 M)
+// 436 / 372 / 353: there the launched kernels' own register budgets win.
+struct RunArgs {
+    Params side[2];  // the two history-side orientations, first step's first
+    uint32_t steps, capture;
+    uint32_t* counter;  // grid barrier arrivals, zero at launch
+    uint32_t* active;   // receives the active slots after the last step (may be null)
+};
+struct GridBarrier {
+    uint32_t* counter;
+    uint32_t arrived = 0;
+    // Waits for every CTA; `live`: no solver flag was set before (a snapshot
+    // of this CTA).  False when the wait gave up (about two seconds): the CTA
+    // leaves, and so do the others in turn.
+    __device__ __forceinline__ bool sync(const Res& r, bool& live) {
+        __shared__ uint32_t flagged, reached;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            arrived += gridDim.x;
+            __threadfence();
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+            uint32_t seen = 0;
+            for (uint32_t k = 0; k < (1u << 22); ++k) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+                if (seen >= arrived) break;
+            }
+            __threadfence();
+            reached = seen >= arrived;
+            if (!reached) fail(r, F_WAIT);
+            flagged = *reinterpret_cast<volatile uint32_t*>(r.control);
+        }
+        __syncthreads();
+        live = flagged == 0;
+        return reached != 0;
+    }
+};
+// Exclusive scan over the grid: in[0..n) to out, the total to out[n] and
+// *total (where given), with `list` each index of a nonzero value at its
+// offset.  One barrier inside; the caller's follows.
+__device__ __forceinline__ bool runScan(GridBarrier& barrier, bool& live, const Res& r, const uint32_t* in,
+                                        uint32_t* out, uint32_t n, bool writeEnd, uint32_t* total,
+                                        uint32_t* list = nullptr) {
+    __shared__ uint32_t shared[32], tileTotal;
+    const uint32_t chunk = (n + gridDim.x - 1) / gridDim.x;
+    const uint32_t begin = min(n, blockIdx.x * chunk), end = min(n, begin + chunk);
+    uint32_t sum = 0;
+    for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) sum += in[i];
+    sum = blockInclusive(sum, shared);
+    if (threadIdx.x == blockDim.x - 1) r.scanPartials[blockIdx.x] = tileTotal = sum;
+    if (!barrier.sync(r, live)) return false;
+    const uint32_t own = tileTotal;
+    uint32_t before = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) before += r.scanPartials[k];
+    before = blockInclusive(before, shared);
+    __syncthreads();
+    if (threadIdx.x == blockDim.x - 1) tileTotal = before;
+    __syncthreads();
+    uint32_t carry = tileTotal;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        if (writeEnd) out[n] = carry + own;
+        if (total) *total = carry + own;
+    }
+    __syncthreads();
+    for (uint32_t base = begin; base < end; base += blockDim.x) {
+        uint32_t i = base + threadIdx.x;
+        uint32_t v = i < end ? in[i] : 0;
+        uint32_t inc = blockInclusive(v, shared);
+        if (i < end) {
+            out[i] = carry + inc - v;
+            if (list && v) list[carry + inc - v] = i;
+        }
+        if (threadIdx.x == blockDim.x - 1) tileTotal = inc;
+        __syncthreads();
+        carry += tileTotal;
+        __syncthreads();
+    }
+    return true;
+}
+#define RUN_SYNC() do { if (!barrier.sync(r, live)) return; } while (0)
+template <int Threads>
+__global__ void __launch_bounds__(Threads, 1) k_run(const __grid_constant__ RunArgs A) {
+    extern __shared__ __align__(16) GatherScratch runScratch[];
+    GridBarrier barrier{A.counter};
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    bool live = A.side[0].r.control[0] == 0;
+    for (uint32_t k = 0; k < A.steps; ++k) {
+        const Params& P = A.side[k & 1u];
+        const Res& r = P.r;
+        const Config& c = P.c;
+        const bool walls = c.wallCount != 0, guarded = c.activeTimestep != 0;
+        if (guarded) {
+            if (r.control[0] == 0)
+                for (uint32_t id = gtid(); id < c.N; id += gstride()) checkGrainTimestep(r, c, id);
+            RUN_SYNC();
+        }
+        // Drift; the cell rows (read by no grain here); the step's counters.
+        if (r.control[0] == 0) {
+            // (The last CTA's last warps, which have the fewest grains.)
+            const uint32_t fromEnd = blockDim.x - 1 - threadIdx.x;
+            if (blockIdx.x == gridDim.x - 1) {
+                for (uint32_t sp = fromEnd; sp < c.specimens; sp += blockDim.x) advanceCellRow(r, c, sp);
+                if (fromEnd == WARP) resetContacts(r, c, false);
+            }
+            for (uint32_t id = gtid(); id < c.N; id += gstride())
+                if (beginGrain(r, c, id, A.capture != 0)) atomicOr(&r.work[W_MOVED], 1u);
+        }
+        RUN_SYNC();
+        const bool moved = r.work[W_MOVED] != 0;
+        if (first && live) r.control[4] = moved ? 1u : 0u;
+        if (moved) {
+            RUN_SYNC();
+            binsClear(P);
+            RUN_SYNC();
+            binsFill(P);
+            RUN_SYNC();
+            binsOrder(P);
+            RUN_SYNC();
+            pairsCountWarp(P);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.pairCounts, r.pairOffsets, c.N, false, r.control + 1)) return;
+            RUN_SYNC();
+            pairsEmitWarp(P);
+            byJReset(P);
+            RUN_SYNC();
+            byJCount(P);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.byJCounts, r.byJOffsets, c.N, true, nullptr)) return;
+            RUN_SYNC();
+            byJFill(P);
+            RUN_SYNC();
+            byJSort(P);
+            RUN_SYNC();
+        }
+        if (blockIdx.x == gridDim.x - 1 && live) {
+            const uint32_t fromEnd = blockDim.x - 1 - threadIdx.x;
+            for (uint32_t sp = fromEnd; sp < c.specimens; sp += blockDim.x) advanceCellLog(r, c, sp);
+            if (fromEnd == WARP && walls) advanceWallPlanes(r, c);
+            if (fromEnd == 2 * WARP && r.work[W_FILTER_PAIRS] != r.control[1]) atomicOr(&r.work[W_FILTER], 1u);
+        }
+        pairSetup(P);
+        RUN_SYNC();
+        if (first) r.work[W_MOVED] = 0;
+        if (r.work[W_FILTER] != 0) {
+            pairMasks(P);
+            RUN_SYNC();
+            leafCull(P, live);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.dpairLeafCount, r.dpairCandOffset, 2 * activePairs(r, c), true,
+                         r.work + W_CANDIDATES))
+                return;
+            RUN_SYNC();
+            leafEmit(P);
+            RUN_SYNC();
+            nodeFilter(P);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.candSurvCount, r.candSurvOffset,
+                         min(r.work[W_CANDIDATES], c.candidateCapacity), true, r.work + W_SURVIVORS))
+                return;
+            RUN_SYNC();
+            survivorList(P);
+            RUN_SYNC();
+            survivorPrefilter(P);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.survKeep, r.keepOffset, min(r.work[W_SURVIVORS], c.survivorCapacity), true,
+                         r.work + W_KEPT))
+                return;
+            RUN_SYNC();
+            walkList(P);
+            RUN_SYNC();
+            certifyBuild(P, live);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.survKeep, r.keepOffset, min(r.work[W_KEPT], c.survivorCapacity), true,
+                         r.work + W_ACTIVE, r.walkActive))
+                return;
+            RUN_SYNC();
+        }
+        nodeQuery(P, live);
+        RUN_SYNC();
+        bool walked = false;
+        if (r.work[W_LAPSED] != 0) {
+            nodeCertify(P, live);
+            RUN_SYNC();
+            if (r.work[W_SLOW] != 0) {
+                walked = true;
+                nodeWalkSlow(P, live);
+                RUN_SYNC();
+            }
+        }
+        if (first && live && !walked) r.work[W_CERTIFIED] += min(r.work[W_KEPT], c.survivorCapacity);
+        emitSlots<true>(P, live);
+        if (walls) {
+            RUN_SYNC();
+            wallCount(P, live);
+            RUN_SYNC();
+            if (!runScan(barrier, live, r, r.wallCounts, r.wallOffsets, c.N * c.wallCount, true, nullptr)) return;
+            RUN_SYNC();
+            wallEmit(P, live);
+            RUN_SYNC();
+            resolveWalls(P);
+        }
+        RUN_SYNC();
+        gather(P, runScratch[threadIdx.x >> 5], live, !walls && !guarded);
+        if (walls) gatherWallRows(P);
+        RUN_SYNC();
+        if (walls || guarded) {
+            if (guarded) {
+                if (r.control[0] == 0)
+                    for (uint32_t id = gtid(); id < c.N; id += gstride()) checkGrainTimestep(r, c, id);
+                RUN_SYNC();
+            }
+            if (r.control[0] == 0)
+                for (uint32_t id = gtid(); id < c.N; id += gstride()) finishGrain(r, c, id);
+            RUN_SYNC();
+        }
+    }
+    if (first && A.active) *A.active = A.side[0].r.work[W_ACTIVE];
+}
+#undef RUN_SYNC
 
 // ---------------------------------------------------------------- launchers
 static inline uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
@@ -2589,7 +2893,7 @@ static void collectHead(const Params& P, cudaStream_t s) {
     const Res& r = P.r;
     const Config& c = P.c;
     uint32_t T = 256;
-    k_resetContacts<<<1, storedKeep(c) ? T : 1, 0, s>>>(P);
+    k_resetContacts<<<1, 1, 0, s>>>(P);
     k_pairSetup<<<grid(c.cullBlocksPerSM, 8), T, 0, s>>>(P);
     if (c.meshGeometry == 0) {
         k_sdfCount<<<grid(c.queryBlocksPerSM, 8), T, 0, s>>>(P);
@@ -2672,7 +2976,7 @@ static void collectEmit(const Params& P, cudaStream_t s) {
     if (c.meshGeometry == 0) return;
     uint32_t g = grid(c.contactBlocksPerSM, 8);
     if (storedKeep(c)) {
-        k_emitSlots<false><<<g, HIT_BLOCK, 0, s>>>(P);
+        k_emitSlots<false><<<g, 256, 0, s>>>(P);
         return;
     }
     launch_step_scan(r, r.candHitCount, r.candHitOffset, ScanCount{r.work + W_CANDIDATES, c.candidateCapacity, 1, 0}, true,
@@ -2701,11 +3005,26 @@ static void contacts(const Params& P, cudaStream_t s) {
 // in place.
 static void collectTail(const Params& P, cudaStream_t s) {
     collectWalk(P, s);
-    k_emitSlots<true><<<grid(P.c.contactBlocksPerSM, 8), HIT_BLOCK, 0, s>>>(P);
+    k_emitSlots<true><<<grid(P.c.contactBlocksPerSM, 8), 256, 0, s>>>(P);
     collectWalls(P, s);
 }
 static void resolveWalls(const Params& P, cudaStream_t s) {
     if (P.c.wallCount) k_resolveWalls<<<grid(0, 2), 256, 0, s>>>(P);
+}
+
+int launch_run(const Params& first, const Params& second, uint32_t steps, bool wide, uint32_t* active,
+               cudaStream_t s) {
+    RunArgs A{{first, second}, steps, first.c.normalViscosity > 0 ? 1u : 0u, first.r.scanPartials + 2 * SCAN_BLOCKS - 1,
+              active};
+    const void* kernel = wide ? reinterpret_cast<const void*>(k_run<768>) : reinterpret_cast<const void*>(k_run<512>);
+    const uint32_t threads = wide ? 768 : 512;
+    const size_t shared = threads / WARP * sizeof(GatherScratch);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared));
+    if (e == cudaSuccess) e = cudaMemsetAsync(A.counter, 0, sizeof(uint32_t), s);
+    if (e != cudaSuccess) return int(e);
+    void* args[] = {&A};
+    return int(cudaLaunchCooperativeKernel(kernel, dim3(min(smCount(), uint32_t(SCAN_BLOCKS))), dim3(threads), args,
+                                           shared, s));
 }
 
 int launch_contacts(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s) {
@@ -2736,7 +3055,8 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
             if (c.cellListsEnabled) k_cellLists<<<grid(0, 8), T, 0, s>>>(P);
         }
     }
-    else if (name == "gather") k_gather<<<min(blocks(c.N, 8), max(1u, grid(c.gatherWarps, 64) / 8)), T, 0, s>>>(P);
+    else if (name == "gather" || name == "gatherFinish")
+        k_gather<<<min(blocks(c.N, 8), max(1u, grid(c.gatherWarps, 64) / 8)), T, 0, s>>>(P, name == "gatherFinish");
     else if (name == "collectWalls") collectWalls(P, s);
     else if (name == "gatherWallRows") {
         if (c.wallCount) k_gatherWallRows<<<blocks(c.N * c.wallCount, T), T, 0, s>>>(P);

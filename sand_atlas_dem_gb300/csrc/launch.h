@@ -18,6 +18,10 @@ void set_last_error(const std::string& what);
 // Launch a reference-named kernel; 0 = launched, 1 = unknown name.
 int launch_state(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s);
 int launch_contacts(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s);
+// `steps` whole steps (stored filter results) in one persistent launch of
+// 512-thread CTAs, or 768 with `wide`; `active` (host-mapped, may be null)
+// receives the active slots.  A CUDA error code.
+int launch_run(const Params& first, const Params& second, uint32_t steps, bool wide, uint32_t* active, cudaStream_t s);
 void launch_reduce_rows(const float4* input, float4* output, uint32_t n, uint32_t rows, int maxRow, cudaStream_t s);
 void launch_reduce_wall_rows(const float4* input, float4* output, uint32_t n, uint32_t walls, cudaStream_t s);
 

@@ -318,8 +318,8 @@ class Engine:
             "sdfLaneCounts": 4 * 32 * pc if spec.contact_geometry == "sdf" else 16,
             "walkCert": 48 * self.survivor_capacity, "walkState": 4 * self.survivor_capacity,
             "walkActive": 4 * self.survivor_capacity,
-            # A bit per slot, a count per 256 slots and one per 16,384 (csrc slotHitSize).
-            "walkHits": 4 * (9 * (self.survivor_capacity // 256 + 1) + self.survivor_capacity // 16384 + 1),
+            # Counts per 4,096 slots and per 262,144, and a bit per slot (csrc slotHitSize).
+            "walkHits": 4 * (129 * (self.survivor_capacity // 4096 + 1) + self.survivor_capacity // 262144 + 1),
             "walkNode": 16 * self.survivor_capacity, "walkContact": 4 * self.survivor_capacity,
             "wallCounts": 4 * walls, "wallOffsets": 4 * (walls + 1),
         }

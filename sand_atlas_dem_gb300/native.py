@@ -131,6 +131,8 @@ def load():
     lib.sdg_engine_kernels_per_step.restype = ct.c_int
     lib.sdg_engine_branch_kernels.argtypes = [ct.c_void_p, ct.c_int]
     lib.sdg_engine_branch_kernels.restype = ct.c_int
+    lib.sdg_engine_persistent.argtypes = [ct.c_void_p]
+    lib.sdg_engine_persistent.restype = ct.c_int
     _LIB = lib
     return lib
 
@@ -155,6 +157,7 @@ EXPORTS = (
     "sdg_engine_diagnostics",
     "sdg_engine_kernels_per_step",
     "sdg_engine_branch_kernels",
+    "sdg_engine_persistent",
     "sdg_exclusive_scan",
     "sdg_scan_partials",
     "sdg_copy_buffers",
