@@ -160,6 +160,8 @@ int sdg_scan_partials(void);
  * copies (src/sand_atlas_dem/gpu.py:729-743, backend.py copy_buffer).
  */
 int sdg_copy_buffers(void* const* dst, void* const* src, const uint64_t* bytes, uint32_t n, void* stream);
+/* `bytes` of a device buffer to pinned host memory on `stream` (the caller waits). */
+int sdg_copy_to_host(void* host, const void* src, uint64_t bytes, void* stream);
 
 /*
  * The same scan with its block partials in a fixed array of this library
@@ -202,12 +204,16 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
 
 /*
  * Engine.diagnostics (src/sand_atlas_dem/gpu.py:746-891) in one call: the
- * diagnostic rows (solver.slang:922-947) and fabric rows with their 256-wide
- * tree reductions (diagnostic.slang:3-28) through two device scratch buffers
- * of scratch_bytes each (at least ceil(max(N, pairCapacity) / 256) x 8 rows x
- * 16 bytes), then 272 bytes copied to `host` (pinned): the 8 reduced
- * diagnostic rows, the 2 reduced fabric rows, the first 3 cell rows and the
- * 16 control words.  The caller waits on the stream before reading `host`.
+ * diagnostic rows (solver.slang:922-947), fabric rows and, with planes, the
+ * (wall, grain) rows with their 256-wide tree reductions (diagnostic.slang:
+ * 3-49), then 272 bytes copied to `host` (pinned): the 8 reduced diagnostic
+ * rows, the 2 reduced fabric rows, the first 3 cell rows and the 16 control
+ * words; with planes, 96 bytes more per plane: its three reduced rows, plane,
+ * remainder and velocity.  The caller waits on the stream before reading
+ * `host`.  Scratch (both non-null, scratch_bytes each): ceil(max(N,
+ * pairCapacity) / 256) x 8 rows x 16 bytes, and with planes at least (3 x
+ * (ceil(N / 256) x 1.004 + 4) + 6) rows per plane and 17 more.  The row
+ * buffers (diagnosticRows, fabricRows) and the scan partials are overwritten.
  * Replaces the reference's per-reduction dispatches and reads.
  */
 int sdg_engine_diagnostics(void* const* buffers, const uint64_t* bytes, const double* values, uint32_t nvalues,

@@ -433,46 +433,25 @@ int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes
     return rc ? rc : record(cudaGetLastError(), "profile");
 }
 
-// Engine.diagnostics in one call: the per-grain diagnostic rows and the
-// per-pair fabric rows with their 256-wide tree reductions
-// (diagnostic.slang:3-28; the same levels as sdg_reduce_rows), ping-ponged
-// through two scratch buffers, then the final 8 + 2 rows, the first three
-// cell rows and the 16 control words copied to `host` (pinned, 272 bytes:
-// 8 rows, 2 rows, 3 rows, 16 words).  The caller waits on the stream.
-static int reduceLevels(const float4* input, uint32_t n, uint32_t rows, int maxRow, float4* a, float4* b,
-                        uint64_t scratchBytes, const float4** result, cudaStream_t s) {
-    const float4* src = input;
-    float4* out = a;
-    while (n > 1) {
-        uint32_t groups = (n + 255) / 256;
-        if (uint64_t(groups) * rows * 16 > scratchBytes) { g_error = "diagnostics scratch too small"; return 1; }
-        launch_reduce_rows(src, out, n, rows, maxRow, s);
-        src = out;
-        out = out == a ? b : a;
-        n = groups;
-    }
-    *result = src;
-    return 0;
-}
+// Engine.diagnostics in one call (kernels_state.cu), then one copy to `host`.
+// Without planes the rows are collected in the scan partials, free between
+// steps; with planes in scratch_a, behind the per-wall sums.
 int sdg_engine_diagnostics(void* const* buffers, const uint64_t* bytes, const double* values, uint32_t nvalues,
                            void* scratch_a, void* scratch_b, uint64_t scratch_bytes, void* host, void* stream) {
     if (!scratch_a || !scratch_b || !host) { g_error = "null diagnostics argument"; return 1; }
     Params P;
     if (int rc = unpack(buffers, bytes, values, nvalues, P)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const Config& c = P.c;
-    auto* a = static_cast<float4*>(scratch_a);
-    auto* b = static_cast<float4*>(scratch_b);
-    char* out = static_cast<char*>(host);
-    const float4* rows = nullptr;
-    launch_state("diagnosticRows", P, c.N, s);
-    if (int rc = reduceLevels(P.r.diagnosticRows, c.N, 8, 4, a, b, scratch_bytes, &rows, s)) return rc;
-    cudaMemcpyAsync(out, rows, 8 * 16, cudaMemcpyDeviceToHost, s);
-    launch_state("fabricRows", P, c.pairCapacity, s);
-    if (int rc = reduceLevels(P.r.fabricRows, c.pairCapacity, 2, -1, a, b, scratch_bytes, &rows, s)) return rc;
-    cudaMemcpyAsync(out + 128, rows, 2 * 16, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(out + 160, P.r.cell, 3 * 16, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(out + 208, P.r.control, 16 * 4, cudaMemcpyDeviceToHost, s);
+    const uint64_t sums = 3ull * P.c.wallCount * diagnostic_wall_stride(P.c), rows = diagnostic_rows(P.c);
+    auto* scratch = static_cast<float4*>(scratch_a);
+    if (P.c.wallCount && (sums + rows) * sizeof(float4) > scratch_bytes) {
+        g_error = "diagnostics scratch too small";
+        return 1;
+    }
+    static_assert(DIAGNOSTIC_ROWS * sizeof(float4) <= 2 * SCAN_BLOCKS * sizeof(uint32_t), "diagnostic rows");
+    float4* out = P.c.wallCount ? scratch + sums : reinterpret_cast<float4*>(P.r.scanPartials);
+    launch_diagnostics(P, scratch, out, s);
+    cudaMemcpyAsync(host, out, rows * sizeof(float4), cudaMemcpyDeviceToHost, s);
     return record(cudaGetLastError(), "diagnostics");
 }
 
@@ -549,6 +528,12 @@ int sdg_copy_buffers(void* const* dst, void* const* src, const uint64_t* bytes, 
         if (int rc = record(cudaGetLastError(), "copy")) return rc;
     }
     return 0;
+}
+
+// Bytes of a device buffer to pinned host memory, on `stream`.
+int sdg_copy_to_host(void* host, const void* src, uint64_t bytes, void* stream) {
+    if (bytes && (!host || !src)) { g_error = "null copy arguments"; return 1; }
+    return record(cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)), "copy");
 }
 
 void* sdg_engine_create(void) { return new (std::nothrow) Engine(); }

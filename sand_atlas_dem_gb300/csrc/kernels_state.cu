@@ -69,14 +69,10 @@ __global__ void k_checkContactTimestep(const __grid_constant__ Params P) {
 }
 
 // solver.slang:922-936
-__global__ void k_diagnosticRows(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    uint32_t id = gtid();
-    if (id >= P.c.N) return;
+__device__ __forceinline__ void diagnosticRow(const Res& r, uint32_t id, float4 (&row)[8]) {
     f3 v = xyz(r.velocity[id]);
     float m = r.body[id].y;
     float kinetic = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(m, dot(v, v)), dot(xyz(r.momentum[id]), omegaOf(r, id))));
-    float4* row = r.diagnosticRows + 8 * size_t(id);
     row[0] = w4(xyz(r.particleStress[3 * id]), kinetic);
     row[1] = w4(xyz(r.particleStress[3 * id + 1]), r.particleDiagnostic[id].y);
     row[2] = w4(xyz(r.particleStress[3 * id + 2]), length(xyz(r.force[id])));
@@ -87,14 +83,20 @@ __global__ void k_diagnosticRows(const __grid_constant__ Params P) {
     float4 ns = r.normalDamping[id];
     row[7] = make_float4(__fadd_rn(ns.x, ns.y), ns.z, 0.f, 0.f);
 }
+__global__ void k_diagnosticRows(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    uint32_t id = gtid();
+    if (id >= P.c.N) return;
+    float4 row[8];
+    diagnosticRow(r, id, row);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r.diagnosticRows[8 * size_t(id) + k] = row[k];
+}
 
 // solver.slang:938-947
-__global__ void k_fabricRows(const __grid_constant__ Params P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    uint32_t id = gtid();
-    if (id >= c.pairCapacity) return;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+__device__ __forceinline__ void fabricRow(const Res& r, const Config& c, uint32_t id, float4& a, float4& b) {
+    a = make_float4(0.f, 0.f, 0.f, 0.f);
+    b = a;
     if (id < r.control[1] && r.contactCounts[id] > 0) {
         uint2 ij = r.pairs[id];
         f3 d = centerBranch64(r, c, ij.x, ij.y);
@@ -102,8 +104,148 @@ __global__ void k_fabricRows(const __grid_constant__ Params P) {
         a = make_float4(__fmul_rn(n.x, n.x), __fmul_rn(n.y, n.y), __fmul_rn(n.z, n.z), __fmul_rn(n.x, n.y));
         b = make_float4(__fmul_rn(n.x, n.z), __fmul_rn(n.y, n.z), 1.f, 0.f);
     }
-    r.fabricRows[2 * id] = a;
-    r.fabricRows[2 * id + 1] = b;
+}
+__global__ void k_fabricRows(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    uint32_t id = gtid();
+    if (id >= P.c.pairCapacity) return;
+    fabricRow(r, P.c, id, r.fabricRows[2 * id], r.fabricRows[2 * id + 1]);
+}
+
+// ---- all of Engine.diagnostics in two launches.  The reference reduces the
+// per-grain, per-pair and per-(wall, grain) rows by 256-wide trees, level by
+// level (diagnostic.slang:3-49); here the first level is taken where the rows
+// are computed (no row goes through memory: 128 B a grain, 32 B a reserved
+// pair) and the rest by one CTA, a warp a tree.  The pairs past the active
+// ones are zeros of the same tree and are not visited.
+// One 256-wide tree by a warp: value(k) for k < 256 in the order of the
+// reference's strides 128, 64, ..., 1 (the first three within a lane).  With
+// `maximum` the w components' largest instead of their sum, with `count`
+// their sum as integers.
+template <class Value>
+__device__ __forceinline__ float4 treeOf256(Value&& value, bool maximum, bool count) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = value(lane + 32 * j);
+    auto merge = [&](float4 a, float4 b) {
+        float4 s = add4(a, b);
+        if (maximum) s.w = mx(a.w, b.w);
+        if (count) s.w = __uint_as_float(__float_as_uint(a.w) + __float_as_uint(b.w));
+        return s;
+    };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = merge(v[j], v[j + 4]);
+    v[0] = merge(v[0], v[2]);
+    v[1] = merge(v[1], v[3]);
+    v[0] = merge(v[0], v[1]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        float4 w = make_float4(__shfl_down_sync(0xffffffffu, v[0].x, o), __shfl_down_sync(0xffffffffu, v[0].y, o),
+                               __shfl_down_sync(0xffffffffu, v[0].z, o), __shfl_down_sync(0xffffffffu, v[0].w, o));
+        v[0] = merge(v[0], w);
+    }
+    return v[0];
+}
+// First level: CTA g < groups the grains' rows; the next pairGroups the
+// pairs'; the last wallCount x groups the (wall, grain) rows.  The sums go to
+// the start of the row buffers they stand for (diagnosticRows, fabricRows)
+// and to wallSums, `wallStride` rows of three a wall.
+__global__ void __launch_bounds__(256) k_diagnosticGroups(const __grid_constant__ Params P, uint32_t groups,
+                                                          uint32_t pairGroups, float4* wallSums, uint32_t wallStride) {
+    __shared__ float4 rows[8][256];
+    const Res& r = P.r;
+    const Config& c = P.c;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t g = blockIdx.x;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < groups) {
+        const uint32_t id = 256 * g + threadIdx.x;
+        float4 row[8] = {zero, zero, zero, zero, zero, zero, zero, zero};
+        if (id < c.N) diagnosticRow(r, id, row);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) rows[k][threadIdx.x] = row[k];
+        __syncthreads();
+        float4 sum = treeOf256([&](uint32_t k) { return rows[warp][k]; }, warp == 4, false);
+        if (lane == 0) r.diagnosticRows[8 * size_t(g) + warp] = sum;
+        return;
+    }
+    g -= groups;
+    if (g < pairGroups) {
+        if (256 * g >= r.control[1]) return;  // (block-uniform) zeros: not visited above either
+        const uint32_t id = 256 * g + threadIdx.x;
+        float4 a = zero, b = zero;
+        if (id < c.pairCapacity) fabricRow(r, c, id, a, b);
+        rows[0][threadIdx.x] = a;
+        rows[1][threadIdx.x] = b;
+        __syncthreads();
+        if (warp < 2) {
+            float4 sum = treeOf256([&](uint32_t k) { return rows[warp][k]; }, false, false);
+            if (lane == 0) r.fabricRows[2 * size_t(g) + warp] = sum;
+        }
+        return;
+    }
+    g -= pairGroups;
+    const uint32_t wall = g / groups, group = g % groups;
+    if (warp < 3) {
+        float4 sum = treeOf256(
+            [&](uint32_t k) {
+                const uint32_t id = 256 * group + k;
+                return id < c.N ? r.wallRows[3 * (size_t(wall) * c.N + id) + warp] : zero;
+            },
+            false, warp == 0);
+        if (lane == 0) wallSums[3 * (size_t(wall) * wallStride + group) + warp] = sum;
+    }
+}
+// The remaining levels and the words the host reads: 8 grain rows, 2 fabric
+// rows, 3 cell rows, 16 control words, then per wall its 3 rows, plane,
+// remainder and velocity.  One CTA.
+__global__ void __launch_bounds__(1024) k_diagnosticTotals(const __grid_constant__ Params P, uint32_t groups,
+                                                           uint32_t pairGroups, float4* wallSums, uint32_t wallStride,
+                                                           float4* out) {
+    const Res& r = P.r;
+    const Config& c = P.c;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    // A level's results go behind its inputs: the row buffers hold 256 times
+    // the first level's sums, a wall's stride what its levels need.
+    auto totals = [&](float4* rows, uint32_t n, uint32_t present, uint32_t width, int maxRow, int countRow,
+                      float4* result) {
+        float4* in = rows;
+        while (n > 1) {
+            const uint32_t next = (n + 255) / 256, left = (present + 255) / 256;
+            float4* sums = in + size_t(width) * n;
+            for (uint32_t u = warp; u < left * width; u += warps) {
+                const uint32_t g = u / width, row = u % width;
+                float4 sum = treeOf256(
+                    [&](uint32_t k) {
+                        const uint32_t at = 256 * g + k;
+                        return at < present ? in[size_t(width) * at + row] : zero;
+                    },
+                    int(row) == maxRow, int(row) == countRow);
+                if (lane == 0) sums[size_t(width) * g + row] = sum;
+            }
+            __syncthreads();
+            in = sums;
+            n = next;
+            present = left;
+        }
+        if (threadIdx.x < width) result[threadIdx.x] = present ? in[threadIdx.x] : zero;
+    };
+    const uint32_t pairs = min(r.control[1], c.pairCapacity);
+    totals(r.diagnosticRows, groups, groups, 8, 4, -1, out);
+    totals(r.fabricRows, pairGroups, (pairs + 255) / 256, 2, -1, -1, out + 8);
+    if (threadIdx.x < 3) out[10 + threadIdx.x] = r.cell[threadIdx.x];
+    if (threadIdx.x < 16) reinterpret_cast<uint32_t*>(out + 13)[threadIdx.x] = r.control[threadIdx.x];
+    float4* walls = out + 17;
+    for (uint32_t w = 0; w < c.wallCount; ++w) {
+        totals(wallSums + 3 * size_t(w) * wallStride, groups, groups, 3, -1, 0, walls + 6 * w);
+        if (threadIdx.x == 0) {
+            walls[6 * w + 3] = r.wallPlane[w];
+            walls[6 * w + 4] = r.wallRemainder[w];
+            walls[6 * w + 5] = r.wallVelocity[w];
+        }
+    }
 }
 
 // diagnostic.slang:3-28: per 256-row group, values[lane] += values[lane+step]
@@ -191,6 +333,19 @@ int launch_state(const std::string_view& name, const Params& P, uint32_t count, 
     else if (name == "refreshWallPower") k_refreshWallPower<<<blocks(max(1u, P.c.N * P.c.wallCount), T), T, 0, s>>>(P);
     else return 1;
     return 0;
+}
+
+uint64_t diagnostic_rows(const Config& c) { return DIAGNOSTIC_ROWS + 6ull * c.wallCount; }
+uint32_t diagnostic_wall_stride(const Config& c) {
+    uint32_t groups = blocks(c.N, 256), rows = groups;
+    for (uint32_t n = groups; n > 1; rows += n) n = blocks(n, 256);
+    return rows;
+}
+void launch_diagnostics(const Params& P, float4* wallSums, float4* out, cudaStream_t s) {
+    const uint32_t groups = blocks(P.c.N, 256), pairGroups = blocks(P.c.pairCapacity, 256);
+    const uint32_t stride = diagnostic_wall_stride(P.c);
+    k_diagnosticGroups<<<groups * (1 + P.c.wallCount) + pairGroups, 256, 0, s>>>(P, groups, pairGroups, wallSums, stride);
+    k_diagnosticTotals<<<1, 1024, 0, s>>>(P, groups, pairGroups, wallSums, stride, out);
 }
 
 void launch_reduce_rows(const float4* input, float4* output, uint32_t n, uint32_t rows, int maxRow, cudaStream_t s) {

@@ -22,6 +22,13 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
 // 512-thread CTAs, or 768 with `wide`; `active` (host-mapped, may be null)
 // receives the active slots.  A CUDA error code.
 int launch_run(const Params& first, const Params& second, uint32_t steps, bool wide, uint32_t* active, cudaStream_t s);
+// The diagnostics' reduced rows (DIAGNOSTIC_ROWS float4 rows, then six per
+// wall: its three sums, plane, remainder and velocity) to `out`; wallSums
+// holds 3 x diagnostic_wall_stride rows per wall.
+constexpr uint32_t DIAGNOSTIC_ROWS = 17;
+uint64_t diagnostic_rows(const Config& c);
+uint32_t diagnostic_wall_stride(const Config& c);
+void launch_diagnostics(const Params& P, float4* wallSums, float4* out, cudaStream_t s);
 void launch_reduce_rows(const float4* input, float4* output, uint32_t n, uint32_t rows, int maxRow, cudaStream_t s);
 void launch_reduce_wall_rows(const float4* input, float4* output, uint32_t n, uint32_t walls, cudaStream_t s);
 

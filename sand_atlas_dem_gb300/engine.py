@@ -141,28 +141,6 @@ class DeviceBuffer:
         return self.tensor[:nbytes].cpu().numpy().view(dtype).copy()
 
 
-def read_batch(engine, requests):
-    """Several small reads ((buffer, bytes, dtype) each) staged side by side in
-    the engine's pinned buffer and waited for once."""
-    torch = _torch()
-    offsets, total = [], 0
-    for _, nbytes, _ in requests:
-        offsets.append(total)
-        total += (int(nbytes) + 15) // 16 * 16
-    if total > STAGING_BYTES:
-        return [buffer.to_numpy(dtype, nbytes // np.dtype(dtype).itemsize) for buffer, nbytes, dtype in requests]
-    with torch.cuda.stream(engine.stream):
-        for (buffer, nbytes, _), offset in zip(requests, offsets):
-            engine._staging[offset:offset + nbytes].copy_(buffer.tensor[:nbytes], non_blocking=True)
-    engine.stream.synchronize()
-    host = engine._staging.numpy()
-    out = []
-    for (_, nbytes, dtype), offset in zip(requests, offsets):
-        engine.d2h_bytes += nbytes
-        out.append(host[offset:offset + nbytes].view(dtype).copy())
-    return out
-
-
 class GB300Device:
     """The adapter surface callers read through ``engine.m`` (``cpu.py:540-689``)."""
 
@@ -257,6 +235,8 @@ class Engine:
             self.distance_grid, self.filter_margin = False, 0.0
         self._reduce_scratch = {}
         self._array_cache = {}
+        self._value_cache = {}
+        self._backup_plans = {}
         # Host copies that spare a device read: the control words as last
         # read (valid while no device work or upload followed) and the
         # strain-rate rows last written into the cell.
@@ -281,6 +261,7 @@ class Engine:
         self.device = torch.device(device or "cuda")
         self.stream = torch.cuda.Stream(self.device)
         self._staging = torch.empty(STAGING_BYTES, dtype=torch.uint8).pin_memory()
+        self._staging_host = self._staging.numpy()
         self.m = GB300Device(self)
         self.buffers = {}
         n, pc, cc = h.n, h.pair_capacity, h.contact_capacity
@@ -394,13 +375,20 @@ class Engine:
         )
 
     def _values(self, config):
-        values = list(self.layout.config_values(config)) + [
-            float(self.leaf_words), float(self.candidate_capacity), 0.0, float(self.specimens),
-            float(self.culler is not None),
-        ] + [float(self.tuning.get(k, 0)) for k in TUNING_KEYS] + [float(self.survivor_capacity),
-                                                                     float(self.distance_grid),
-                                                                     self.filter_margin]
-        return (ct.c_double * len(values))(*values), len(values)
+        """The value block of a config (built once per distinct content)."""
+        key = (tuple(config.values()), self.culler is not None, tuple(self.tuning.items()))
+        cached = self._value_cache.get(key)
+        if cached is None:
+            values = list(self.layout.config_values(config)) + [
+                float(self.leaf_words), float(self.candidate_capacity), 0.0, float(self.specimens),
+                float(self.culler is not None),
+            ] + [float(self.tuning.get(k, 0)) for k in TUNING_KEYS] + [float(self.survivor_capacity),
+                                                                         float(self.distance_grid),
+                                                                         self.filter_margin]
+            if len(self._value_cache) >= 16:
+                self._value_cache.clear()
+            cached = self._value_cache[key] = ((ct.c_double * len(values))(*values), len(values))
+        return cached
 
     def _touch(self):
         """Device work or an upload follows: host copies of device words are stale."""
@@ -433,6 +421,16 @@ class Engine:
     def check_errors(self):
         ctrl = self.read("control", np.uint32, (16,))
         return self._checked(ctrl)
+
+    def _read_control(self):
+        """The control words once the stream is done (the chunk's only wait)."""
+        self._ctrl_cache = None
+        native.check(self.lib.sdg_copy_to_host(ct.c_void_p(self._staging.data_ptr()),
+                                               ct.c_void_p(self.buffers["control"].ptr()), 64,
+                                               ct.c_void_p(self.stream.cuda_stream)))
+        self.stream.synchronize()
+        self.d2h_bytes += 64
+        return self._staging_host[:64].view(np.uint32).copy()
 
     def _checked(self, ctrl):
         self._ctrl_cache = (self._device_version, ctrl.copy())
@@ -540,18 +538,25 @@ class Engine:
             count = int(self.read("control", np.uint32, (16,))[2])
         if count < 0 or count > self.contact_capacity:
             raise ValueError("Committed contact count is outside capacity")
-        copies = []
-        for name, backup in self.backups.items():
-            src, dst = (backup, self.buffers[name]) if restore else (self.buffers[name], backup)
-            copies.append((dst, src, min(dst.size, src.size)))
-        for name, backup in self.history_backup.items():
-            src, dst = (backup, committed[name]) if restore else (committed[name], backup)
-            nbytes = 16 * count if name in ("meta", "slip", "normalArea") else min(dst.size, src.size)
-            copies.append((dst, src, nbytes))
-        n = len(copies)
-        native.check(self.lib.sdg_copy_buffers(
-            (ct.c_void_p * n)(*(d.ptr() for d, _, _ in copies)), (ct.c_void_p * n)(*(s.ptr() for _, s, _ in copies)),
-            (ct.c_uint64 * n)(*(b for _, _, b in copies)), n, ct.c_void_p(self.stream.cuda_stream)))
+        # One copy plan per history side and direction: only the committed
+        # contacts' bytes change from call to call.
+        key = (self.active, restore)
+        plan = self._backup_plans.get(key)
+        if plan is None:
+            pairs = [(self.buffers[name], backup) for name, backup in self.backups.items()]
+            history = [name in ("meta", "slip", "normalArea") for name in self.history_backup]
+            pairs += [(committed[name], backup) for name, backup in self.history_backup.items()]
+            n = len(pairs)
+            to, source = (0, 1) if restore else (1, 0)
+            plan = self._backup_plans[key] = (
+                (ct.c_void_p * n)(*(p[to].ptr() for p in pairs)),
+                (ct.c_void_p * n)(*(p[source].ptr() for p in pairs)),
+                (ct.c_uint64 * n)(*(min(a.size, b.size) for a, b in pairs)), n,
+                [len(self.backups) + k for k, h in enumerate(history) if h])
+        to, source, sizes, n, contacts = plan
+        for k in contacts:
+            sizes[k] = 16 * count
+        native.check(self.lib.sdg_copy_buffers(to, source, sizes, n, ct.c_void_p(self.stream.cuda_stream)))
         self._backup_count = count
 
     def _advance_once(self, steps, *, rate=(0, 0, 0), drag=0, wall_velocities=None):
@@ -596,9 +601,8 @@ class Engine:
             self.history = True
             done = 1
         self._launch_steps(steps - done, drag)
-        self.synchronize()
         try:
-            self.check_errors()
+            self._checked(self._read_control())
         except RuntimeError:
             self.active, self.history = original_active, original_history
             self._backup(restore=True)
@@ -736,41 +740,30 @@ class Engine:
         self.step = step
 
     def _diagnostic_rows(self, config):
-        """The reduced diagnostic and fabric rows, the cell rows and the control
-        words (``sdg_engine_diagnostics``)."""
+        """The reduced diagnostic and fabric rows, the cell rows, the control
+        words and the per-wall rows (``sdg_engine_diagnostics``: two launches,
+        one copy, one wait)."""
+        w = self.wall_count
+        nbytes = 272 + 96 * w
         if self._diagnostic_scratch is None:
-            size = 16 * 8 * ((max(self.n, self.pair_capacity) + 255) // 256)
-            self._diagnostic_scratch = (DeviceBuffer(self, size), DeviceBuffer(self, size), size)
-        a, b, size = self._diagnostic_scratch
+            groups = (max(self.n, self.pair_capacity) + 255) // 256
+            wall_rows = 17 + w * (3 * (groups + groups // 255 + 4) + 6) if w else 0
+            size = 16 * max(8 * groups, wall_rows)
+            host = self._staging if nbytes <= STAGING_BYTES else _torch().empty(nbytes, dtype=_torch().uint8).pin_memory()
+            self._diagnostic_scratch = (DeviceBuffer(self, size), DeviceBuffer(self, size), size, host)
+        a, b, size, host = self._diagnostic_scratch
         self._touch()
         ptrs, sizes = self._arrays(self.active)
         values, nv = self._values(config)
-        host = self._staging[:272]
         native.check(self.lib.sdg_engine_diagnostics(ptrs, sizes, values, nv, ct.c_void_p(a.ptr()),
                                                      ct.c_void_p(b.ptr()), size, ct.c_void_p(host.data_ptr()),
                                                      ct.c_void_p(self.stream.cuda_stream)))
         self.stream.synchronize()
-        raw = host.numpy().copy()
-        self.d2h_bytes += 272
+        raw = host.numpy()[:nbytes].copy()
+        self.d2h_bytes += nbytes
+        walls = raw[272:].view(np.float32).reshape(w, 6, 4)
         return (raw[:128].view(np.float32), raw[128:160].view(np.float32), raw[160:208].view(np.float32),
-                raw[208:272].view(np.uint32))
-
-    def _reduce(self, name, rows, max_row, read=True):
-        """Reference 256-wide tree reduction to one row set (``diagnostic.slang:3-28``);
-        with ``read=False`` the device buffer holding the rows is returned."""
-        src = self.buffers[name]
-        n = self.n if name == "diagnosticRows" else self.pair_capacity
-        level = 0
-        while n > 1:
-            groups = (n + 255) // 256
-            key = (name, level)
-            out = self._reduce_scratch.get(key)
-            if out is None or out.size < 16 * rows * groups:
-                out = self._reduce_scratch[key] = DeviceBuffer(self, 16 * rows * groups)
-            native.check(self.lib.sdg_reduce_rows(ct.c_void_p(src.ptr()), ct.c_void_p(out.ptr()), n, rows,
-                                                  max_row, ct.c_void_p(self.stream.cuda_stream)))
-            src, n, level = out, groups, level + 1
-        return self.m.read_prefix(src, 4 * rows, np.float32, shape=(rows, 4)) if read else src
+                raw[208:272].view(np.uint32), walls)
 
     def _reduce_walls(self):
         """Per-wall sums of the (wall, grain) rows (``gpu.py:774-786``); the
@@ -810,25 +803,8 @@ class Engine:
 
     def diagnostics(self):
         """Stress, energies, contact counts, fabric and wall rows (``gpu.py:746-891``)."""
-        c = self.config()
         w = self.wall_count
-        if w:
-            self.dispatch("diagnosticRows", self.n, c)
-            rows = self._reduce("diagnosticRows", 8, 4, read=False)
-            self.dispatch("fabricRows", self.pair_capacity, c)
-            fabric_rows = self._reduce("fabricRows", 2, -1, read=False)
-            reads = [(rows, 16 * 8, np.float32), (fabric_rows, 16 * 2, np.float32),
-                     (self.buffers["cell"], 16 * 3, np.float32), (self.buffers["control"], 4 * 16, np.uint32)]
-            reads += [(self._reduce_walls(), 48 * w, np.float32), (self.buffers["wallPlane"], 16 * w, np.float32),
-                      (self.buffers["wallRemainder"], 16 * w, np.float32),
-                      (self.buffers["wallVelocity"], 16 * w, np.float32)]
-            # One wait for all the small reads.
-            data, fabric_data, cell, ctrl, *wall_reads = read_batch(self, reads)
-        else:
-            # Without planes: the rows, their reductions and the reads in one
-            # native call and one wait.
-            data, fabric_data, cell, ctrl = self._diagnostic_rows(c)
-            wall_reads = []
+        data, fabric_data, cell, ctrl, wall_rows = self._diagnostic_rows(self.config())
         data, fabric_data, cell = data.reshape(8, 4), fabric_data.reshape(2, 4), cell.reshape(3, 4)
         ctrl = self._checked(ctrl)
         active_pairs = round(float(fabric_data[1, 2]))
@@ -843,9 +819,7 @@ class Engine:
         domain = box.copy()
         walls = []
         if w:
-            wall_data, plane, remainder, velocity = wall_reads
-            walls, offsets = self._wall_results(wall_data.reshape(w, 3, 4), plane.reshape(w, 4),
-                                                remainder.reshape(w, 4), velocity.reshape(w, 4))
+            walls, offsets = self._wall_results(wall_rows[:, :3], wall_rows[:, 3], wall_rows[:, 4], wall_rows[:, 5])
             if self.spec.boundary_box is not None:
                 box = box_extents(offsets, self.spec.boundary_box, domain)
         volume = float(box.prod())

@@ -98,6 +98,8 @@ def load():
     lib.sdg_engine_diagnostics.restype = ct.c_int
     lib.sdg_copy_buffers.argtypes = [P(ct.c_void_p), P(ct.c_void_p), P(ct.c_uint64), ct.c_uint32, ct.c_void_p]
     lib.sdg_copy_buffers.restype = ct.c_int
+    lib.sdg_copy_to_host.argtypes = [ct.c_void_p, ct.c_void_p, ct.c_uint64, ct.c_void_p]
+    lib.sdg_copy_to_host.restype = ct.c_int
     lib.sdg_exclusive_scan_static.argtypes = [ct.c_void_p, ct.c_void_p, ct.c_uint32, ct.c_void_p, ct.c_void_p]
     lib.sdg_exclusive_scan_static.restype = ct.c_int
     V = ct.c_void_p
@@ -161,6 +163,7 @@ EXPORTS = (
     "sdg_exclusive_scan",
     "sdg_scan_partials",
     "sdg_copy_buffers",
+    "sdg_copy_to_host",
     "sdg_exclusive_scan_static",
     "sdg_culler_param_count",
     "sdg_culler_sample",
