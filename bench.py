@@ -476,27 +476,27 @@ def run_gb300(args, cpu=True):
     dormant = filter_cache["dormant_slots"]
     step_bytes, query_bytes, walk_bytes = algorithmic_bytes(w.grains, pairs, contacts, items, nodes, survivors,
                                                             kept, 0, lib_bytes, dormant)
-    kernel_name = ("k_nodeWalkKnown + k_nodeWalkStaged/k_nodeWalkSlow (exact queries: certified triangles, "
-                   "then full BVH walks)"
+    kernel_name = ("k_nodeQuery + k_nodeCertify/k_nodeWalkSlow (exact queries: certified triangles, "
+                   "then cell lists, then leaf scans)"
                    if e.filter_margin > 0 and e.culler is None else "k_nodeWalk (exact BVH queries, one thread per kept node)")
     group_name = "k_nodeFilter, k_survivorList, k_survivorPrefilter, k_walkList, k_nodeWalk + scans"
     if e.sdf:
-        # SDF emit (k_sdfEmit, one warp per pair), counted at its minimum:
-        # every node of both grains read once (its sample, 16 B), the 8 grid
-        # values of each contact node's cell (32 B) and 52 B written per
-        # contact; the count pass reads the samples once more.
+        # SDF queries and emit, counted at their minimum: every node of both
+        # grains read once (its sample, 16 B), the 8 grid values of each
+        # contact node's cell (32 B) and 52 B written per contact.
         node_count = pairs * 2 * w.config["nodes_per_grain"]
         walk_bytes = 16 * node_count + (32 + 52) * contacts + sum(e.layout.geometry[k].nbytes for k in ("distance", "sample"))
-        query_bytes = walk_bytes + 16 * node_count + 32 * contacts
+        query_bytes = walk_bytes
         step_bytes = 516 * w.grains + 264 * pairs + 272 * contacts + query_bytes
-        kernel_name = "k_sdfEmit (SDF node queries and contact writes, one warp per pair)"
-        group_name = "k_sdfCount, contact scan, k_sdfEmit"
+        kernel_name = "k_sdfQuery (SDF node queries, one warp per pair) + k_sdfEmit"
+        group_name = "k_sdfQuery, contact scan, k_sdfEmit"
     hbm, peak_kind = peaks()
     top = max(phase_ms, key=phase_ms.get)
     query_ms = phase_ms["node_filter"] + phase_ms["node_query"] + (phase_ms["pair_cull"] if e.sdf else 0.0)
     query_gbs = query_bytes / (query_ms / 1e3) / 1e9
-    # The dominant kernel, k_nodeWalk, is the whole "node_query" phase (one launch).
-    walk_gbs = walk_bytes / (phase_ms["node_query"] / 1e3) / 1e9
+    # The exact queries are the whole "node_query" phase (with the SDF geometry
+    # they run in the pair set-up's group).
+    walk_gbs = walk_bytes / ((query_ms if e.sdf else phase_ms["node_query"]) / 1e3) / 1e9
     # End to end through the public API: advance() chunks plus diagnostics().
     chunk = 10
     chunks = max(1, args.steps // chunk)
