@@ -968,6 +968,68 @@ __device__ __forceinline__ bool cellQuery(const Res& r, uint32_t shape, f3 p, fl
     f = distanceResult(r, p, n.best, n.point, n.normal, true, false);
     return true;
 }
+// The same query by a whole warp (p and record the same on every lane): the
+// lanes evaluate the whole list together, two triangles at most each, instead
+// of one after the other: a few microseconds for a slot with many triangles
+// at about its nearest distance, where a lane took up to 150.  Every lane
+// returns the result.
+__device__ __forceinline__ bool cellQueryWarp(const Res& r, uint32_t shape, f3 p, uint4* record, float4& f) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float4 info = __ldg(&r.distanceGridInfo[shape]);
+    f3 centre;
+    uint32_t cell = nearestCell(info, p, centre);
+    const uint32_t* words = r.cellLists + (size_t(shape) * GRID * GRID * GRID + cell) * CELL_WORDS;
+    float limit = __uint_as_float(__ldg(words));
+    float off = __fadd_rn(__fmul_rn(1.00001f, length(p - centre)), 1e-6f);
+    NearestTriangle n{1e30f, mk(0.f, 0.f, 0.f), 0, EMPTY, false, false};
+    const uint32_t t0 = __ldg(words + 2 + lane), t1 = lane < CELL_TRIANGLES - 32 ? __ldg(words + 34 + lane) : EMPTY;
+    float d0 = 1e30f, d1 = 1e30f;
+    if (t0 != EMPTY) d0 = considerTriangle<true>(r, shape, p, t0, n);
+    if (t1 != EMPTY) d1 = considerTriangle<true>(r, shape, p, t1, n);
+    // Squared distances are not negative: their bits order as they do.
+    const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(n.best)));
+    const uint32_t tied = __ballot_sync(0xffffffffu, n.triangle != EMPTY && n.best == best);
+    if (tied == 0) return false;
+    float root = __fsqrt_rn(best), bound = __fsub_rn(limit, off);
+    if (!(__fsub_rn(bound, root) > distanceSlack(p))) return false;
+    uint32_t winner = __ffs(tied) - 1, triangle = __shfl_sync(0xffffffffu, n.triangle, winner);
+    uint32_t normal = __shfl_sync(0xffffffffu, n.normal, winner);
+    f3 point = mk(__shfl_sync(0xffffffffu, n.point.x, winner), __shfl_sync(0xffffffffu, n.point.y, winner),
+                  __shfl_sync(0xffffffffu, n.point.z, winner));
+    // Ties: where the results differ, the first a walk reaches.
+    const bool differs = ((tied >> lane) & 1u) && !sameResult(r, n.point, n.normal, point, normal);
+    if (__any_sync(0xffffffffu, differs)) {
+        for (uint32_t rest = tied & (tied - 1); rest; rest &= rest - 1) {
+            const uint32_t other = __ffs(rest) - 1, next = __shfl_sync(0xffffffffu, n.triangle, other);
+            const uint32_t leaf = __ldg(&r.triangleLeaf[next]), held = __ldg(&r.triangleLeaf[triangle]);
+            if (leaf == held ? next < triangle : leafVisitedFirst(r, shape, p, leaf, held)) {
+                winner = other;
+                triangle = next;
+            }
+        }
+        normal = __shfl_sync(0xffffffffu, n.normal, winner);
+        point = mk(__shfl_sync(0xffffffffu, n.point.x, winner), __shfl_sync(0xffffffffu, n.point.y, winner),
+                   __shfl_sync(0xffffffffu, n.point.z, winner));
+    }
+    // The nearest eight, in order, for the certificate.
+    CertificateBuilder list;
+#pragma unroll
+    for (uint32_t k = 0; k <= CERT_TRIANGLES; ++k) {
+        const float least = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(fminf(d0, d1))));
+        const uint32_t from = __ballot_sync(0xffffffffu, least < 1e30f && fminf(d0, d1) == least);
+        if (from == 0) break;
+        const uint32_t source = __ffs(from) - 1;
+        list.d[k] = least;
+        list.id[k] = __shfl_sync(0xffffffffu, d0 == least ? t0 : t1, source);
+        if (lane == source) {
+            if (d0 == least) d0 = 1e30f;
+            else d1 = 1e30f;
+        }
+    }
+    if (lane == 0) list.write(record, p, __fsub_rn(bound, root));
+    f = distanceResult(r, p, best, point, normal, true, false);
+    return true;
+}
 // The triangle nearest to the centre of the cell holding `local` (a seed
 // for meshDistance), or EMPTY outside the grid.
 __device__ __forceinline__ uint32_t gridSeed(const Res& r, uint32_t shape, f3 local) {

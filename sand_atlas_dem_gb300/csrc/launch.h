@@ -18,9 +18,21 @@ void set_last_error(const std::string& what);
 // Launch a reference-named kernel; 0 = launched, 1 = unknown name.
 int launch_state(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s);
 int launch_contacts(const std::string_view& name, const Params& P, uint32_t count, cudaStream_t s);
-// `steps` whole steps (stored filter results) in one persistent launch of
-// 512-thread CTAs, or 768 with `wide`; `active` (host-mapped, may be null)
-// receives the active slots.  A CUDA error code.
+// The persistent step (run_device.cuh): whole steps in one cooperative launch
+// of `ctas` CTAs, a translation unit per form; CUDA error codes.
+struct RunArgs {
+    Params side[2];  // the two history-side orientations, first step's first
+    uint32_t steps, capture;
+    uint32_t* counter;  // grid barrier arrivals, zero at launch
+    uint32_t* active;   // receives the active slots after the last step (may be null)
+};
+int launch_run_mesh(const RunArgs& A, uint32_t ctas, cudaStream_t s);
+int launch_run_mesh_wide(const RunArgs& A, uint32_t ctas, cudaStream_t s);
+int launch_run_walls(const RunArgs& A, uint32_t ctas, cudaStream_t s);
+int launch_run_walls_wide(const RunArgs& A, uint32_t ctas, cudaStream_t s);
+int launch_run_sdf(const RunArgs& A, uint32_t ctas, cudaStream_t s);
+// Picks the form: 768-thread CTAs with `wide` (mesh geometry), else 512;
+// `active` (host-mapped, may be null) receives the active slots.
 int launch_run(const Params& first, const Params& second, uint32_t steps, bool wide, uint32_t* active, cudaStream_t s);
 // The diagnostics' reduced rows (DIAGNOSTIC_ROWS float4 rows, then six per
 // wall: its three sums, plane, remainder and velocity) to `out`; wallSums

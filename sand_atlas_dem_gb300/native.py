@@ -16,7 +16,8 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBDIR = PACKAGE / "_lib"
 LIBRARY = LIBDIR / "libsanddem_gb300.so"
-SOURCES = ("kernels_state.cu", "kernels_contacts.cu", "capi.cu", "culler.cu", "scan_static.cu", "trees.cu")
+SOURCES = ("run_mesh_wide.cu", "run_walls_wide.cu", "run_mesh.cu", "run_walls.cu", "run_sdf.cu", "kernels_state.cu",
+           "kernels_contacts.cu", "capi.cu", "culler.cu", "scan_static.cu", "trees.cu")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # --fmad=false keeps the reference's FP32 operation order (no contraction);
 # division and square root stay IEEE (no fast math).
