@@ -399,39 +399,69 @@ __device__ __forceinline__ void pairSetup(const Params& P) {
         for (uint32_t g = gtid(); g < counts; g += gstride()) r.walkHits[g] = 0;
     }
 }
-// Root cull masks and source-to-target transforms of every directed pair
-// (prepareMeshPairs, solver.slang:468-489), on steps that build the filter
-// results, with the tests grown by the margin.
-__device__ __forceinline__ void pairMasks(const Params& P) {
-    const Res& r = P.r;
-    const Config& c = P.c;
-    if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
-    uint32_t n = activePairs(r, c);
-    float margin = buildMargin(r, c);
-    for (uint32_t p = gtid(); p < n; p += gstride()) {
-        uint2 ij = r.pairs[p];
-        f3 branch[2] = {xyz(r.dpairBranch[2 * p]), xyz(r.dpairBranch[2 * p + 1])};
-        uint32_t mask = 0;
-        if (meshClusterMayContact(r, ij.x, ij.y, r.meshClusterInfo[r.shapeId[ij.x]].x, branch[0], margin)) mask |= 1;
-        if (meshClusterMayContact(r, ij.y, ij.x, r.meshClusterInfo[r.shapeId[ij.y]].x, branch[1], margin)) mask |= 2;
-        for (uint32_t pass = 0; pass < 2; ++pass) {
-            if ((mask & (1u << pass)) == 0) continue;
-            uint32_t i = pass == 0 ? ij.x : ij.y, j = pass == 0 ? ij.y : ij.x;
-            float4 qi = r.rotation[i], qj = r.rotation[j];
-            float sj = r.body[j].x;
-            float ratio = __fdiv_rn(r.body[i].x, sj);
-            f3 a = qinv(qj, qrot(qi, mk(ratio, 0.f, 0.f)));
-            f3 b = qinv(qj, qrot(qi, mk(0.f, ratio, 0.f)));
-            f3 cz = qinv(qj, qrot(qi, mk(0.f, 0.f, ratio)));
-            f3 offset = qinv(qj, -branch[pass]) / sj;
-            uint32_t base = 4 * (2 * p + pass);
-            r.meshPairTransform[base] = make_float4(a.x, b.x, cz.x, offset.x);
-            r.meshPairTransform[base + 1] = make_float4(a.y, b.y, cz.y, offset.y);
-            r.meshPairTransform[base + 2] = make_float4(a.z, b.z, cz.z, offset.z);
-            r.meshPairTransform[base + 3] = make_float4(__fdiv_rn(length(branch[pass]), sj), 0.f, 0.f, 0.f);
-        }
-        r.meshPairMask[p] = mask;
+// Root cull mask and source-to-target transform of directed pair d
+// (prepareMeshPairs, solver.slang:468-489), by its warp: the box corners a
+// lane each, the hull group's planes 32 at a time, the transform's columns a
+// lane each.  With the test grown by the margin on steps that build the
+// filter results.  A thread a pair, one corner and one plane after the other,
+// was the longest chain of a build (20 to 30 us whatever the size).
+__device__ __forceinline__ bool rootMayContact(const Res& r, uint32_t d, uint32_t i, uint32_t j, f3 branch, float margin) {
+    const uint32_t lane = laneId(), cluster = r.meshClusterInfo[r.shapeId[i]].x, shape = r.shapeId[j];
+    const f3 sl = xyz(r.meshClusterMin[cluster]), sh = xyz(r.meshClusterMax[cluster]);
+    const float4 qs = r.rotation[i], qd = r.rotation[j];
+    const float ss = r.body[i].x, sd = r.body[j].x;
+    // solver.slang:290-305 (meshClusterMayContact): the transformed corners' box.
+    f3 p = mk((lane & 1) ? sh.x : sl.x, (lane & 2) ? sh.y : sl.y, (lane & 4) ? sh.z : sl.z);
+    p = qinv(qd, qrot(qs, p * ss) - branch) / sd;
+    f3 low = p, high = p;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        low = mn3(low, mk(__shfl_xor_sync(0xffffffffu, low.x, o), __shfl_xor_sync(0xffffffffu, low.y, o),
+                          __shfl_xor_sync(0xffffffffu, low.z, o)));
+        high = mx3(high, mk(__shfl_xor_sync(0xffffffffu, high.x, o), __shfl_xor_sync(0xffffffffu, high.y, o),
+                            __shfl_xor_sync(0xffffffffu, high.z, o)));
     }
+    float pad = __fmul_rn(0.00000762939453125f,
+        __fadd_rn(__fadd_rn(__fadd_rn(1.0f, mx(mx(fabsf(low.x), fabsf(low.y)), fabsf(low.z))),
+                            mx(mx(fabsf(high.x), fabsf(high.y)), fabsf(high.z))), __fdiv_rn(length(branch), sd)));
+    if (margin > 0.0f) pad = __fadd_rn(pad, margin);
+    low = low - mk(pad, pad, pad);
+    high = high + mk(pad, pad, pad);
+    f3 centre, half;
+    uint32_t group;
+    bool open = meshBoxGroup(r, shape, low, high, centre, half, group);
+    if (open) {  // (the same on every lane)
+        uint4 info = __ldg(&r.meshHullInfo[6 * shape + group]);
+        bool outside = false;
+        for (uint32_t q = lane; q < info.y; q += WARP) {
+            float4 plane = __ldg(&r.meshPlanes[info.x + q]);
+            outside |= __fsub_rn(__fadd_rn(dot(xyz(plane), centre), plane.w), dot(abs3(xyz(plane)), half)) > 0;
+        }
+        open = !__any_sync(0xffffffffu, outside);
+    }
+    if (open) {
+        // Lanes 0-2 the rotated axes, lane 3 the offset; row k from them.
+        const float ratio = __fdiv_rn(ss, sd);
+        f3 column;
+        if (lane < 3) column = qinv(qd, qrot(qs, mk(lane == 0 ? ratio : 0.f, lane == 1 ? ratio : 0.f, lane == 2 ? ratio : 0.f)));
+        else column = qinv(qd, -branch) / sd;
+        float row[3][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            row[0][k] = __shfl_sync(0xffffffffu, column.x, k);
+            row[1][k] = __shfl_sync(0xffffffffu, column.y, k);
+            row[2][k] = __shfl_sync(0xffffffffu, column.z, k);
+        }
+        float4* out = r.meshPairTransform + 4 * size_t(d);
+        if (lane == 0) {
+            out[0] = make_float4(row[0][0], row[0][1], row[0][2], row[0][3]);
+            out[1] = make_float4(row[1][0], row[1][1], row[1][2], row[1][3]);
+            out[2] = make_float4(row[2][0], row[2][1], row[2][2], row[2][3]);
+            out[3] = make_float4(__fdiv_rn(length(branch), sd), 0.f, 0.f, 0.f);
+        }
+    }
+    __syncwarp();
+    return open;
 }
 // resetMeshContacts (solver.slang:396-403)
 // The stored filter results (items, survivor masks and list) serve this step
@@ -571,7 +601,7 @@ __device__ __forceinline__ void leafCull(const Params& P, bool live) {
             r.filterRefBranch[p] = r.dpairBranch[d];
         }
         uint32_t count = 0;
-        if (live && ((r.meshPairMask[p] >> pass) & 1u)) {
+        if (live && rootMayContact(r, d, i, j, xyz(r.dpairBranch[d]), margin)) {
             uint4 li = __ldg(&r.meshLeafInfo[r.shapeId[i]]);
             uint32_t targetShape = r.shapeId[j];
             float4 plane;
@@ -755,12 +785,19 @@ __device__ __forceinline__ void survivorPrefilter(const Params& P) {
         uint2 ij = r.pairs[p];
         uint32_t src = pass ? ij.y : ij.x, dst = pass ? ij.x : ij.y;
         uint32_t node = __ldg(&r.meshSampleIndices[__ldg(&r.meshClusterRanges[cd.y]).x + sv.y]);
-        float4 plane = r.dpairPlane[d];
-        f3 arm, local;
-        bool keep = nodePrefilter(r, src, dst, node, xyz(r.dpairBranch[d]), &plane, arm, local, grow);
-        // A node certified outside the target by the distance-bound grid
-        // cannot be a contact (the exact query would find phi > 0).
-        if (keep && c.distanceGridEnabled && distanceBound(r, r.shapeId[dst], local) > grow) keep = false;
+        // Placement as nodePrefilter's; a node certified outside the target by
+        // the distance-bound grid cannot be a contact (the exact query would
+        // find phi > 0).  Each test only rejects, so the order is free: the
+        // grid first, one load that drops most, then the plane and the hull,
+        // a load a plane.
+        f3 arm = qrot(r.rotation[src], xyz(__ldg(&r.sample[__ldg(&r.sampleInfo[r.shapeId[src]].x) + node])) * r.body[src].x);
+        f3 local = qinv(r.rotation[dst], arm - xyz(r.dpairBranch[d])) / r.body[dst].x;
+        const uint32_t shape = r.shapeId[dst];
+        bool keep = !(c.distanceGridEnabled && distanceBound(r, shape, local) > grow);
+        if (keep) {
+            float4 plane = r.dpairPlane[d];
+            keep = nodeTests(r, shape, &plane, local, grow);
+        }
         r.survKeep[s] = keep ? 1u : 0u;
     }
 }

@@ -194,7 +194,6 @@ __global__ void k_byJCount(const __grid_constant__ Params P) { byJCount(P); }
 __global__ void k_byJFill(const __grid_constant__ Params P) { byJFill(P); }
 __global__ void k_byJSort(const __grid_constant__ Params P) { byJSort(P); }
 __global__ void k_pairSetup(const __grid_constant__ Params P) { pairSetup(P); }
-__global__ void k_pairMasks(const __grid_constant__ Params P) { pairMasks(P); }
 __global__ void k_resetContacts(const __grid_constant__ Params P) {
     if (P.r.control[0] == 0) resetContacts(P.r, P.c, true);
 }
@@ -637,7 +636,6 @@ static void cullBuild(const Params& P, cudaStream_t s) {
     const Config& c = P.c;
     if (c.meshGeometry == 0) return;
     uint32_t T = 256, g = grid(c.cullBlocksPerSM, 8);
-    k_pairMasks<<<g, T, 0, s>>>(P);
     k_leafCull<<<g, T, 0, s>>>(P);
     launch_step_scan(r, r.dpairLeafCount, r.dpairCandOffset, ScanCount{r.control + 1, c.pairCapacity, 2, 0}, true,
                 r.work + W_CANDIDATES, r.work + W_FILTER, s);

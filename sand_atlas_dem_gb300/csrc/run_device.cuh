@@ -100,7 +100,7 @@ namespace rare {
 #define RARE(name) static __device__ __noinline__ void name(const Params& P) { sdg::name(P); }
 #define RARE_LIVE(name) static __device__ __noinline__ void name(const Params& P, bool live) { sdg::name(P, live); }
 RARE(binsClear) RARE(binsFill) RARE(binsOrder) RARE(pairsCountWarp) RARE(pairsEmitWarp) RARE(byJReset)
-RARE(byJCount) RARE(byJFill) RARE(byJSort) RARE(pairMasks) RARE(leafEmit) RARE(nodeFilter) RARE(survivorList)
+RARE(byJCount) RARE(byJFill) RARE(byJSort) RARE(leafEmit) RARE(nodeFilter) RARE(survivorList)
 RARE(survivorPrefilter) RARE(walkList)
 RARE_LIVE(leafCull) RARE_LIVE(certifyBuild) RARE_LIVE(nodeCertify) RARE_LIVE(nodeWalkSlow)
 #undef RARE
@@ -170,8 +170,6 @@ __global__ void __launch_bounds__(Threads, 1) k_run(const __grid_constant__ RunA
         RUN_SYNC();
         if (first) r.work[W_MOVED] = 0;
         if (Mesh && r.work[W_FILTER] != 0) {
-            rare::pairMasks(P);
-            RUN_SYNC();
             rare::leafCull(P, live);
             RUN_SYNC();
             if (!runScan(barrier, live, r, r.dpairLeafCount, r.dpairCandOffset, 2 * activePairs(r, c), true,
