@@ -110,6 +110,14 @@ def tree_levels(counts, leaf, small=256):
     return [tuple(level) for level in levels]
 
 
-def tree_launches(counts, leaf):
-    """Kernel launches of one ``sdg_median_trees`` call."""
-    return 2 + sum(2 + (small > 0) + 12 * (large > 0) for _, _, small, large in tree_levels(counts, leaf))
+def tree_launches(counts, leaf, small=256, middle=8192):
+    """Kernel launches of one ``sdg_median_trees`` call: two, and per level the
+    reduction and the nodes, the shared-memory sorts (by rank, by a CTA's radix
+    passes) and the four radix passes where the level has such nodes."""
+    sizes, total = {int(c) for c in counts}, 2
+    while sizes:
+        inner = {m for m in sizes if m > leaf}
+        total += 2 + any(m <= small for m in inner) + any(small < m <= middle for m in inner)
+        total += 12 * any(m > middle for m in inner)
+        sizes = {half for m in inner for half in (m // 2, m - m // 2)}
+    return total

@@ -73,6 +73,15 @@ def test_large_shape(gpu_library):
     same(device_median_trees(items, 64), host_median_trees(items, 64))
 
 
+@pytest.mark.parametrize("sizes", [[257], [511, 512, 513], [8191, 8192], [16385, 300, 8192, 257], [16383, 16384]])
+def test_sorts_by_size(gpu_library, sizes):
+    """Edges of the sorts: a node's items in one CTA (257 to 8,192), its last
+    warp short, nodes of several sorts on one level."""
+    rng = np.random.default_rng(sum(sizes))
+    items = [(cloud(rng, n, k % 2 == 0), None, None) for k, n in enumerate(sizes)]
+    same(device_median_trees(items, 16), host_median_trees(items, 16))
+
+
 @pytest.mark.parametrize("kind,count", [("uneven", 12), ("f8", 4)])
 def test_packed_library_matches_host(gpu_library, kind, count):
     library = synthetic_library(kind, count)
