@@ -188,3 +188,25 @@ def test_both_cell_list_paths_give_the_reference_pairs(gpu_library, pairs_per_pa
     np.testing.assert_array_equal(gpu_buffer(g, "pairs", np.uint32, pairs, 2), o.buffers["pairs"][:pairs])
     n = spec.particles
     np.testing.assert_array_equal(gpu_buffer(g, "pairOffsets", np.uint32, n, 1), o.buffers["pairOffsets"][:n].reshape(n, 1))
+
+
+@pytest.mark.parametrize("spacing", [1.05, 0.8])
+def test_pair_rows_longer_than_their_scratch(gpu_library, spacing):
+    """The pair search keeps a grain's first partners for the emit pass in a
+    row of pairs_per_particle words; a grain with more is searched again.  With
+    just enough pairs for all grains on average the low ids have more, the high
+    ids fewer: the pair list is the oracle's either way."""
+    from dataclasses import replace
+
+    library, spec, case = lattice_case(spacing=spacing)
+    o = build(OracleEngine, library, spec, case)
+    o.initialize()
+    n, pairs = spec.particles, int(o.check_errors()[1])
+    room = -(-pairs // n)
+    starts = o.buffers["pairOffsets"][:n].reshape(-1).astype(np.int64)
+    counts = np.diff(np.append(starts, pairs))
+    assert counts.max() > room > counts.min()
+    g = build(Engine, library, replace(spec, pairs_per_particle=room), case)
+    g.initialize()
+    assert g.check_errors()[1] == pairs and g.pair_capacity == room * n
+    np.testing.assert_array_equal(gpu_buffer(g, "pairs", np.uint32, pairs, 2), o.buffers["pairs"][:pairs])
