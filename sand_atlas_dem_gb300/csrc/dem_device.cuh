@@ -758,7 +758,14 @@ __device__ __forceinline__ uint32_t gridCell(const Res& r, uint32_t shape, f3 lo
 __device__ __forceinline__ float distanceBound(const Res& r, uint32_t shape, f3 local) {
     uint32_t cell = gridCell(r, shape, local);
     if (cell == 0xFFFFFFFFu) return -1e30f;
-    return __ldg(&r.distanceGrid[size_t(shape) * GRID * GRID * GRID + cell]);
+    const float4 info = __ldg(&r.distanceGridInfo[shape]);
+    const f3 centre = xyz(info) + mk(__fmul_rn(float(cell % GRID) + 0.5f, info.w),
+                                     __fmul_rn(float((cell / GRID) % GRID) + 0.5f, info.w),
+                                     __fmul_rn(float(cell / (GRID * GRID)) + 0.5f, info.w));
+    // The cell's value allows its half diagonal; the point is nearer to the centre.
+    const float reach = __fmul_rn(__fmul_rn(0.8660254f, info.w), 1.001f);
+    const float spare = __fsub_rn(reach, __fmul_rn(1.001f, length(local - centre)));
+    return __fadd_rn(__ldg(&r.distanceGrid[size_t(shape) * GRID * GRID * GRID + cell]), fmaxf(spare, 0.0f));
 }
 // Triangle list of a grid cell, 256 bytes: word 0 the limit L and word 1 the
 // distance d1 of the nearest triangle, both from the cell centre (floats);
