@@ -1044,23 +1044,22 @@ __device__ __forceinline__ void certifyBuild(const Params& P, bool live) {
     if (!live || r.work[W_FILTER] == 0) return;
     uint32_t n = min(r.work[W_KEPT], c.survivorCapacity);
     const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]), reach = certificateReach(margin);
-    for (uint32_t base = 0; base < n; base += gstride()) {
-        uint32_t t = base + gtid();
+    uint32_t slept = 0;
+    for (uint32_t t = gtid(); t < n; t += gstride()) {
         bool asleep = false;
-        if (t < n) {
-            if (c.cellListsEnabled) {
-                WalkNode w = walkNode(r, t);
-                float4 f;
-                if (cellQuery(r, r.shapeId[w.rec.y], w.local, reach, r.walkCert + size_t(CERT_ROWS) * t, f)) {
-                    asleep = fallsAsleep(w, f.w, margin);
-                    r.walkState[t] = asleep ? DORMANT : CERTIFIED;
-                }
+        if (c.cellListsEnabled) {
+            WalkNode w = walkNode(r, t);
+            float4 f;
+            if (cellQuery(r, r.shapeId[w.rec.y], w.local, reach, r.walkCert + size_t(CERT_ROWS) * t, f)) {
+                asleep = fallsAsleep(w, f.w, margin);
+                r.walkState[t] = asleep ? DORMANT : CERTIFIED;
             }
-            r.survKeep[t] = asleep ? 0u : 1u;
         }
-        uint32_t slept = __syncthreads_count(asleep);
-        if (threadIdx.x == 0 && slept) atomicAdd(&r.work[W_DORMANT], slept);
+        r.survKeep[t] = asleep ? 0u : 1u;
+        slept += asleep;
     }
+    slept = __reduce_add_sync(0xffffffffu, slept);
+    if (laneId() == 0 && slept) atomicAdd(&r.work[W_DORMANT], slept);
 }
 // The listed active slots, from their grid cells' triangle lists: a warp a
 // slot where there are few (cellQueryWarp), a lane a slot where many lapsed at
