@@ -5,11 +5,16 @@
 // (cpu_scheduling.slang:53-91): pair index, then direction, then leaf cluster
 // in preorder, then node in meshSampleIndices order.  The collector keeps it
 // with no atomics on contact slots: a flat leaf cull per directed pair, an
-// exclusive scan to (directed pair, leaf) work items, one warp per item for
-// the exact node queries (two nodes per lane, ballot hit masks), an
-// exclusive scan of hit counts, and an emit pass that recomputes only the
-// hits.  The history merge and the gather then walk sorted runs instead of a
-// hash table and linked lists, so every run is reproducible bit for bit.
+// exclusive scan to (directed pair, leaf) work items, a filter per item (a
+// ballot mask of its nodes), a scan to surviving nodes and a scan to the stored
+// exact-query slots, which are therefore in contact order.  A step queries the
+// slots that are awake and marks its hits as bits; a hit's contact index is the
+// number of hit bits before it.  The history merge and the gather then walk
+// sorted runs instead of a hash table and linked lists, so every run is
+// reproducible bit for bit.
+//
+// Every phase is a device function: kernels_contacts.cu launches each as a
+// kernel, run_device.cuh runs them all in one.
 #pragma once
 #include <cuda_runtime.h>
 #include "culler.cuh"

@@ -13,7 +13,7 @@ import pytest
 
 from oracle.engine import OracleEngine
 from sand_atlas_dem_gb300.engine import Engine
-from tests.specimens import build, lattice_case
+from tests.specimens import build, lattice_case, walled_lattice
 
 pytestmark = pytest.mark.gpu
 COUNTS = ("step", "candidate_pairs", "active_surface_contacts", "active_grain_pairs")
@@ -55,3 +55,34 @@ def test_diagnostics_match_oracle(gpu_library):
         oo = o.diagnostics()
         compare(g.diagnostics(), oo, 1e-5)
     assert oo["sliding_fraction"] > 0 and oo["normal_contact_dissipation"] > 0 and oo["p"] > 0
+
+
+@pytest.mark.parametrize("side,spacing", [(4, 0.985), (4, 1.6), (7, 1.05)])
+def test_group_edges_match_oracle(gpu_library, side, spacing):
+    """The reductions by groups of 256 rows: a short last group, several groups
+    (343 grains), a specimen without a pair; as above, to float64 rounding."""
+    library, spec, case = lattice_case(side=side, spacing=spacing)
+    o = build(OracleEngine, library, spec, case, threads=8)
+    g = build(Engine, library, spec, case)
+    o.initialize()
+    g.initialize()
+    want = o.diagnostics()
+    assert (want["candidate_pairs"] == 0) == (spacing == 1.6)
+    compare(g.diagnostics(), want, 0)
+
+
+@pytest.mark.parametrize("side", [1, 3, 7])
+def test_wall_rows_match_oracle(gpu_library, side):
+    """The per-wall rows of the same reduction: one grain, several groups."""
+    library, spec, case, _ = walled_lattice(side=side)
+    o = build(OracleEngine, library, spec, case, threads=8)
+    g = build(Engine, library, spec, case)
+    o.initialize()
+    g.initialize()
+    want, got = o.diagnostics(), g.diagnostics()
+    compare(got | {"walls": 0}, want | {"walls": 0}, 0)
+    assert len(got["walls"]) == len(want["walls"]) == 7
+    for a, b in zip(got["walls"], want["walls"]):
+        assert a.keys() == b.keys()
+        for key in a:
+            np.testing.assert_array_equal(np.asarray(a[key]), np.asarray(b[key]), err_msg=key)
