@@ -102,11 +102,6 @@ WORKLOADS = {
                            pairs_per_particle=8, contacts_per_particle=256, strain_rate_per_s=0.0),
 }
 DATA = ROOT / "sand_atlas_dem_gb300" / "data"
-# DRAM bytes (read + write) of one reuse step's exact queries
-# (k_nodeWalkKnown and k_nodeWalkStaged; k_nodeWalkSlow returns at once on a
-# short list) from an ncu capture of the same workload
-# (profiles/walk-dense-10k.md); None where not captured.
-WALK_TRAFFIC = {"dense-10k": 40.03e6 + 0.48e6 + 9.26e6}
 # work[] counters (csrc/dem_device.cuh): the stored node-filter results and
 # the neighbour-list rebuilds.
 W_FILTER_MARGIN, W_FILTER_BUILDS, W_FILTER_STEPS, W_CERTIFIED, W_REBUILDS, W_DORMANT = 8, 9, 10, 15, 17, 18
@@ -546,7 +541,7 @@ def run_gb300(args, cpu=True):
             "peak_source": peak_kind,
             "unit": "GB/s",
             "frac": walk_gbs / hbm,
-            "traffic": WALK_TRAFFIC.get(w.name),
+            "traffic": None,
             "algorithmic_bytes": walk_bytes,
             "kernel_ms": phase_ms["node_query"],
             "launch_group": group_name,

@@ -13,7 +13,7 @@ import pytest
 
 from oracle.engine import OracleEngine
 from sand_atlas_dem_gb300.engine import Engine
-from tests.specimens import build, lattice_case, walled_lattice
+from tests.specimens import build, lattice_case
 
 pytestmark = pytest.mark.gpu
 COUNTS = ("step", "candidate_pairs", "active_surface_contacts", "active_grain_pairs")
@@ -69,20 +69,3 @@ def test_group_edges_match_oracle(gpu_library, side, spacing):
     want = o.diagnostics()
     assert (want["candidate_pairs"] == 0) == (spacing == 1.6)
     compare(g.diagnostics(), want, 0)
-
-
-@pytest.mark.parametrize("side", [1, 3, 7])
-def test_wall_rows_match_oracle(gpu_library, side):
-    """The per-wall rows of the same reduction: one grain, several groups."""
-    library, spec, case, _ = walled_lattice(side=side)
-    o = build(OracleEngine, library, spec, case, threads=8)
-    g = build(Engine, library, spec, case)
-    o.initialize()
-    g.initialize()
-    want, got = o.diagnostics(), g.diagnostics()
-    compare(got | {"walls": 0}, want | {"walls": 0}, 0)
-    assert len(got["walls"]) == len(want["walls"]) == 7
-    for a, b in zip(got["walls"], want["walls"]):
-        assert a.keys() == b.keys()
-        for key in a:
-            np.testing.assert_array_equal(np.asarray(a[key]), np.asarray(b[key]), err_msg=key)
