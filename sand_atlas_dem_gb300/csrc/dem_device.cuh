@@ -185,6 +185,7 @@ constexpr int W_DORMANT = 18;       // dormant slots in the stored exact-query l
 constexpr int W_LAPSED = 20;        // stored walk slots without a certificate that holds this step
 constexpr int W_ACTIVE = 21;        // stored walk slots listed as live when the results were built
 constexpr int W_MOVED = 22;         // a grain asks for a neighbour build (cleared when control[4] is set)
+constexpr int W_WALL_HITS = 23;     // plane contacts listed this step (hitScratch)
 constexpr int W_CULL_ROWS = 19;     // kept survivors in the culler's shape-sorted list
 
 struct Params {

@@ -329,3 +329,23 @@ def test_wall_and_grain_histories_coexist_and_wall_work_reduces_over_bodies(gpu_
     total_moment += state["torque"][:, :3].sum(0) * engine.energy_unit
     assert np.linalg.norm(total_moment + row["walls"][0]["reaction_moment_origin"]) < np.linalg.norm(
         total_force) * 0.006 * 1e-5
+
+
+@pytest.mark.parametrize("geometry,nodes", [("sdf", 1700), ("sdf", 3001), ("mesh", None)])
+def test_deep_cut_lists_every_round(gpu_library, geometry, nodes):
+    """One grain cut in the middle: its item has more rounds of 32 nodes with a
+    contact than a warp holds at once (SDF: 3,001 nodes in order; mesh: 2,562
+    in cluster order), or just as many (1,700); keys, order and records are the oracle's."""
+    from sand_atlas_dem_gb300.shapes import perturbed_grain
+
+    shape = analytic_sphere(samples=nodes) if geometry == "sdf" else perturbed_grain(16, seed=3)
+    spec = Experiment(periodic=False, particles=1, timestep=1e-9, max_overlap_fraction=0.95, contact_geometry=geometry,
+                      contacts_per_particle=4096, planes=[plane(offset=0.0021), plane((0, 0, -1), -0.0019)])
+    o, g = (cls(ShapeLibrary([shape]), spec, [[0.002] * 3], [0.006] * 3, [0], [1]) for cls in (OracleEngine, Engine))
+    o.initialize()
+    g.initialize()
+    so, sg = o.state(), g.state()
+    assert so["contacts"] == sg["contacts"] > 1024
+    np.testing.assert_array_equal(sg["meta"], so["meta"])
+    for name in ("normalArea", "slip", "force", "torque"):
+        assert sg[name].tobytes() == so[name].tobytes(), name
