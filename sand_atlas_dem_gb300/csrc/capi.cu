@@ -143,13 +143,11 @@ int unpack_params(void* const* buffers, const uint64_t* bytes, const double* val
 // stored and rebuilt only on the steps whose motion check asks for it.
 static bool storedFilters(const Config& c) { return c.meshGeometry != 0 && storedKeep(c); }
 
-// Contacts and their law; `build(body)` runs the filter build where the
-// results are stored.
-template <class Build>
-static void collectAndResolve(const Params& P, cudaStream_t s, Build&& build) {
+// Contacts and their law, all parts launched.
+static void collectAndResolve(const Params& P, cudaStream_t s) {
     if (storedFilters(P.c) || P.c.meshGeometry == 0) {
         launch_contacts("collectHead", P, 0, s);
-        if (P.c.meshGeometry != 0) build([&](cudaStream_t b) { launch_contacts("collectBuild", P, 0, b); });
+        if (P.c.meshGeometry != 0) launch_contacts("collectBuild", P, 0, s);
         launch_contacts("collectTail", P, 0, s);
         launch_contacts("resolveWalls", P, 0, s);
     } else {
@@ -162,7 +160,7 @@ void launch_forces(const Params& P, cudaStream_t s, bool captureKinematics) {
     const Config& c = P.c;
     if (c.normalViscosity > 0 && captureKinematics) launch_state("captureContactKinematics", P, c.N, s);
     launch_contacts("neighbours", P, c.N, s);
-    collectAndResolve(P, s, [&](auto&& body) { body(s); });
+    collectAndResolve(P, s);
     launch_contacts("gather", P, c.N, s);
     launch_contacts("gatherWallRows", P, c.N, s);
     if (c.activeTimestep) launch_state("checkContactTimestep", P, c.N, s);
@@ -172,9 +170,14 @@ void launch_forces(const Params& P, cudaStream_t s, bool captureKinematics) {
 // is fused into beginStep when the normal law is viscous.  The two parts that
 // most steps skip -- the neighbour build (device flag control[4], set by
 // beginStep and advanceCell) and the filter build (work[W_FILTER], set by the pair set-up's
-// motion check) -- go through `branch(flag, body)`: plain launches run the
-// body on s (its kernels return at once when the flag is clear); graph
-// capture makes it the body of a conditional node keyed on the flag.
+// motion check) -- go through `branch(flag, other, body, rest)`: plain launches
+// run the bodies on s (their kernels return at once when their flag is clear);
+// graph capture makes them, in that order, the body of one conditional node
+// that runs where either flag is set.  A conditional node that does not run
+// costs 10 us, so with stored filters both parts share one: the pair set-up
+// and its motion check come first on the steps that keep their pairs, and in
+// the body, after the new pairs, on those that do not (327 -> XX us at 50,000
+// grains).
 template <class Branch>
 static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
     const Config& c = P.c;
@@ -185,8 +188,19 @@ static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
     launch_state("beginStep", B, c.N, s);
     launch_state("advanceCell", P, c.specimens, s);
     if (c.wallCount) launch_state("advanceWalls", P, 1, s);
-    branch(P.r.control + 4, [&](cudaStream_t b) { launch_contacts("neighbours", P, c.N, b); });
-    collectAndResolve(P, s, [&](auto&& body) { branch(P.r.work + W_FILTER, body); });
+    auto neighbours = [&](cudaStream_t b) { launch_contacts("neighbours", P, c.N, b); };
+    if (storedFilters(c)) {
+        launch_contacts("collectHeadKept", P, 0, s);
+        branch(P.r.control + 4, P.r.work + W_FILTER, neighbours, [&](cudaStream_t b) {
+            launch_contacts("collectHeadRebuilt", P, 0, b);
+            launch_contacts("collectBuild", P, 0, b);
+        });
+        launch_contacts("collectTail", P, 0, s);
+        launch_contacts("resolveWalls", P, 0, s);
+    } else {
+        branch(P.r.control + 4, P.r.control + 4, neighbours, [](cudaStream_t) {});
+        collectAndResolve(P, s);
+    }
     if (!c.wallCount && !c.activeTimestep) {
         launch_contacts("gatherFinish", P, c.N, s);
         return;
@@ -198,12 +212,15 @@ static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
 }
 
 void launch_step(const Params& P, cudaStream_t s) {
-    stepSequence(P, s, [&](const uint32_t*, auto&& body) { body(s); });
+    stepSequence(P, s, [&](const uint32_t*, const uint32_t*, auto&& body, auto&& rest) {
+        body(s);
+        rest(s);
+    });
 }
 
-// Sets a conditional node's value from a device flag (graph replay).
-__global__ void k_setCondition(cudaGraphConditionalHandle handle, const uint32_t* flag) {
-    cudaGraphSetConditional(handle, *flag != 0u ? 1u : 0u);
+// Sets a conditional node's value from two device flags (graph replay).
+__global__ void k_setCondition(cudaGraphConditionalHandle handle, const uint32_t* flag, const uint32_t* other) {
+    cudaGraphSetConditional(handle, (*flag | *other) != 0u ? 1u : 0u);
 }
 
 // Committed/new history sides swap every step (gpu.py:725).
@@ -303,10 +320,10 @@ static uint32_t kernelNodes(cudaGraph_t graph) {
     return k;
 }
 
-// One step as a graph: the step sequence captured on s, each branch an IF
+// One step as a graph: the step sequence captured on s, its branch an IF
 // node whose condition a one-thread kernel sets from the branch's device
-// flag just before it (the condition defaults to 1 -- run -- on every
-// launch), its body captured on aux into the node's body graph.
+// flags just before it (the condition defaults to 1 -- run -- on every
+// launch), the two bodies captured on aux into the node's body graph.
 static int capture(const Params& P, cudaStream_t s, cudaStream_t aux, cudaGraphExec_t* out, StepKernels* kernels) {
     cudaGraph_t graph = nullptr;
     int rc = record(cudaGraphCreate(&graph, 0), "graph create");
@@ -315,15 +332,13 @@ static int capture(const Params& P, cudaStream_t s, cudaStream_t aux, cudaGraphE
                 "begin capture");
     if (rc) { cudaGraphDestroy(graph); return rc; }
     StepKernels counted;
-    int branches = 0;
-    stepSequence(P, s, [&](const uint32_t* flag, auto&& body) {
-        int index = branches++;
+    stepSequence(P, s, [&](const uint32_t* flag, const uint32_t* other, auto&& body, auto&& rest) {
         if (rc) return;
         cudaGraphConditionalHandle handle;
         rc = record(cudaGraphConditionalHandleCreate(&handle, graph, 1u, cudaGraphCondAssignDefault),
                     "conditional handle");
         if (rc) return;
-        k_setCondition<<<1, 1, 0, s>>>(handle, flag);
+        k_setCondition<<<1, 1, 0, s>>>(handle, flag, other);
         cudaStreamCaptureStatus status;
         cudaGraph_t target = nullptr;
         const cudaGraphNode_t* deps = nullptr;
@@ -347,9 +362,20 @@ static int capture(const Params& P, cudaStream_t s, cudaStream_t aux, cudaGraphE
                                                   cudaStreamCaptureModeThreadLocal), "begin body capture");
         if (rc) return;
         body(aux);
+        // The nodes the rest follows.
+        rc = record(cudaStreamGetCaptureInfo(aux, &status, nullptr, &target, &deps, &edges, &count), "body capture info");
+        const std::vector<cudaGraphNode_t> last(deps, deps + (rc ? 0 : count));
         cudaGraph_t done = nullptr;
+        int end = record(cudaStreamEndCapture(aux, &done), "end body capture");
+        rc = rc ? rc : end;
+        if (rc) return;
+        counted.branch[0] = kernelNodes(bodyGraph);
+        rc = record(cudaStreamBeginCaptureToGraph(aux, bodyGraph, last.data(), nullptr, last.size(),
+                                                  cudaStreamCaptureModeThreadLocal), "begin body capture");
+        if (rc) return;
+        rest(aux);
         rc = record(cudaStreamEndCapture(aux, &done), "end body capture");
-        if (!rc && index < 2) counted.branch[index] = kernelNodes(bodyGraph);
+        if (!rc) counted.branch[1] = kernelNodes(bodyGraph) - counted.branch[0];
     });
     cudaGraph_t captured = nullptr;
     int end = record(cudaStreamEndCapture(s, &captured), "end capture");

@@ -197,6 +197,21 @@ __global__ void k_pairSetup(const __grid_constant__ Params P) { pairSetup(P); }
 __global__ void k_resetContacts(const __grid_constant__ Params P) {
     if (P.r.control[0] == 0) resetContacts(P.r, P.c, true);
 }
+// The same before a step's neighbour build: the pairs, and their set-up, are
+// known only where the step keeps them ...
+__global__ void k_resetContactsKept(const __grid_constant__ Params P) {
+    if (P.r.control[0] == 0) resetContacts(P.r, P.c, P.r.control[4] == 0);
+}
+__global__ void k_pairSetupKept(const __grid_constant__ Params P) {
+    if (P.r.control[4] == 0) pairSetup(P);
+}
+// ... else after the build.
+__global__ void k_pairSetupRebuilt(const __grid_constant__ Params P) {
+    const Res& r = P.r;
+    if (r.control[4] == 0) return;
+    if (gtid() == 0 && r.work[W_FILTER_PAIRS] != r.control[1]) atomicOr(&r.work[W_FILTER], 1u);
+    pairSetup(P);
+}
 __global__ void k_leafCull(const __grid_constant__ Params P) { leafCull(P, P.r.control[0] == 0); }
 __global__ void k_leafEmit(const __grid_constant__ Params P) { leafEmit(P); }
 __global__ void __launch_bounds__(256) k_nodeFilter(const __grid_constant__ Params P) { nodeFilter(P); }
@@ -783,6 +798,11 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
     else if (name == "collect") contacts(P, s);
     else if (name == "collectCull") collectCull(P, s);
     else if (name == "collectHead") collectHead(P, s);
+    else if (name == "collectHeadKept") {
+        k_resetContactsKept<<<1, 1, 0, s>>>(P);
+        k_pairSetupKept<<<grid(c.cullBlocksPerSM, 8), T, 0, s>>>(P);
+    }
+    else if (name == "collectHeadRebuilt") k_pairSetupRebuilt<<<grid(c.cullBlocksPerSM, 8), T, 0, s>>>(P);
     else if (name == "prefetch") {
         if (c.meshGeometry != 0) k_prefetch<<<grid(0, 2), 64, 0, s>>>(P);
     }
