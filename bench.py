@@ -44,10 +44,10 @@ Data are synthetic (seeded); the reference's Hostun assets are not used.
              builds and neighbour rebuilds its motion caused, the step-time
              median, 99th percentile and maximum, and its kernel launches.
 ``gpu_launches``: kernel launches of the timed steps: each captured step runs
-             its unconditional kernels; the neighbour-build and filter-build
-             bodies are conditional graph nodes that run only on the steps
-             whose device flag asks for them (counted from the device's
-             rebuild and build counters).
+             its unconditional kernels; the neighbour and filter builds are
+             the body of a conditional graph node that runs only on the
+             steps whose device flags ask for one (counted from the device's
+             rebuild and build counters); a persistent step is one launch.
 ``e2e``    : the public API a caller uses (``Engine.advance`` chunks of 10
              steps plus ``diagnostics()``), host wall clock, including the
              host<->device traffic of those calls (counted by the engine).
@@ -364,13 +364,13 @@ def algorithmic_bytes(n, pairs, contacts, items, nodes, survivors, kept, rebuild
 
 def launches(e, steps, rebuilds, builds):
     """Kernel launches of ``steps`` graph-replayed steps: the ones every step
-    runs, plus the neighbour-build body on rebuild steps and the filter-build
-    body on filter-build steps."""
+    runs, plus the neighbour and filter builds' on the steps that take either
+    (one conditional body holds both)."""
     lib, h = e.lib, e._native
     if lib.sdg_engine_persistent(h) == 1:
         return steps  # each step its own persistent launch, the bodies inside
-    return (lib.sdg_engine_kernels_per_step(h) * steps + lib.sdg_engine_branch_kernels(h, 0) * rebuilds
-            + lib.sdg_engine_branch_kernels(h, 1) * builds)
+    neighbours, filters = lib.sdg_engine_branch_kernels(h, 0), lib.sdg_engine_branch_kernels(h, 1)
+    return lib.sdg_engine_kernels_per_step(h) * steps + (neighbours + filters) * max(rebuilds, builds if filters else 0)
 
 
 def counters(e):

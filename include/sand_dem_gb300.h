@@ -276,17 +276,17 @@ int sdg_culler_inside_max_cells(const void* points, const void* predictions, uin
                                 void* counts, void* stream);
 
 /*
- * Kernel launches of a captured step that skips both conditional bodies (0
+ * Kernel launches of a captured step that skips the conditional body (0
  * before the first advance).  The captured step holds the neighbour build
- * and, with stored filter results, the filter build as conditional-node
- * bodies keyed on device flags (the reference re-encodes the rebuild
+ * and, with stored filter results, the filter build as the body of one
+ * conditional node that runs where either's device flag is set (the reference re-encodes the rebuild
  * dispatches every step and lets them exit early, gpu.py:547-565).
  */
 int sdg_engine_kernels_per_step(void* engine);
 /*
- * Kernel launches inside conditional body `branch` of a captured step: 0 =
- * the neighbour build (steps whose rebuild flag is set), 1 = the filter build
- * (steps that build the stored filter results).  -1 for a bad argument.
+ * Kernel launches in part `branch` of that body: 0 = the neighbour build, 1 =
+ * the filter build (0 launches without stored filter results).  Each part's
+ * kernels return at once where their own flag is clear.  -1 for a bad argument.
  */
 int sdg_engine_branch_kernels(void* engine, int branch);
 /* 1 if the last sdg_engine_advance ran its steps in one persistent launch. */

@@ -176,7 +176,7 @@ void launch_forces(const Params& P, cudaStream_t s, bool captureKinematics) {
 // that runs where either flag is set.  A conditional node that does not run
 // costs 10 us, so with stored filters both parts share one: the pair set-up
 // and its motion check come first on the steps that keep their pairs, and in
-// the body, after the new pairs, on those that do not (327 -> XX us at 50,000
+// the body, after the new pairs, on those that do not (327 -> 316 us at 50,000
 // grains).
 template <class Branch>
 static void stepSequence(const Params& P, cudaStream_t s, Branch&& branch) {
@@ -239,8 +239,8 @@ static Params swapSides(const Params& P) {
 }
 
 // Kernel launches of a captured step: those every step runs, and those of
-// the neighbour-build and filter-build bodies (run only on steps whose flag
-// is set).
+// the neighbour-build and filter-build parts of its conditional body (run only
+// on steps where either flag is set).
 struct StepKernels {
     uint32_t always = 0, branch[2] = {0, 0};
 };
@@ -271,16 +271,16 @@ struct Engine {
 };
 
 // The persistent step serves up to 300,000 active slots (both forms measured
-// beside it: at 185 k it takes 89 us against the launched step's 121, at
-// 425 k 376 against 354); before the first report a dense packing's 18 slots
+// beside it: at 185 k it takes 87 us against the launched step's 109, at
+// 425 k 265 against 240); before the first report a dense packing's 18 slots
 // a grain are assumed.  Up to 6,000 grains its phases are latency-bound and
 // take the 512-thread form.
 constexpr uint32_t RUN_ACTIVE_SLOTS = 300'000, RUN_SLOTS_PER_GRAIN = 18, RUN_NARROW_GRAINS = 6'000;
 // Steps of one launch (even: each starts on the same history side): a few
 // milliseconds at a time, so that a long chunk shares the GPU.
 constexpr uint32_t RUN_STEPS = 64;
-// With the SDF geometry up to 2,048 grains (68 us against 78 launched at
-// 1,000; 101 against 98 at 2,197).
+// With the SDF geometry up to 2,048 grains (73 us against 79 launched at
+// 1,000; 107 against 100 at 2,197).
 constexpr uint32_t RUN_SDF_GRAINS = 2'048;
 static bool cooperative() {
     static const bool supported = [] {
@@ -641,16 +641,15 @@ static const StepKernels& stepKernels(Engine* e) {
     return e->kernels;
 }
 
-// Kernel launches of a captured step that skips both conditional bodies (0
+// Kernel launches of a captured step that skips the conditional body (0
 // before the first advance).
 int sdg_engine_kernels_per_step(void* engine) {
     Engine* e = static_cast<Engine*>(engine);
     return e ? int(stepKernels(e).always) : -1;
 }
 
-// Kernel launches inside conditional body `branch` of a captured step: 0 =
-// the neighbour build (run on rebuild steps), 1 = the filter build (run on
-// steps that build the stored filter results; absent without them).
+// Kernel launches in part `branch` of the conditional body of a captured step:
+// 0 = the neighbour build, 1 = the filter build (absent without stored results).
 int sdg_engine_branch_kernels(void* engine, int branch) {
     Engine* e = static_cast<Engine*>(engine);
     if (!e || branch < 0 || branch > 1) return -1;

@@ -9,8 +9,8 @@ namespace sdg {
 // CTA per SM going through all of them with a barrier over the grid in
 // between, and the neighbour and filter builds taken when their device flags
 // ask for them.  What a launched step costs besides its kernels -- 4 us per
-// graph launch, 1.2 us per kernel boundary and 10 us per conditional node
-// that does not run (two a step) -- becomes five barriers of 1.3 us.
+// graph launch, 1.2 us per kernel boundary and 10 us for a conditional node
+// that does not run -- becomes five barriers of 1.3 us.
 //
 // The barriers carry everything a kernel boundary would: writes before one
 // are visible after it on every SM.  Branches around barriers depend only on
@@ -19,10 +19,11 @@ namespace sdg {
 //
 // Two widths: 512 threads (up to 128 registers, no spills) where the phases
 // are chains of dependent latencies, 768 (80 registers) where they fill the
-// SMs.  Step, us (512 / 768 / launched): 125 grains 50 / 54 / 78; 1,000 loose
-// 36 / 40 / 69; 343 walled 95 / 102 / 129; 10,000 dense (185 k active slots)
-// 93 / 89 / 121; but 4,913 walled (425 k) 402 / 376 / 354 and 50,000 (1.1 M)
-// 436 / 372 / 353: there the launched kernels' own register budgets win.
+// SMs (125 grains 50 / 54 us, 1,000 loose 36 / 40, 343 walled 95 / 102, 10,000
+// dense 93 / 89 when both were tried).  Step, us (persistent / launched): 125
+// grains 44 / 67; 1,000 loose 40 / 66; 343 walled 88 / 115; 10,000 dense (185 k
+// active slots) 87 / 109; but 4,913 walled (425 k) 265 / 240 and 50,000 (1.1 M)
+// 328 / 312: there the launched kernels' own register budgets win.
 struct GridBarrier {
     uint32_t* counter;
     uint32_t arrived = 0;
