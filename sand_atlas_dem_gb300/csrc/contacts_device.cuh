@@ -781,8 +781,7 @@ __device__ __forceinline__ void nodeFilter(const Params& P) {
         }
     }
 }
-// Source node, partner and target-frame position of survivor s (the same
-// expressions as nodePrefilter: the same arm and local bits).
+// Source node, partner and target-frame position of survivor s.
 struct SurvivorNode {
     uint32_t item, slot, src, dst, node;
     f3 arm, local;
@@ -803,8 +802,8 @@ __device__ __forceinline__ SurvivorNode survivorNode(const Res& r, uint32_t s) {
     v.local = qinv(r.rotation[v.dst], v.arm - xyz(r.dpairBranch[d])) / r.body[v.dst].x;
     return v;
 }
-// Exact placement, target-frame enclosure plane and hull of every survivor
-// of the one-dot test (nodePrefilter, one thread each): survKeep[s] = 1 for
+// Exact placement, distance grid, target-frame enclosure plane and hull of
+// every survivor of the one-dot test, a thread each: survKeep[s] = 1 for
 // the nodes that go on to the exact query.
 // When the exact-query list is stored with the filter results, this pass
 // runs only on build steps, with the plane, hull and grid tests grown by the
@@ -824,7 +823,7 @@ __device__ __forceinline__ void survivorPrefilter(const Params& P) {
         uint2 ij = r.pairs[p];
         uint32_t src = pass ? ij.y : ij.x, dst = pass ? ij.x : ij.y;
         uint32_t node = __ldg(&r.meshSampleIndices[__ldg(&r.meshClusterRanges[cd.y]).x + sv.y]);
-        // Placement as nodePrefilter's; a node certified outside the target by
+        // Placed with survivorNode's expressions; a node certified outside the target by
         // the distance-bound grid cannot be a contact (the exact query would
         // find phi > 0).  Each test only rejects, so the order is free: the
         // grid first, one load that drops most, then the plane and the hull,
@@ -2020,10 +2019,6 @@ constexpr uint32_t GATHER_CHAINS = 22;
 // Row stride: 16-byte rows for the replay's float4 reads; at 36 words a
 // quarter warp's reads (and a warp's word stores) touch every bank once.
 constexpr uint32_t GATHER_STRIDE = WARP + 4;
-__device__ __forceinline__ f3 shfl3(f3 v, int lane) {
-    return mk(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
-              __shfl_sync(0xffffffffu, v.z, lane));
-}
 // Lane `chain` replays its accumulator chain over the `count` terms of one
 // round, in order.  Every chain runs the same instructions: the compensated
 // step (y = t + low, next = acc + y, low = y - (next - acc)), whose residual

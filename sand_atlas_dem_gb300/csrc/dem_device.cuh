@@ -673,11 +673,11 @@ __device__ __forceinline__ void meshPairBounds(const Res& r, uint32_t direction,
     high = high + mk(pad, pad, pad);
 }
 // solver.slang:319-343; the directed-pair branch is precomputed (same bits).
-// Split in two so that work can be filtered between the cheap conservative
-// rejections and the exact query: nodePrefilter places the node in the
-// target's frame and applies, with `plane`, the reference CPU backend's
-// per-directed-pair enclosure-plane prefilter (cpu.py:56-76), then the hull
-// cull; nodeExact is the exact distance query and the contact record.  Both
+// Split so that work can be filtered between the cheap conservative rejections
+// and the exact query: nodeTests applies to a node placed in the target's
+// frame, with `plane`, the reference CPU backend's per-directed-pair
+// enclosure-plane prefilter (cpu.py:56-76), then the hull cull;
+// nodeContactWith makes the contact record of an exact distance.  Both
 // rejections are conservative and change no contact.  `grow` > 0 widens both
 // tests by that distance (for the stored filter results).
 __device__ __forceinline__ bool nodeTests(const Res& r, uint32_t targetShape, const float4* plane, f3 local,
@@ -690,16 +690,6 @@ __device__ __forceinline__ bool nodeTests(const Res& r, uint32_t targetShape, co
     }
     return meshMayContain(r, targetShape, local, grow);
 }
-__device__ __forceinline__ bool nodePrefilter(const Res& r, uint32_t src, uint32_t dst, uint32_t node, f3 branch,
-                                              const float4* plane, f3& arm, f3& local, float grow = 0.0f) {
-    uint32_t sid = r.shapeId[src];
-    float4 sp = __ldg(&r.sample[__ldg(&r.sampleInfo[sid].x) + node]);
-    float4 qs = r.rotation[src], qd = r.rotation[dst];
-    arm = qrot(qs, xyz(sp) * r.body[src].x);
-    local = qinv(qd, arm - branch) / r.body[dst].x;
-    return nodeTests(r, r.shapeId[dst], plane, local, grow);
-}
-// The contact record from the target's signed distance f at the node.
 // The contact record of a node whose target-frame query gave f, from the
 // node's sample `sp`, both grains' body rows and the target's rotation
 // (loaded by the caller); `src` is read only for the source-surface normal.
@@ -726,24 +716,7 @@ __device__ __forceinline__ bool nodeContactFrom(const Res& r, const Config& c, u
     float4 sp = __ldg(&r.sample[__ldg(&r.sampleInfo[sid].x) + node]);
     return nodeContactWith(r, c, src, sp, r.body[src], r.body[dst], r.rotation[dst], arm, f, pd, na);
 }
-__device__ __forceinline__ bool nodeExact(const Res& r, const Config& c, uint32_t src, uint32_t dst, uint32_t node,
-                                          f3 arm, f3 local, float4& pd, float4& na, uint32_t seed = 0xFFFFFFFFu) {
-    float4 f = meshDistance(r, r.shapeId[dst], local, false, seed);
-    return nodeContactFrom(r, c, src, dst, node, arm, f, pd, na);
-}
-__device__ __forceinline__ bool nodeContact(const Res& r, const Config& c, uint32_t src, uint32_t dst, uint32_t node,
-                                            f3 branch, float4& pd, float4& na, const float4* plane = nullptr) {
-    f3 arm, local;
-    if (!nodePrefilter(r, src, dst, node, branch, plane, arm, local)) return false;
-    return nodeExact(r, c, src, dst, node, arm, local, pd, na);
-}
 
-// Certified lower bound of the target shape's signed distance at `local`
-// (shape frame, unscaled), from its cell of the distance-bound grid.  The
-// signed distance to a closed mesh is 1-Lipschitz, so every point of a cell
-// lies at least phi(centre) - (half diagonal) from the surface; the grid
-// stores that bound less a slack above the FP32 error of the centre query.
-// Points outside the grid (outside the shape's root box) get -inf.
 // Index of the grid cell holding `local` in the shape's grid, or EMPTY
 // outside it.
 __device__ __forceinline__ uint32_t gridCell(const Res& r, uint32_t shape, f3 local) {
@@ -756,6 +729,12 @@ __device__ __forceinline__ uint32_t gridCell(const Res& r, uint32_t shape, f3 lo
         return 0xFFFFFFFFu;
     return (uint32_t(gz) * GRID + uint32_t(gy)) * GRID + uint32_t(gx);
 }
+// Certified lower bound of the target shape's signed distance at `local`
+// (shape frame, unscaled), from its cell of the distance-bound grid.  The
+// signed distance to a closed mesh is 1-Lipschitz, so every point of a cell
+// lies at least phi(centre) - (half diagonal) from the surface; the grid
+// stores that bound less a slack above the FP32 error of the centre query.
+// Points outside the grid (outside the shape's root box) get -inf.
 __device__ __forceinline__ float distanceBound(const Res& r, uint32_t shape, f3 local) {
     uint32_t cell = gridCell(r, shape, local);
     if (cell == 0xFFFFFFFFu) return -1e30f;
