@@ -982,16 +982,19 @@ __device__ __forceinline__ bool fallsAsleep(const WalkNode& w, float phi, float 
     return phi > __fadd_rn(sleep, slack);
 }
 __device__ __forceinline__ float certificateReach(float margin) { return __fadd_rn(__fmul_rn(2.01f, margin), 1e-4f); }
-// Appends the warp's flagged lanes' values to a list (called by whole warps).
+// Appends the warp's flagged lanes' values to a list of `room` words (called by
+// whole warps); the count goes on past them, the stores do not.
 // Few slots lapse, so few warps append: a block's one atomic for all of its
 // warps cost every block a barrier a round (a quarter of the query's stalls).
-__device__ __forceinline__ void appendWarp(bool flagged, uint32_t value, uint32_t* list, uint32_t* count) {
+__device__ __forceinline__ void appendWarp(bool flagged, uint32_t value, uint32_t* list, uint32_t room,
+                                           uint32_t* count) {
     const uint32_t ballot = __ballot_sync(0xffffffffu, flagged);
     if (ballot == 0) return;
     uint32_t base = 0;
     if (laneId() == 0) base = atomicAdd(count, uint32_t(__popc(ballot)));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (flagged) list[base + __popc(ballot & lanesBelow())] = value;
+    base += __popc(ballot & lanesBelow());
+    if (flagged && base < room) list[base] = value;
 }
 // The slot's contact record, in its scratch slot; whether it is a contact.
 __device__ __forceinline__ bool recordSlot(const Res& r, const Config& c, uint32_t t, const WalkNode& w, float4 f) {
@@ -1008,7 +1011,8 @@ __device__ __forceinline__ void lateHit(const SlotHits& hits, uint32_t i) {
     atomicAdd(&hits.sets[i / (32 * HIT_WORDS * HIT_GROUPS)], 1u);
 }
 // The active slots whose certificates hold: their hit bits and counts.  The
-// others are listed in survKeep.  Only the slots their build left awake are
+// others are listed in walkList (which lists built every step use; survKeep holds
+// keep flags and nothing else).  Only the slots their build left awake are
 // visited (walkActive): 185 of 449 thousand on a dense packing of 10,000
 // grains, and warps full of them instead of a third full.
 __device__ __forceinline__ void nodeQuery(const Params& P, bool live) {
@@ -1037,7 +1041,7 @@ __device__ __forceinline__ void nodeQuery(const Params& P, bool live) {
                 atomicAdd(&hits.sets[i / (32 * HIT_WORDS * HIT_GROUPS)], uint32_t(__popc(ballot)));
             }
         }
-        appendWarp(lapsed, i, r.survKeep, &r.work[W_LAPSED]);
+        appendWarp(lapsed, i, r.walkList, c.survivorCapacity, &r.work[W_LAPSED]);
     }
 }
 // A new list's slots, certified from their grid cells' triangle lists (in the
@@ -1084,7 +1088,7 @@ __device__ __forceinline__ void nodeCertify(const Params& P, bool live) {
         uint32_t i = 0;
         bool slow = false;
         if (k < n) {
-            i = r.survKeep[k];
+            i = r.walkList[k];
             slow = !single || laneId() == 0;
             if (c.cellListsEnabled) {
                 const uint32_t t = r.walkActive[i];
@@ -1103,7 +1107,7 @@ __device__ __forceinline__ void nodeCertify(const Params& P, bool live) {
             }
         }
         __syncwarp();
-        appendWarp(slow, i, r.walkKey, &r.work[W_SLOW]);
+        appendWarp(slow, i, r.walkKey, c.survivorCapacity, &r.work[W_SLOW]);
     }
 }
 // Records a slot's query: its certificate from the triangles at the nearest

@@ -128,7 +128,8 @@ struct Res {
     uint2* survivors;                 // survivorCapacity: (item, node slot) of each surviving node
     uint32_t* survKeep;               // survivorCapacity+1: 1 = the learned culler keeps the survivor
     uint32_t* keepOffset;             // survivorCapacity+1: exclusive scan of survKeep
-    uint32_t* walkList;               // survivorCapacity: survivors left for the exact query (lists built every step)
+    uint32_t* walkList;               // survivorCapacity: survivors left for the exact query (lists built every
+                                      // step), the step's lapsed slots (stored lists)
     float4* dpairSourcePlane;         // 4*pairCapacity: the enclosure plane in the source frame, and its bound terms
     const float4* meshChildren;       // 4 per BVH node: both children's bounds (internal) or the triangle range
     float* distanceGrid;              // shapes x GRID^3: certified lower bound of the signed distance per cell

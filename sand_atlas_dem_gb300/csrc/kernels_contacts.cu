@@ -6,9 +6,15 @@
 namespace sdg {
 
 // ---------------------------------------------------------------- kernels
-__global__ void k_scanReduce(const uint32_t* in, ScanCount count, const uint32_t* gate, uint32_t* partials) {
+// A scan is skipped where *gate is zero, and where *failed (the solver flags) is
+// not: on a failed step the phases before it return and leave stale input.
+__device__ __forceinline__ bool scanSkipped(const uint32_t* gate, const uint32_t* failed) {
+    return (gate && *gate == 0) || (failed && *failed != 0);
+}
+__global__ void k_scanReduce(const uint32_t* in, ScanCount count, const uint32_t* gate, const uint32_t* failed,
+                             uint32_t* partials) {
     __shared__ uint32_t shared[32];
-    if (gate && *gate == 0) return;
+    if (scanSkipped(gate, failed)) return;
     uint32_t n = scanCount(count);
     uint32_t chunk = (n + gridDim.x - 1) / gridDim.x;
     uint32_t begin = blockIdx.x * chunk, end = min(n, begin + chunk);
@@ -18,9 +24,9 @@ __global__ void k_scanReduce(const uint32_t* in, ScanCount count, const uint32_t
     if (threadIdx.x == blockDim.x - 1) partials[blockIdx.x] = sum;
 }
 __global__ void k_scanTop(ScanCount count, uint32_t* out, bool writeEnd, uint32_t* totalDst, const uint32_t* gate,
-                          uint32_t* partials, uint32_t blocks) {
+                          const uint32_t* failed, uint32_t* partials, uint32_t blocks) {
     __shared__ uint32_t shared[32];
-    if (gate && *gate == 0) return;
+    if (scanSkipped(gate, failed)) return;
     // blocks <= 1024: one element per thread.
     uint32_t v = threadIdx.x < blocks ? partials[threadIdx.x] : 0;
     uint32_t inc = blockInclusive(v, shared);
@@ -31,11 +37,13 @@ __global__ void k_scanTop(ScanCount count, uint32_t* out, bool writeEnd, uint32_
         if (totalDst) *totalDst = inc;
     }
 }
+// With `list`, the input holds flags (0 or 1): a set flag's index goes to its
+// place, and a place at or past `room` is dropped whatever the input holds.
 __global__ void k_scanApply(const uint32_t* in, uint32_t* out, ScanCount count, const uint32_t* gate,
-                            const uint32_t* partials, uint32_t* list) {
+                            const uint32_t* failed, const uint32_t* partials, uint32_t* list, uint32_t room) {
     __shared__ uint32_t shared[32];
     __shared__ uint32_t tileTotal;
-    if (gate && *gate == 0) return;
+    if (scanSkipped(gate, failed)) return;
     uint32_t n = scanCount(count);
     uint32_t chunk = (n + gridDim.x - 1) / gridDim.x;
     uint32_t begin = blockIdx.x * chunk, end = min(n, begin + chunk);
@@ -46,7 +54,7 @@ __global__ void k_scanApply(const uint32_t* in, uint32_t* out, ScanCount count, 
         uint32_t inc = blockInclusive(v, shared);
         if (i < end) {
             out[i] = carry + inc - v;
-            if (list && v) list[carry + inc - v] = i;
+            if (list && v && carry + inc - v < room) list[carry + inc - v] = i;
         }
         if (threadIdx.x == blockDim.x - 1) tileTotal = inc;
         __syncthreads();
@@ -580,19 +588,27 @@ __global__ void __launch_bounds__(128) k_gatherTail(const __grid_constant__ Para
 
 void launch_scan(const uint32_t* in, uint32_t* out, ScanCount count, bool writeEnd, uint32_t* totalDst,
                  const uint32_t* gate, uint32_t* partials, cudaStream_t s) {
-    k_scanReduce<<<SCAN_BLOCKS, 256, 0, s>>>(in, count, gate, partials);
-    k_scanTop<<<1, 1024, 0, s>>>(count, out, writeEnd, totalDst, gate, partials, SCAN_BLOCKS);
-    k_scanApply<<<SCAN_BLOCKS, 256, 0, s>>>(in, out, count, gate, partials, nullptr);
+    k_scanReduce<<<SCAN_BLOCKS, 256, 0, s>>>(in, count, gate, nullptr, partials);
+    k_scanTop<<<1, 1024, 0, s>>>(count, out, writeEnd, totalDst, gate, nullptr, partials, SCAN_BLOCKS);
+    k_scanApply<<<SCAN_BLOCKS, 256, 0, s>>>(in, out, count, gate, nullptr, partials, nullptr, 0);
 }
 
-// The step's scans (r.scanPartials); with `list`, the apply pass also lists
-// each index whose value is nonzero at its scanned offset (stream compaction
-// in index order).
+// The step's scans (r.scanPartials).
 void launch_step_scan(const Res& r, const uint32_t* in, uint32_t* out, ScanCount count, bool writeEnd,
-                      uint32_t* totalDst, const uint32_t* gate, cudaStream_t s, uint32_t* list = nullptr) {
-    k_scanReduce<<<SCAN_BLOCKS, 256, 0, s>>>(in, count, gate, r.scanPartials);
-    k_scanTop<<<1, 1024, 0, s>>>(count, out, writeEnd, totalDst, gate, r.scanPartials, SCAN_BLOCKS);
-    k_scanApply<<<SCAN_BLOCKS, 256, 0, s>>>(in, out, count, gate, r.scanPartials, list);
+                      uint32_t* totalDst, const uint32_t* gate, cudaStream_t s) {
+    launch_scan(in, out, count, writeEnd, totalDst, gate, r.scanPartials, s);
+}
+// The scan of the keep flags (survKeep, to keepOffset and *totalDst), skipped on
+// a failed step; with `list`, the apply pass also lists each index whose flag is
+// set at its scanned offset (stream compaction in index order).
+void launch_keep_scan(const Params& P, const uint32_t* count, uint32_t* totalDst, const uint32_t* gate,
+                      uint32_t* list, cudaStream_t s) {
+    const Res& r = P.r;
+    const ScanCount n{count, P.c.survivorCapacity, 1, 0};
+    k_scanReduce<<<SCAN_BLOCKS, 256, 0, s>>>(r.survKeep, n, gate, r.control, r.scanPartials);
+    k_scanTop<<<1, 1024, 0, s>>>(n, r.keepOffset, true, totalDst, gate, r.control, r.scanPartials, SCAN_BLOCKS);
+    k_scanApply<<<SCAN_BLOCKS, 256, 0, s>>>(r.survKeep, r.keepOffset, n, gate, r.control, r.scanPartials, list,
+                                            P.c.survivorCapacity);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -704,13 +720,11 @@ static void collectFilter(const Params& P, cudaStream_t s) {
         k_cullSurvivors<<<grid(0, 4), CULLER_ROWS, 0, s>>>(P);  // 4 x 64 TMEM columns per SM
     }
     const bool stored = storedKeep(c);
-    launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_SURVIVORS, c.survivorCapacity, 1, 0}, true,
-                     r.work + W_KEPT, stored ? r.work + W_FILTER : nullptr, s);
+    launch_keep_scan(P, r.work + W_SURVIVORS, r.work + W_KEPT, stored ? r.work + W_FILTER : nullptr, nullptr, s);
     k_walkList<<<grid(c.contactBlocksPerSM, 8), 256, 0, s>>>(P);
     if (stored) {
         k_certifyBuild<<<grid(c.walkBlocksPerSM, 8), 256, 0, s>>>(P);
-        launch_step_scan(r, r.survKeep, r.keepOffset, ScanCount{r.work + W_KEPT, c.survivorCapacity, 1, 0}, true,
-                         r.work + W_ACTIVE, r.work + W_FILTER, s, r.walkActive);
+        launch_keep_scan(P, r.work + W_KEPT, r.work + W_ACTIVE, r.work + W_FILTER, r.walkActive, s);
     }
 }
 // The exact queries.

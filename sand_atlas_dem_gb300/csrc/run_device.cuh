@@ -53,11 +53,13 @@ struct GridBarrier {
     }
 };
 // Exclusive scan over the grid: in[0..n) to out, the total to out[n] and
-// *total (where given), with `list` each index of a nonzero value at its
-// offset.  One barrier inside; the caller's follows.
+// *total (where given).  With `list` the input holds flags (0 or 1), and a set
+// flag's index goes to its place: not on a failed step, whose phases return and
+// leave stale flags, and never at or past `room`.  One barrier inside, which
+// every CTA takes (`live` may differ among them); the caller's follows.
 static __device__ __noinline__ bool runScan(GridBarrier& barrier, bool& live, const Res& r, const uint32_t* in,
                                         uint32_t* out, uint32_t n, bool writeEnd, uint32_t* total,
-                                        uint32_t* list = nullptr) {
+                                        uint32_t* list = nullptr, uint32_t room = 0) {
     __shared__ uint32_t shared[32], tileTotal;
     const uint32_t chunk = (n + gridDim.x - 1) / gridDim.x;
     const uint32_t begin = min(n, blockIdx.x * chunk), end = min(n, begin + chunk);
@@ -85,7 +87,7 @@ static __device__ __noinline__ bool runScan(GridBarrier& barrier, bool& live, co
         uint32_t inc = blockInclusive(v, shared);
         if (i < end) {
             out[i] = carry + inc - v;
-            if (list && v) list[carry + inc - v] = i;
+            if (list && v && live && carry + inc - v < room) list[carry + inc - v] = i;
         }
         if (threadIdx.x == blockDim.x - 1) tileTotal = inc;
         __syncthreads();
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(Threads, 1) k_run(const __grid_constant__ RunA
             rare::certifyBuild(P, live);
             RUN_SYNC();
             if (!runScan(barrier, live, r, r.survKeep, r.keepOffset, min(r.work[W_KEPT], c.survivorCapacity), true,
-                         r.work + W_ACTIVE, r.walkActive))
+                         r.work + W_ACTIVE, r.walkActive, c.survivorCapacity))
                 return;
             RUN_SYNC();
         }
