@@ -67,8 +67,10 @@
  * SM, node-filter warps per CTA (4 or 8), pair set-up/leaf-cull CTAs per SM,
  * contact emit/law CTAs per SM, gather warps per SM and exact-query CTAs per
  * SM (launch shapes never change results), the survivor capacity (nodes
- * left for the exact query per step; overflow raises the contact-capacity
- * flag), whether nodes the distance-bound grid certifies outside their
+ * left for the exact query per step; it also bounds the grain contacts of
+ * the SDF geometry, which wait in the survivors' scratch rows, and, doubled,
+ * the plane contacts of a step: at least contactCapacity serves both; overflow
+ * raises the contact-capacity flag), whether nodes the distance-bound grid certifies outside their
  * target skip the exact query, and the filter margin: the reach, in the
  * target shape's unscaled frame, by which the leaf cull and node filter grow
  * their tests when they store their results; the results are reused while
@@ -90,11 +92,19 @@
 extern "C" {
 #endif
 
+/*
+ * Revision 2: four extension buffers more (140 for 136 pointers; a caller built
+ * for revision 1 passes a shorter block), three others hold different records
+ * (walkCert, walkState and walkContact for walkCertPoint, walkCertTriangle and
+ * walkItem), survivorCapacity bounds SDF and plane contacts too, and
+ * sdg_engine_diagnostics copies 96 bytes more per plane.
+ */
+#define SDG_ABI_VERSION 2
 #define SDG_BUFFER_COUNT 140
 #define SDG_VALUE_COUNT 39
 #define SDG_PHASES 9
 
-/* ABI revision of this header. */
+/* SDG_ABI_VERSION as compiled into the library; compare it before any other call. */
 int sdg_abi_version(void);
 /* SDG_BUFFER_COUNT and SDG_VALUE_COUNT as compiled into the library. */
 int sdg_buffer_count(void);

@@ -395,7 +395,10 @@ using namespace sdg;
 
 extern "C" {
 
-int sdg_abi_version(void) { return 1; }
+// SDG_ABI_VERSION of the header: one more whenever a caller built for it would
+// pass something else.
+static constexpr int ABI_VERSION = 2;
+int sdg_abi_version(void) { return ABI_VERSION; }
 int sdg_buffer_count(void) { return BUFFER_COUNT; }
 int sdg_value_count(void) { return VALUE_COUNT; }
 const char* sdg_last_error(void) { return g_error.c_str(); }

@@ -16,6 +16,7 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBDIR = PACKAGE / "_lib"
 LIBRARY = LIBDIR / "libsanddem_gb300.so"
+ABI_VERSION = 2  # of the header this module's callers are written for
 SOURCES = ("run_mesh_wide.cu", "run_walls_wide.cu", "run_mesh.cu", "run_walls.cu", "run_sdf.cu", "kernels_state.cu",
            "kernels_contacts.cu", "capi.cu", "culler.cu", "scan_static.cu", "trees.cu")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -72,6 +73,8 @@ def load():
     lib = ct.CDLL(str(LIBRARY))
     P = ct.POINTER
     lib.sdg_abi_version.restype = ct.c_int
+    if lib.sdg_abi_version() != ABI_VERSION:
+        raise RuntimeError(f"GB300 CUDA library ABI {lib.sdg_abi_version()}, not {ABI_VERSION}: build() it again")
     lib.sdg_buffer_count.restype = ct.c_int
     lib.sdg_value_count.restype = ct.c_int
     lib.sdg_last_error.restype = ct.c_char_p

@@ -48,6 +48,14 @@ def test_buffer_and_value_counts(library):
     assert len(RESOURCE_ORDER) == 77
 
 
+def test_abi_revision(library):
+    """The revision is the header's, and a new one for a new buffer block."""
+    revision = int(re.search(r"#define SDG_ABI_VERSION (\d+)", HEADER.read_text())[1])
+    library.sdg_abi_version.restype = ct.c_int
+    assert library.sdg_abi_version() == revision == native.ABI_VERSION
+    assert len(BUFFER_ORDER) == 140 and revision == 2
+
+
 def test_argument_errors_are_reported_without_a_device(library):
     lib = native.load()
     rc = lib.sdg_dispatch(b"beginStep", 1, None, None, None, 0, None)
