@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include "dem_device.cuh"
 #include "launch.h"
+#include "step_form.h"
 
 namespace sdg {
 
@@ -254,6 +255,7 @@ struct Engine {
     cudaStream_t aux = nullptr;  // captures the conditional bodies
     Params last = {};            // of the last advance
     bool persistent = false;     // the last advance ran persistent launches
+    bool refused = false;        // the runtime refused one: this engine replays graphs
     // Active slots as last reported by the device (pinned), which picks the
     // step's form; UINT32_MAX before the first report.
     uint32_t *active = nullptr, *activeDevice = nullptr;
@@ -276,9 +278,6 @@ struct Engine {
 // a grain are assumed.  Up to 6,000 grains its phases are latency-bound and
 // take the 512-thread form.
 constexpr uint32_t RUN_ACTIVE_SLOTS = 300'000, RUN_SLOTS_PER_GRAIN = 18, RUN_NARROW_GRAINS = 6'000;
-// Steps of one launch (even: each starts on the same history side): a few
-// milliseconds at a time, so that a long chunk shares the GPU.
-constexpr uint32_t RUN_STEPS = 64;
 // With the SDF geometry up to 2,048 grains (73 us against 79 launched at
 // 1,000; 107 against 100 at 2,197).
 constexpr uint32_t RUN_SDF_GRAINS = 2'048;
@@ -590,15 +589,19 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
         return record(cudaGetLastError(), "advance");
     }
     e->last = P;
-    e->persistent = P.c.meshGeometry == 0 ? P.c.N <= RUN_SDF_GRAINS && cooperative()
-                                          : storedFilters(P.c) && runsPersistent(*e, P.c);
+    e->persistent = !e->refused && (P.c.meshGeometry == 0 ? P.c.N <= RUN_SDF_GRAINS && cooperative()
+                                                          : storedFilters(P.c) && runsPersistent(*e, P.c));
+    uint32_t done = 0;
     if (e->persistent) {
-        for (uint32_t k = 0; k < steps; k += RUN_STEPS)
-            if (int rc = record(cudaError_t(launch_run(side[0], side[1], std::min(RUN_STEPS, steps - k),
-                                                       P.c.N > RUN_NARROW_GRAINS, e->activeDevice, s)),
-                                "persistent steps"))
-                return rc;
-        return 0;
+        done = runSteps(steps, [&](uint32_t n) {
+            return launch_run(side[0], side[1], n, P.c.N > RUN_NARROW_GRAINS, e->activeDevice, s) == 0;
+        });
+        if (done == steps) return 0;
+        // Refused at launch (a context with fewer SMs than the device, say): the
+        // captured steps ask for no co-residency.
+        cudaGetLastError();
+        e->refused = true;
+        e->persistent = false;
     }
     // Orientation-independent key: the side whose buffers sort first is 0.
     bool flipped = std::memcmp(&side[0], &side[1], sizeof(Params)) > 0;
@@ -618,7 +621,7 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
         e->key = key;
     }
     uint32_t start = flipped ? 1u : 0u;
-    for (uint32_t k = 0; k < steps; ++k)
+    for (uint32_t k = done; k < steps; ++k)
         if (int rc = record(cudaGraphLaunch(e->exec[(start + k) & 1], s), "graph launch")) return rc;
     if (storedFilters(P.c) && e->active && steps)
         return record(cudaMemcpyAsync(e->active, P.r.work + W_ACTIVE, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "active");
