@@ -275,7 +275,8 @@ __global__ void k_triangleLeaf(const __grid_constant__ Params P) {
 // 5,120, now 4.5 and 11.7.  Cells that no exact query reaches hold an empty list: a stored
 // node lies within 1.001 margins (16 at most) of its target at the build, by its
 // cell's bound, and moves by less than as much again, which with the cells'
-// extent is what the line below allows.  (A query there would walk.)
+// extent is what the line below allows.  (A query there would walk: with the
+// distance grid off no bound holds the stored nodes near, and every cell is listed.)
 __global__ void __launch_bounds__(256) k_cellLists(const __grid_constant__ Params P) {
     const Res& r = P.r;
     const Config& c = P.c;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(256) k_cellLists(const __grid_constant__ Param
         uint32_t* out = r.cellLists + size_t(i) * CELL_WORDS;
         const uint32_t seed = r.distanceGridTriangle[i];
         const float reached = __fadd_rn(__fmul_rn(33.0f, c.filterMargin), __fmul_rn(2.0f, info.w));
-        const bool listed = seed != EMPTY && r.distanceGrid[i] <= reached;
+        const bool listed = seed != EMPTY && (!c.distanceGridEnabled || r.distanceGrid[i] <= reached);
         auto squared = [&](uint32_t t) {
             uint32_t feature;
             f3 q = closestTriangle(p, xyz(__ldg(&r.meshTriangles[3 * t])), xyz(__ldg(&r.meshTriangles[3 * t + 1])),

@@ -84,3 +84,25 @@ def test_contact_counts_and_starts_follow_the_contacts(gpu_library):
     owner = np.repeat(np.arange(pairs), np.diff(starts))
     np.testing.assert_array_equal(np.sort(meta[:, :2], axis=1), ij[owner])
     assert (counts == 0).sum() > pairs // 4
+
+
+def test_lists_without_the_distance_grid(gpu_library):
+    """Without the grid's bound a stored node may lie in any cell: every cell
+    has its list, and a new slot is certified from it instead of by a scan."""
+    library = grains("rough")
+    case = contact_lattice(library, 4, spacing=0.985, seed=3, speed=0.05)
+    spec = Experiment(particles=64, contact_geometry="mesh", timestep=2e-9, max_overlap_fraction=0.9,
+                      contacts_per_particle=256, pairs_per_particle=32)
+    engines = [build(Engine, library, spec, case, distance_grid=flag) for flag in (True, False)]
+    first = [e.read("cellLists", np.uint32).reshape(-1, 64)[:, 2] for e in engines]
+    assert (first[0] == 0xFFFFFFFF).any() and not (first[1] == 0xFFFFFFFF).any()
+    for e in engines:
+        e.initialize()
+        kept, slow, lapsed = (int(e.read("work", np.uint32, (64,))[k]) for k in (3, 14, 20))
+        assert kept > 0 and lapsed == slow == 0
+        e.advance(5)
+    a, b = (e.state() for e in engines)
+    assert a["contacts"] == b["contacts"] > 0
+    for key, value in a.items():
+        if isinstance(value, np.ndarray):
+            assert value.tobytes() == b[key].tobytes(), key
