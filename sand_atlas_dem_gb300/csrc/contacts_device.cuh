@@ -533,7 +533,8 @@ __device__ __forceinline__ void resetContacts(const Res& r, const Config& c, boo
     const uint32_t runs = r.work[W_FILTER_STEPS], age = r.work[W_FILTER_AGE] + 1u, current = r.control[1];
     const float margin = __uint_as_float(r.work[W_FILTER_MARGIN]);
     bool on = c.filterMargin > 0.0f;
-    bool valid = complete != 0 && configured == __float_as_uint(c.filterMargin);
+    // Steps with the learned culler keep the survivors but no slots (1, not 2).
+    bool valid = complete >= (storedKeep(c) ? 2u : 1u) && configured == __float_as_uint(c.filterMargin);
     bool build = !on || !valid || (pairsKnown && pairs != current);
     r.control[2] = 0;
     r.control[6] = 0;
@@ -637,10 +638,10 @@ __device__ __forceinline__ void leafCull(const Params& P, bool live) {
     uint32_t n = 2 * activePairs(r, c);
     float margin = buildMargin(r, c);
     float grow = __fmul_rn(1.001f, margin);
+    if (gtid() == 0) r.work[W_FILTER_VALID] = 0;  // (also where this build stores nothing: it overwrites the lists)
     if (margin > 0.0f) {
         for (uint32_t g = gtid(); g < c.N; g += gstride()) r.filterRefRotation[g] = r.rotation[g];
         if (gtid() == 0) {
-            r.work[W_FILTER_VALID] = 0;
             r.work[W_FILTER_PAIRS] = r.control[1];
             r.work[W_FILTER_MARGIN] = __float_as_uint(margin);
             r.work[W_FILTER_BASE] = __float_as_uint(c.filterMargin);
@@ -910,8 +911,10 @@ __device__ __forceinline__ void survivorList(const Params& P) {
     const Config& c = P.c;
     if (r.control[0] != 0 || r.work[W_FILTER] == 0) return;
     uint32_t n = min(r.work[W_CANDIDATES], c.candidateCapacity);
-    if (gtid() == 0 && c.filterMargin > 0.0f)
-        r.work[W_FILTER_VALID] = r.work[W_CANDIDATES] <= c.candidateCapacity && r.work[W_SURVIVORS] <= c.survivorCapacity;
+    if (gtid() == 0 && c.filterMargin > 0.0f) {
+        const bool complete = r.work[W_CANDIDATES] <= c.candidateCapacity && r.work[W_SURVIVORS] <= c.survivorCapacity;
+        r.work[W_FILTER_VALID] = complete ? (storedKeep(c) ? 2u : 1u) : 0u;
+    }
     for (uint32_t item = warpGlobal(); item < n; item += warpStride()) {
         uint2 m = r.candSurvMask[item];
         if ((m.x | m.y) == 0) continue;

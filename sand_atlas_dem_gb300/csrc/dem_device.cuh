@@ -170,7 +170,7 @@ constexpr int W_CANDIDATES = 0;
 constexpr int W_SURVIVORS = 2;
 constexpr int W_KEPT = 3;
 constexpr int W_FILTER = 5;         // 1 = build the filter results this step, 0 = reuse them
-constexpr int W_FILTER_VALID = 6;   // 1 = the stored filter results are complete
+constexpr int W_FILTER_VALID = 6;   // the stored filter results: 0 incomplete, 1 up to the survivors, 2 with the slots
 constexpr int W_FILTER_PAIRS = 7;   // pair count they were built on
 constexpr int W_FILTER_MARGIN = 8;  // margin they were built with (float bits)
 constexpr int W_FILTER_BUILDS = 9;  // steps that built them (counter)

@@ -111,3 +111,27 @@ def test_culled_step_has_zero_missed_contacts(gpu_library, side):
     assert work_culled[3] < work_culled[2]          # of which fewer go to the exact query
     print(dict(side=side, survivors=int(work_culled[2]), exact_queries=int(work_culled[3]),
                culled_share=1 - int(work_culled[3]) / int(work_culled[2])))
+
+
+@pytest.mark.parametrize("speed", [0.05, 50.0])  # one list build in all, one every few steps
+def test_steps_after_a_detached_culler_build_their_own_list(gpu_library, speed):
+    """A step with the culler keeps the survivors but no exact-query slots: the
+    first step after it is detached must not take an earlier list's, or none."""
+    library, spec, case = lattice_case(side=4, viscosity=4e5, speed=speed)
+    plain = build(Engine, library, spec, case, filter_margin=0.0)
+    culled = build(Engine, library, spec, case)
+    c = small_culler(culled)
+    c.train()
+    c.attach(culled)
+    for e in (plain, culled):
+        e.initialize()
+    for attached in (True, False, True, False):
+        (c.attach if attached else c.detach)(culled)
+        for steps in (1, 12):
+            for e in (plain, culled):
+                e.advance(steps, rate=(-0.5, -0.5, -0.5))
+            sp, sc = plain.state(), culled.state()
+            assert sp["contacts"] == sc["contacts"] > 0
+            for key, value in sp.items():
+                if isinstance(value, np.ndarray):
+                    assert value.tobytes() == sc[key].tobytes(), (attached, steps, key)

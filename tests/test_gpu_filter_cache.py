@@ -127,3 +127,13 @@ def test_margin_is_validated(gpu_library):
     library, spec, case = lattice_case()
     with pytest.raises(ValueError, match="filter margin"):
         build(Engine, library, spec, case, filter_margin=-1.0)
+
+
+def test_a_margin_set_aside_and_taken_up_again(gpu_library):
+    """Steps without a margin overwrite the lists that were stored with one."""
+    plain, stored = engines(1e-3, speed=50.0)
+    for margin, steps in ((1e-3, 2), (0.0, 30), (1e-3, 1), (1e-3, 9), (2e-3, 3), (1e-3, 3)):
+        stored.filter_margin = margin
+        for e in (plain, stored):
+            e.advance(steps, rate=RATE)
+        assert_same(plain, stored)
