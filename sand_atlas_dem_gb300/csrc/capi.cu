@@ -63,6 +63,7 @@ static int unpack(void* const* buffers, const uint64_t* bytes, const double* val
             c.library16[k] = bytes ? uint32_t(std::min<uint64_t>(bytes[library[k]] / 16, 0xFFFFFFFFu)) : 0u;
     }
     // The triangle lists are optional: used where the buffer holds them.
+    c.triangleLeafEnabled = bytes && bytes[77 + 60] >= bytes[31] / 48 * 4;
     c.cellListsEnabled = bytes && bytes[77 + 59] >= uint64_t(c.shapes) * GRID * GRID * GRID * CELL_WORDS * 4;
     if (!(c.filterMargin >= 0.0f) || c.filterMargin > 1.0f) {
         g_error = "filter margin must lie in [0, 1] (target shape frame)";
@@ -115,7 +116,7 @@ static int unpack(void* const* buffers, const uint64_t* bytes, const double* val
             (c.meshGeometry == 0 && bytes[77 + 50] < uint64_t(c.pairCapacity) * 32 * 4) ||
             bytes[77 + 51] < uint64_t(c.survivorCapacity) * 16 * CERT_ROWS ||
             bytes[77 + 52] < uint64_t(c.survivorCapacity) * 4 ||
-            (c.meshGeometry != 0 && storedKeep(c) && bytes[77 + 60] < bytes[31] / 48 * 4) ||
+            (c.meshGeometry != 0 && storedKeep(c) && !c.triangleLeafEnabled) ||
             bytes[77 + 61] < uint64_t(c.survivorCapacity) * 4 ||
             bytes[77 + 62] < slotHitSize(c.survivorCapacity) * 4 ||
             bytes[77 + 57] < uint64_t(c.survivorCapacity) * 16 || bytes[77 + 58] < uint64_t(c.survivorCapacity) * 4 ||

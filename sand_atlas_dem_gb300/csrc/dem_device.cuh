@@ -63,6 +63,7 @@ struct Config {
     // Whether the caller's buffers hold the per-cell triangle lists (cellLists
     // and triangleLeaf at full size).
     uint32_t cellListsEnabled;
+    uint32_t triangleLeafEnabled;  // ... hold triangleLeaf at full size
 };
 
 // Buffers: the reference Resources block (solver.slang:20-100) in declaration

@@ -835,7 +835,7 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
     else if (name == "distanceGrid") {
         if (c.meshGeometry != 0) {
             k_distanceGrid<<<grid(0, 8), T, 0, s>>>(P);
-            if (storedKeep(c)) k_triangleLeaf<<<min(c.shapes, grid(0, 8)), T, 0, s>>>(P);
+            if (c.triangleLeafEnabled) k_triangleLeaf<<<min(c.shapes, grid(0, 8)), T, 0, s>>>(P);
             if (c.cellListsEnabled) k_cellLists<<<grid(0, 8), T, 0, s>>>(P);
         }
     }

@@ -305,11 +305,12 @@ class Engine:
             "wallCounts": 4 * walls, "wallOffsets": 4 * (walls + 1),
         }
         # The triangle lists serve the stored exact-query list (not the SDF
-        # geometry, nor an engine that filters every step).
+        # geometry, nor an engine built to filter every step; without them
+        # lapsed slots are scanned, with the BVH leaf of each triangle).
         lists = CELL_LIST_BYTES * len(library.shapes) * DISTANCE_GRID**3
         listed = self.filter_margin > 0 and lists <= CELL_LIST_LIMIT
         sizes["cellLists"] = lists if listed else 16
-        sizes["triangleLeaf"] = self.buffers["meshTriangles"].size // 12 if self.filter_margin > 0 else 16
+        sizes["triangleLeaf"] = 16 if self.sdf else self.buffers["meshTriangles"].size // 12
         for name, nbytes in sizes.items():
             self.buffers[name] = DeviceBuffer(self, nbytes)
         side_sizes = {

@@ -137,3 +137,13 @@ def test_a_margin_set_aside_and_taken_up_again(gpu_library):
         for e in (plain, stored):
             e.advance(steps, rate=RATE)
         assert_same(plain, stored)
+
+
+def test_a_margin_set_on_an_engine_built_without_one(gpu_library):
+    plain, other = engines(0.0, speed=50.0)
+    other.filter_margin = 1e-3
+    for steps in (1, 20):
+        for e in (plain, other):
+            e.advance(steps, rate=RATE)
+        assert_same(plain, other)
+    assert 0 < counters(other)[0] < 21
