@@ -298,10 +298,15 @@ __device__ __forceinline__ void findPairsWarp(const Res& r, const Config& c, uin
 #pragma unroll
                             for (int a = 0; a < 3; ++a) e[a] -= floorf(e[a] * perBox[a] + 0.5f) * box[a];
                         }
-                        // An estimate, good to ~1e-6: only the pairs near the range need the FP64 branch.
+                        // An estimate: only the pairs near the range need the FP64 branch.  A
+                        // component is off by a few roundings of a box length (the raw
+                        // separation across the boundary, its remainder: below 2.5e-7 of it),
+                        // which counts in boxes of thousands of ranges.
                         const float ee = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
-                        near = ee <= 1.002f * rr;
-                        inside = ee <= 0.998f * rr;
+                        const float unsure = 0.002f * rr + 1e-6f * (box[0] + box[1] + box[2]) *
+                                                               (range + 5e-7f * (box[0] + box[1] + box[2]));
+                        near = ee <= rr + unsure;
+                        inside = ee <= rr - unsure;
                     }
                     if (inside) {
                         pass = true;
