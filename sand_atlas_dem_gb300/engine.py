@@ -181,6 +181,94 @@ class GB300Device:
         )
 
 
+def capacities(h):
+    """Leaf mask words of a directed pair, (directed pair, leaf) items and survivors
+    of a layout."""
+    # Survivors: nodes left for the exact query after the conservative filters,
+    # per step; overflow raises the contact-capacity flag and grows with it.
+    return (h.max_leaves + 31) // 32, max(1, 2 * h.pair_capacity * h.max_leaves), 4 * h.contact_capacity
+
+
+def scratch_sizes(h, filter_margin):
+    """Bytes of each buffer of a layout that holds no host array (16 at least each)."""
+    n, pc, cc = h.n, h.pair_capacity, h.contact_capacity
+    leaf_words, candidates, survivors = capacities(h)
+    shapes, walls, sdf = len(h.library.shapes), h.wall_count * n, h.spec.contact_geometry == "sdf"
+    sizes = {
+        "meshPairMask": 4 * pc, "meshPairTransform": 16 * 8 * pc, "fabricRows": 16 * 2 * pc,
+        "binCounts": 4 * h.bin_count, "binParticles": 4 * h.bin_count * h.bin_capacity,
+        "pairCounts": 4 * n, "pairOffsets": 4 * n, "pairs": 8 * pc, "contactCounts": 4 * pc,
+        "contactOffsets": 4 * pc, "pointDepth": 16 * cc, "contactForce": 16 * cc,
+        "normalLossPower": 4 * cc, "heads": 4 * n, "next": 16,
+        "byJCounts": 4 * (n + 1), "byJOffsets": 4 * (n + 1), "byJCursor": 4 * n, "byJPairs": 4 * pc,
+        "dpairBranch": 16 * 2 * pc, "dpairLeafCount": 4 * (2 * pc + 1),
+        "dpairCandOffset": 4 * (2 * pc + 1), "leafMask": 4 * 2 * pc * leaf_words,
+        "candidates": 8 * candidates, "candHitCount": 4 * (candidates + 1),
+        "candHitOffset": 4 * (candidates + 1), "candHitMask": 8 * candidates,
+        "contactPair": 4 * cc, "work": 4 * 64, "scanPartials": 4 * 2 * SCAN_BLOCKS,
+        "hitScratch": 32 * survivors, "candSurvCount": 4 * (candidates + 1),
+        "dpairPlane": 16 * 2 * pc, "candSurvMask": 8 * candidates,
+        "candSurvOffset": 4 * (candidates + 1), "survivors": 8 * survivors,
+        "survKeep": 4 * (survivors + 1), "keepOffset": 4 * (survivors + 1),
+        "walkList": 4 * survivors, "dpairSourcePlane": 16 * 4 * pc,
+        "distanceGrid": 4 * shapes * DISTANCE_GRID**3, "distanceGridInfo": 16 * shapes,
+        "distanceGridTriangle": 4 * shapes * DISTANCE_GRID**3,
+        "cullerParams": 4 * CULLER_PARAMS * shapes, "cullerW1": 2 * 4096 * shapes,
+        "cullerMargin": 4 * CULLER_MARGINS * shapes, "cullerStats": 16,
+        "filterRefRotation": 16 * n, "filterRefBranch": 16 * pc, "filterRefPairs": 8 * pc,
+        "walkKey": 4 * survivors, "walkBucketCount": 4 * (shapes * WALK_BUCKETS + 1),
+        "walkBucketOffset": 4 * (shapes * WALK_BUCKETS + 1),
+        "sdfLaneCounts": 4 * 32 * pc if sdf else 16,
+        "walkCert": 48 * survivors, "walkState": 4 * survivors,
+        "walkActive": 4 * survivors,
+        # Counts per 4,096 slots and per 262,144, and a bit per slot (csrc slotHitSize).
+        "walkHits": 4 * (129 * (survivors // 4096 + 1) + survivors // 262144 + 1),
+        "walkNode": 16 * survivors, "walkContact": 4 * survivors,
+        "wallCounts": 4 * walls, "wallOffsets": 4 * (walls + 1),
+    }
+    # The triangle lists serve the stored exact-query list (not the SDF
+    # geometry, nor an engine built to filter every step; without them
+    # lapsed slots are scanned, with the BVH leaf of each triangle).
+    lists = CELL_LIST_BYTES * shapes * DISTANCE_GRID**3
+    listed = filter_margin > 0 and lists <= CELL_LIST_LIMIT
+    sizes["cellLists"] = lists if listed else 16
+    sizes["triangleLeaf"] = 16 if sdf else h.geometry["meshTriangles"].nbytes // 12
+    return sizes
+
+
+def side_sizes(h):
+    """Bytes of one contact-history side's buffers."""
+    n, pc, cc = h.n, h.pair_capacity, h.contact_capacity
+    return {
+        "meta": 16 * cc, "slip": 16 * cc, "normalArea": 16 * cc, "hash": 16,
+        "sidePairOffsets": 4 * (n + 1), "sidePairB": 4 * pc, "sideContactStart": 4 * (pc + 1),
+        "sideWallStart": 4 * (h.wall_count * n + 1),
+    }
+
+
+def backup_names(h):
+    """The buffers the rollback copy of a chunk holds, beside the committed side."""
+    return (
+        "position", "velocity", "rotation", "momentum", "cell", "force", "torque", "referencePosition",
+        "referenceCell", "control", "pairs", "pairCounts", "pairOffsets", "particleStress",
+        "particleDiagnostic", "timestepRows", "accumulated", "referencePositionRemainder",
+        *RESIDUAL_STATE, *DAMPING_STATE, "contactCounts", "byJOffsets", "byJPairs",
+        *(WALL_STATE if h.wall_count else ()),
+    )
+
+
+def working_set(h, filter_margin=FILTER_MARGIN):
+    """Device bytes of an engine of a layout: its buffers, both history sides and the
+    rollback copy."""
+    if h.spec.contact_geometry == "sdf":
+        filter_margin = 0.0
+    own = {name: array.nbytes for group in (h.geometry, h.initial_state(), h.walls) for name, array in group.items()}
+    own.update(scratch_sizes(h, filter_margin))
+    own = {name: max(16, int(nbytes)) for name, nbytes in own.items()}
+    side = sum(max(16, int(nbytes)) for nbytes in side_sizes(h).values())
+    return sum(own.values()) + 3 * side + sum(own[name] for name in backup_names(h))
+
+
 class Engine:
     """GPU-resident DEM engine: mesh or SDF contact geometry, periodic cells or
     one nonperiodic specimen bounded by penalty planes."""
@@ -250,89 +338,34 @@ class Engine:
                      "ids", "scales", "body", "skin", "cutoff", "bins", "bin_count", "pair_capacity",
                      "contact_capacity", "hash_size", "bin_capacity", "initial_cell"):
             setattr(self, name, getattr(h, name))
-        self.estimated_bytes = h.estimated_bytes()
         volumes = np.array([shape.volume for shape in library.shapes])
         self.solid_volume = float(np.sum(volumes[self.ids] * np.asarray(self.scales, float) ** 3))
-        self.leaf_words = (h.max_leaves + 31) // 32
-        self.candidate_capacity = max(1, 2 * h.pair_capacity * h.max_leaves)
-        # Nodes left for the exact query after the conservative filters, per
-        # step; overflow raises the contact-capacity flag and grows with it.
-        self.survivor_capacity = 4 * h.contact_capacity
+        self.leaf_words, self.candidate_capacity, self.survivor_capacity = capacities(h)
         self.device = torch.device(device or "cuda")
         self.stream = torch.cuda.Stream(self.device)
         self._staging = torch.empty(STAGING_BYTES, dtype=torch.uint8).pin_memory()
         self._staging_host = self._staging.numpy()
         self.m = GB300Device(self)
         self.buffers = {}
-        n, pc, cc = h.n, h.pair_capacity, h.contact_capacity
         for name, array in h.geometry.items():
             self._add(name, array)
         for name, array in h.initial_state().items():
             self._add(name, array)
         for name, array in h.walls.items():
             self._add(name, array)
-        walls = h.wall_count * n
-        sizes = {
-            "meshPairMask": 4 * pc, "meshPairTransform": 16 * 8 * pc, "fabricRows": 16 * 2 * pc,
-            "binCounts": 4 * h.bin_count, "binParticles": 4 * h.bin_count * h.bin_capacity,
-            "pairCounts": 4 * n, "pairOffsets": 4 * n, "pairs": 8 * pc, "contactCounts": 4 * pc,
-            "contactOffsets": 4 * pc, "pointDepth": 16 * cc, "contactForce": 16 * cc,
-            "normalLossPower": 4 * cc, "heads": 4 * n, "next": 16,
-            "byJCounts": 4 * (n + 1), "byJOffsets": 4 * (n + 1), "byJCursor": 4 * n, "byJPairs": 4 * pc,
-            "dpairBranch": 16 * 2 * pc, "dpairLeafCount": 4 * (2 * pc + 1),
-            "dpairCandOffset": 4 * (2 * pc + 1), "leafMask": 4 * 2 * pc * self.leaf_words,
-            "candidates": 8 * self.candidate_capacity, "candHitCount": 4 * (self.candidate_capacity + 1),
-            "candHitOffset": 4 * (self.candidate_capacity + 1), "candHitMask": 8 * self.candidate_capacity,
-            "contactPair": 4 * cc, "work": 4 * 64, "scanPartials": 4 * 2 * SCAN_BLOCKS,
-            "hitScratch": 32 * self.survivor_capacity, "candSurvCount": 4 * (self.candidate_capacity + 1),
-            "dpairPlane": 16 * 2 * pc, "candSurvMask": 8 * self.candidate_capacity,
-            "candSurvOffset": 4 * (self.candidate_capacity + 1), "survivors": 8 * self.survivor_capacity,
-            "survKeep": 4 * (self.survivor_capacity + 1), "keepOffset": 4 * (self.survivor_capacity + 1),
-            "walkList": 4 * self.survivor_capacity, "dpairSourcePlane": 16 * 4 * pc,
-            "distanceGrid": 4 * len(library.shapes) * DISTANCE_GRID**3, "distanceGridInfo": 16 * len(library.shapes),
-            "distanceGridTriangle": 4 * len(library.shapes) * DISTANCE_GRID**3,
-            "cullerParams": 4 * CULLER_PARAMS * len(library.shapes), "cullerW1": 2 * 4096 * len(library.shapes),
-            "cullerMargin": 4 * CULLER_MARGINS * len(library.shapes), "cullerStats": 16,
-            "filterRefRotation": 16 * n, "filterRefBranch": 16 * pc, "filterRefPairs": 8 * pc,
-            "walkKey": 4 * self.survivor_capacity, "walkBucketCount": 4 * (len(library.shapes) * WALK_BUCKETS + 1),
-            "walkBucketOffset": 4 * (len(library.shapes) * WALK_BUCKETS + 1),
-            "sdfLaneCounts": 4 * 32 * pc if spec.contact_geometry == "sdf" else 16,
-            "walkCert": 48 * self.survivor_capacity, "walkState": 4 * self.survivor_capacity,
-            "walkActive": 4 * self.survivor_capacity,
-            # Counts per 4,096 slots and per 262,144, and a bit per slot (csrc slotHitSize).
-            "walkHits": 4 * (129 * (self.survivor_capacity // 4096 + 1) + self.survivor_capacity // 262144 + 1),
-            "walkNode": 16 * self.survivor_capacity, "walkContact": 4 * self.survivor_capacity,
-            "wallCounts": 4 * walls, "wallOffsets": 4 * (walls + 1),
-        }
-        # The triangle lists serve the stored exact-query list (not the SDF
-        # geometry, nor an engine built to filter every step; without them
-        # lapsed slots are scanned, with the BVH leaf of each triangle).
-        lists = CELL_LIST_BYTES * len(library.shapes) * DISTANCE_GRID**3
-        listed = self.filter_margin > 0 and lists <= CELL_LIST_LIMIT
-        sizes["cellLists"] = lists if listed else 16
-        sizes["triangleLeaf"] = 16 if self.sdf else self.buffers["meshTriangles"].size // 12
-        for name, nbytes in sizes.items():
+        for name, nbytes in scratch_sizes(h, self.filter_margin).items():
             self.buffers[name] = DeviceBuffer(self, nbytes)
-        side_sizes = {
-            "meta": 16 * cc, "slip": 16 * cc, "normalArea": 16 * cc, "hash": 16,
-            "sidePairOffsets": 4 * (n + 1), "sidePairB": 4 * pc, "sideContactStart": 4 * (pc + 1),
-            "sideWallStart": 4 * (walls + 1),
-        }
-        self.sides = [{k: DeviceBuffer(self, v) for k, v in side_sizes.items()} for _ in (0, 1)]
+        sides = side_sizes(h)
+        self.sides = [{k: DeviceBuffer(self, v) for k, v in sides.items()} for _ in (0, 1)]
         for name in BUFFER_ORDER:
             if name not in self.buffers and name not in dict(SIDE_FIELDS) and name not in dict(
                 (o, k) for k, o in SIDE_FIELDS
             ):
                 raise RuntimeError(f"unallocated buffer {name}")
-        backup_names = (
-            "position", "velocity", "rotation", "momentum", "cell", "force", "torque", "referencePosition",
-            "referenceCell", "control", "pairs", "pairCounts", "pairOffsets", "particleStress",
-            "particleDiagnostic", "timestepRows", "accumulated", "referencePositionRemainder",
-            *RESIDUAL_STATE, *DAMPING_STATE, "contactCounts", "byJOffsets", "byJPairs",
-            *(WALL_STATE if self.wall_count else ()),
-        )
-        self.backups = {name: DeviceBuffer(self, self.buffers[name].size) for name in backup_names}
-        self.history_backup = {k: DeviceBuffer(self, self.sides[0][k].size) for k in side_sizes}
+        self.backups = {name: DeviceBuffer(self, self.buffers[name].size) for name in backup_names(h)}
+        self.history_backup = {k: DeviceBuffer(self, self.sides[0][k].size) for k in sides}
+        self.estimated_bytes = sum(buffer.size for group in (self.buffers, *self.sides, self.backups, self.history_backup)
+                                   for buffer in group.values())
         self._native = self.lib.sdg_engine_create()
         if not self._native:
             raise MemoryError("GB300 engine allocation failed")

@@ -411,16 +411,9 @@ class HostLayout:
         state["invI"] = self.invI.copy()
         return state
 
-    def estimated_bytes(self):
-        """Device working set of this backend, including its own scratch."""
-        n, p, c = self.n, self.pair_capacity, self.contact_capacity
-        geometry = sum(a.nbytes for a in self.geometry.values())
-        candidates = 2 * p * self.max_leaves
-        return int(
-            1184 * n
-            + 8 * self.bin_count * self.bin_capacity
-            + 196 * p + 2 * 8 * p * (self.max_leaves + 31) // 32
-            + 16 * candidates
-            + 2 * 96 * c + 64 * c
-            + geometry
-        )
+    def estimated_bytes(self, **settings):
+        """Device working set of this backend, including its own scratch and the
+        library's triangle lists (``engine.working_set``; ``filter_margin``)."""
+        from .engine import working_set
+
+        return working_set(self, **settings)
