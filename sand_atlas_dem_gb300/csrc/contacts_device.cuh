@@ -1468,7 +1468,7 @@ __device__ __forceinline__ void sdfQueryPairs(const Params& P, uint32_t* list, u
         }
         if (listed) evaluate(listed);
         __syncwarp();
-        r.sdfLaneCounts[size_t(WARP) * p + lane] = counts[lane] | (counts[lane + WARP] << 16);  // at most 81 each
+        r.sdfLaneCounts[size_t(WARP) * p + lane] = counts[lane] | (counts[lane + WARP] << 16);  // each below 65,536 (the host checks)
         if (lane == 0) r.contactCounts[p] = total;
     }
 }

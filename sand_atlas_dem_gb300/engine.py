@@ -236,6 +236,15 @@ def scratch_sizes(h, filter_margin):
     return sizes
 
 
+def check_lane_counts(h):
+    """A pair's SDF contacts are counted per virtual lane (every 64th node of its two
+    grains) in 16 bits; refuses a layout where a lane could hold more."""
+    lane = -(-2 * max(len(shape.samples) for shape in h.library.shapes) // 64)
+    if min(lane, h.contact_capacity) > 0xFFFF:
+        raise ValueError("SDF contacts need fewer than 65,536 nodes of a grain pair per virtual lane "
+                         "(two grains of at most 2,097,120 nodes)")
+
+
 def side_sizes(h):
     """Bytes of one contact-history side's buffers."""
     n, pc, cc = h.n, h.pair_capacity, h.contact_capacity
@@ -321,6 +330,7 @@ class Engine:
         self.sdf = spec.contact_geometry == "sdf"
         if self.sdf:
             self.distance_grid, self.filter_margin = False, 0.0
+            check_lane_counts(h)
         self._reduce_scratch = {}
         self._array_cache = {}
         self._value_cache = {}
