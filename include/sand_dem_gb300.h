@@ -232,8 +232,10 @@ int sdg_engine_diagnostics(void* const* buffers, const uint64_t* bytes, const do
 /*
  * One committed step with CUDA events between phases; writes SDG_PHASES
  * device milliseconds: drift, neighbours, pair cull, node filter (with the
- * survivor list and the learned culler), exact node queries, contact emit,
- * friction history + contact law, force gather, final kick.
+ * survivor list and the learned culler), exact node queries, contact emit
+ * (with stored exact-query lists and with the SDF geometry: and the grain
+ * contacts' law, one kernel), friction history + contact law (there: of the
+ * plane contacts), force gather, final kick.
  * Replaces Engine.profile_step's timestamp queries (gpu.py:938-1014).
  */
 int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes, const double* values,

@@ -10,6 +10,8 @@ on), decide occupancy against latency; the best choice depends on the
 workload (grains, contacts per grain, triangle counts) and on whether the
 culler runs.  None of these choices changes which work is done or the order
 in which any sum is accumulated, so every choice gives bit-identical results.
+The choices are those of launched steps (captured or not) and of the force
+pass; steps that run in one persistent launch have one CTA per SM and take none.
 
 :func:`tune` times each phase with CUDA events (``Engine.profile_phases``)
 for each candidate of its parameter in turn (coordinate descent, phases are

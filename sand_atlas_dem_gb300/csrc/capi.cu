@@ -424,6 +424,8 @@ int sdg_dispatch(const char* kernel, uint32_t count, void* const* buffers, const
 // drift (checkContactTimestep, beginStep, advanceCell),
 // neighbours, pair setup + leaf cull + item emit, node filter + survivor
 // list, exact node queries, contact emit, friction history + contact law, force gather, final kick.
+// The emit and the law are the step's own: one kernel, timed as the emit, with
+// stored lists and with the SDF geometry, where only the plane contacts' law is left.
 int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes, const double* values,
                        uint32_t nvalues, float* phase_ms, void* stream) {
     if (!engine || !phase_ms) { g_error = "null argument"; return 1; }
@@ -449,12 +451,13 @@ int sdg_engine_profile(void* engine, void* const* buffers, const uint64_t* bytes
     cudaEventRecord(ev[3], s);
     launch_contacts("collectFilter", P, 0, s);
     cudaEventRecord(ev[4], s);
-    launch_contacts("collectWalk", P, 0, s);
+    const bool fused = storedFilters(c) || c.meshGeometry == 0;
+    if (c.meshGeometry != 0) launch_contacts("collectWalk", P, 0, s);
     cudaEventRecord(ev[5], s);
-    launch_contacts("collectEmit", P, 0, s);
-    launch_contacts("collectWalls", P, 0, s);
+    if (!fused) launch_contacts("collectEmit", P, 0, s);
+    launch_contacts(fused ? "collectEmitLaw" : "collectWalls", P, 0, s);
     cudaEventRecord(ev[6], s);
-    launch_contacts("resolveContacts", P, 0, s);
+    launch_contacts(fused ? "resolveWalls" : "resolveContacts", P, 0, s);
     cudaEventRecord(ev[7], s);
     launch_contacts("gather", P, c.N, s);
     launch_contacts("gatherWallRows", P, c.N, s);

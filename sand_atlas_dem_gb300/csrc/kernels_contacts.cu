@@ -779,17 +779,19 @@ static void contacts(const Params& P, cudaStream_t s) {
     collectEmit(P, s);
     collectWalls(P, s);
 }
-// The exact queries, contact records with their law, and plane contacts: the
-// part of the collector every step runs once the stored filter results are
-// in place.
-static void collectTail(const Params& P, cudaStream_t s) {
-    if (P.c.meshGeometry == 0) {
+// Contact records with their law, and plane contacts.
+static void collectEmitLaw(const Params& P, cudaStream_t s) {
+    if (P.c.meshGeometry == 0)
         k_sdfEmit<true><<<grid(P.c.queryBlocksPerSM, 8), 256, 0, s>>>(P);
-    } else {
-        collectWalk(P, s);
+    else
         k_emitSlots<true><<<grid(P.c.contactBlocksPerSM, 8), 256, 0, s>>>(P);
-    }
     collectWalls(P, s);
+}
+// The exact queries and the above: the part of the collector every step runs
+// once the stored filter results are in place.
+static void collectTail(const Params& P, cudaStream_t s) {
+    if (P.c.meshGeometry != 0) collectWalk(P, s);
+    collectEmitLaw(P, s);
 }
 static void resolveWalls(const Params& P, cudaStream_t s) {
     if (P.c.wallCount) k_resolveWalls<<<grid(0, 2), 256, 0, s>>>(P);
@@ -823,6 +825,7 @@ int launch_contacts(const std::string_view& name, const Params& P, uint32_t coun
     }
     else if (name == "collectBuild") { cullBuild(P, s); collectFilter(P, s); }
     else if (name == "collectTail") collectTail(P, s);
+    else if (name == "collectEmitLaw") collectEmitLaw(P, s);
     else if (name == "collectQuery") collectQuery(P, s);
     else if (name == "collectFilter") collectFilter(P, s);
     else if (name == "collectWalk") collectWalk(P, s);

@@ -61,3 +61,27 @@ def test_tune_restores_state_and_caches(gpu_library, tmp_path):
     ref.initialize()
     ref.advance(4)
     assert g.state()["position"].tobytes() == ref.state()["position"].tobytes()
+
+
+@pytest.mark.parametrize("settings", [{}, dict(filter_margin=0.0)])
+@pytest.mark.parametrize("geometry", ["mesh", "sdf"])
+def test_profiled_phases_are_the_launched_step(gpu_library, geometry, settings):
+    """The timed phases run the launched step's kernels: the law with the emit
+    where the step fuses them (which then leaves contactPair alone)."""
+    from tests.specimens import walled_lattice
+
+    library, spec, case, _ = walled_lattice(geometry)
+    a, b = (build(Engine, library, spec, case, use_graph=False, **settings) for _ in range(2))
+    for e in (a, b):
+        e.initialize()
+        e.buffers["contactPair"].copy_from_numpy(np.full(e.contact_capacity, 0xABCDEF01, np.uint32))
+    phases = a.profile_phases()
+    b.advance(1)
+    assert all(ms >= 0 for ms in phases.values()) and a.step == b.step == 1
+    sa, sb = a.state(), b.state()
+    for k, v in sb.items():
+        if isinstance(v, np.ndarray):
+            assert v.tobytes() == sa[k].tobytes(), k
+    pairs = [e.read("contactPair", np.uint32) for e in (a, b)]
+    assert pairs[0].tobytes() == pairs[1].tobytes()
+    assert (pairs[0] == 0xABCDEF01).all() == (geometry == "sdf" or not settings)
