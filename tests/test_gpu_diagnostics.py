@@ -69,3 +69,22 @@ def test_group_edges_match_oracle(gpu_library, side, spacing):
     want = o.diagnostics()
     assert (want["candidate_pairs"] == 0) == (spacing == 1.6)
     compare(g.diagnostics(), want, 0)
+
+
+@pytest.mark.parametrize("side", [3, 7])
+def test_wall_rows_match_oracle(gpu_library, side):
+    """The per-wall rows the diagnostics read (reaction and contacts, moment and
+    power, work), bit for bit, in one group of 256 grains and in two levels."""
+    from tests.specimens import walled_lattice
+
+    library, spec, case, _ = walled_lattice(side=side)
+    o, g = build(OracleEngine, library, spec, case, threads=8), build(Engine, library, spec, case)
+    o.initialize()
+    g.initialize()
+    want = o.wall_rows()
+    walls = g._diagnostic_rows(g.config())[4]
+    assert walls[:, :3].tobytes() == want.tobytes()
+    for k, name in enumerate(("wallPlane", "wallRemainder", "wallVelocity")):
+        assert walls[:, 3 + k].tobytes() == np.ascontiguousarray(g.read(name, np.float32, (g.wall_count, 4))).tobytes()
+    assert all(wall["active_surface_contacts"] == int(want[w, 0, 3].view(np.uint32))
+               for w, wall in enumerate(g.diagnostics()["walls"]))
