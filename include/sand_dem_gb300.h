@@ -24,9 +24,10 @@
  *             two counters, the survivor mask and first survivor of each
  *             item and the (item, node slot) list of survivors -- the nodes
  *             left for the exact query after the conservative filters --
- *             and, for the learned culler, a keep flag per survivor, its
- *             exclusive scan and the list of kept survivors, and per
- *             directed pair the enclosure plane carried into the source
+ *             and a keep flag per survivor (then: per stored slot), its
+ *             exclusive scan and a list (survivors left for the exact query
+ *             where lists are built every step, else the step's slots
+ *             without a certificate that holds), and per directed pair the enclosure plane carried into the source
  *             grain's frame with its rejection-bound terms, and the
  *             triangle BVH as one record per node with both children's
  *             bounds, and per shape a 48^3 grid of certified lower bounds of
@@ -165,7 +166,7 @@ int sdg_scan_partials(void);
 
 /*
  * Device-to-device copies of n buffers on `stream` (dst[k] <- src[k],
- * bytes[k] each, one cudaMemcpyAsync per buffer).  The transactional backup
+ * bytes[k] each, up to 64 buffers a kernel launch).  The transactional backup
  * of a chunk and its restore, which the reference does with encoder buffer
  * copies (src/sand_atlas_dem/gpu.py:729-743, backend.py copy_buffer).
  */
@@ -220,9 +221,9 @@ int sdg_engine_advance(void* engine, void* const* buffers, const uint64_t* bytes
  * rows, the 2 reduced fabric rows, the first 3 cell rows and the 16 control
  * words; with planes, 96 bytes more per plane: its three reduced rows, plane,
  * remainder and velocity.  The caller waits on the stream before reading
- * `host`.  Scratch (both non-null, scratch_bytes each): ceil(max(N,
- * pairCapacity) / 256) x 8 rows x 16 bytes, and with planes at least (3 x
- * (ceil(N / 256) x 1.004 + 4) + 6) rows per plane and 17 more.  The row
+ * `host`.  scratch_a is used with planes only: at least (3 x (ceil(N / 256) x
+ * 1.004 + 4) + 6) rows of 16 bytes per plane and 17 more in scratch_bytes;
+ * scratch_b is not used.  Neither may be null.  The row
  * buffers (diagnosticRows, fabricRows) and the scan partials are overwritten.
  * Replaces the reference's per-reduction dispatches and reads.
  */

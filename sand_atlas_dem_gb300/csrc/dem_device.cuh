@@ -127,7 +127,7 @@ struct Res {
     uint2* candSurvMask;              // candidateCapacity: 64-bit mask of the item's surviving nodes
     uint32_t* candSurvOffset;         // candidateCapacity+1: first survivor of each item
     uint2* survivors;                 // survivorCapacity: (item, node slot) of each surviving node
-    uint32_t* survKeep;               // survivorCapacity+1: 1 = the learned culler keeps the survivor
+    uint32_t* survKeep;               // survivorCapacity+1: 1 = the survivor (then: the slot) stays, else 0
     uint32_t* keepOffset;             // survivorCapacity+1: exclusive scan of survKeep
     uint32_t* walkList;               // survivorCapacity: survivors left for the exact query (lists built every
                                       // step), the step's lapsed slots (stored lists)
@@ -596,25 +596,8 @@ __device__ __forceinline__ bool meshMayContain(const Res& r, uint32_t shape, f3 
     }
     return true;
 }
-// solver.slang:274-288
-__device__ __forceinline__ bool meshBoxMayContact(const Res& r, uint32_t shape, f3 low, f3 high) {
-    uint32_t root = __ldg(&r.meshRoots[shape].x);
-    f3 tl = xyz(__ldg(&r.meshMin[root])), th = xyz(__ldg(&r.meshMax[root]));
-    if (high.x < tl.x || high.y < tl.y || high.z < tl.z || low.x > th.x || low.y > th.y || low.z > th.z) return false;
-    f3 center = 0.5f * (low + high), half = 0.5f * (high - low);
-    f3 direction = (center - 0.5f * (tl + th)) / (th - tl);
-    f3 a = abs3(direction);
-    uint32_t axis = a.x >= a.y && a.x >= a.z ? 0 : (a.y >= a.z ? 1 : 2);
-    uint32_t group = 2 * axis + (comp(direction, axis) >= 0 ? 1 : 0);
-    uint4 info = __ldg(&r.meshHullInfo[6 * shape + group]);
-    for (uint32_t i = 0; i < info.y; ++i) {
-        float4 plane = __ldg(&r.meshPlanes[info.x + i]);
-        if (__fsub_rn(__fadd_rn(dot(xyz(plane), center), plane.w), dot(abs3(xyz(plane)), half)) > 0) return false;
-    }
-    return true;
-}
-// The first half of meshBoxMayContact: the target's root box test, and the
-// centre, half extent and hull group its plane loop would use.
+// solver.slang:274-288 up to its plane loop (which a warp runs): the target's root
+// box test, and the centre, half extent and hull group the loop uses.
 __device__ __forceinline__ bool meshBoxGroup(const Res& r, uint32_t shape, f3 low, f3 high, f3& center, f3& half,
                                              uint32_t& group) {
     uint32_t root = __ldg(&r.meshRoots[shape].x);
@@ -627,29 +610,6 @@ __device__ __forceinline__ bool meshBoxGroup(const Res& r, uint32_t shape, f3 lo
     uint32_t axis = a.x >= a.y && a.x >= a.z ? 0 : (a.y >= a.z ? 1 : 2);
     group = 2 * axis + (comp(direction, axis) >= 0 ? 1 : 0);
     return true;
-}
-// solver.slang:290-305, with the directed-pair branch supplied.
-// With `margin`, the box is grown by that distance (the test then holds for
-// every placement within `margin` of this one).
-__device__ __forceinline__ bool meshClusterMayContact(const Res& r, uint32_t src, uint32_t dst, uint32_t cluster, f3 branch,
-                                                      float margin = 0.0f) {
-    f3 sl = xyz(r.meshClusterMin[cluster]), sh = xyz(r.meshClusterMax[cluster]);
-    f3 low = mk(1e30f, 1e30f, 1e30f), high = mk(-1e30f, -1e30f, -1e30f);
-    float4 qs = r.rotation[src], qd = r.rotation[dst];
-    float ss = r.body[src].x, sd = r.body[dst].x;
-    for (uint32_t corner = 0; corner < 8; ++corner) {
-        f3 p = mk((corner & 1) ? sh.x : sl.x, (corner & 2) ? sh.y : sl.y, (corner & 4) ? sh.z : sl.z);
-        p = qinv(qd, qrot(qs, p * ss) - branch) / sd;
-        low = mn3(low, p);
-        high = mx3(high, p);
-    }
-    float pad = __fmul_rn(0.00000762939453125f,
-        __fadd_rn(__fadd_rn(__fadd_rn(1.0f, mx(mx(fabsf(low.x), fabsf(low.y)), fabsf(low.z))),
-                            mx(mx(fabsf(high.x), fabsf(high.y)), fabsf(high.z))), __fdiv_rn(length(branch), sd)));
-    if (margin > 0.0f) pad = __fadd_rn(pad, margin);
-    low = low - mk(pad, pad, pad);
-    high = high + mk(pad, pad, pad);
-    return meshBoxMayContact(r, r.shapeId[dst], low, high);
 }
 // solver.slang:404-417
 // With `margin`, the bounds are grown by that distance.
@@ -1059,8 +1019,7 @@ __device__ __forceinline__ uint32_t hitsBefore(const SlotHits& hits, uint32_t w)
     return __reduce_add_sync(0xffffffffu, sum);
 }
 // Whether the exact-query list itself is stored with the filter results
-// (built with grown tests and ordered by target shape and coarse cell).  Not
-// with the learned culler, whose calibrated decision is taken every step.
+// (built with grown tests, in contact order).  Not with the learned culler, whose calibrated decision is taken every step.
 __host__ __device__ __forceinline__ bool storedKeep(const Config& c) { return c.filterMargin > 0.0f && c.cullerEnabled == 0; }
 // Margin the filter results are built with on this step (0 without them).
 __device__ __forceinline__ float buildMargin(const Res& r, const Config& c) {

@@ -1,5 +1,5 @@
 // The integrator's per-grain steps, shared by the kernels of a launched step
-// (kernels_state.cu) and the persistent step (kernels_contacts.cu): the
+// (kernels_state.cu) and the persistent step (run_device.cuh): the
 // arithmetic of the reference kernel named beside each, in its FP32 order.
 #pragma once
 #include "dem_device.cuh"
