@@ -420,7 +420,7 @@ class Engine:
 
     def _values(self, config):
         """The value block of a config (built once per distinct content)."""
-        key = (tuple(config.items()), self.culler is not None, tuple(self.tuning.items()), self.leaf_words,
+        key = (tuple(config), tuple(config.values()), self.culler is not None, tuple(self.tuning.items()), self.leaf_words,
                self.candidate_capacity, self.specimens, self.survivor_capacity, self.distance_grid,
                self.filter_margin)
         cached = self._value_cache.get(key)
